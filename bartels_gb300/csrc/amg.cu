@@ -33,13 +33,15 @@
 //
 // V-cycle (the PCG preconditioner, symmetric): on level 0 one Chebyshev step
 // of the smoother before and after the coarse correction; on coarse levels
-// `deg` steps (1 on level 1, 5 below by default). The smoother of level 0 is
-// block-Jacobi or the learned factor M = G^T G (the network's output on the
-// Hessian's lower block pattern). The smoothing passes read exactly
-// symmetric BF16 copies of the operators (the fine one in padded rows); the
-// Galerkin products use the FP32 values. Every kernel becomes a no-op once
-// the PCG's convergence flag is set, so fixed-length CUDA graphs of PCG
-// iterations can contain it.
+// `deg` steps (by default 1 on level 1, 2 where it is in the cluster launch, 5
+// below). The smoother of level 0 is block-Jacobi or the learned factor
+// M = G^T G (the network's output on the Hessian's lower block pattern). The
+// smoothing passes read exactly symmetric BF16 copies of the operators (the
+// fine one in padded rows); the Galerkin products use the FP32 values. The
+// levels that fit the shared memory of one thread-block cluster run as one
+// kernel (k_mgc_cluster). Every kernel becomes a no-op once the PCG's
+// convergence flag is set, so fixed-length CUDA graphs of PCG iterations can
+// contain it.
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -60,7 +62,7 @@ int plan_lanes_tri(bartels_ctx ctx, bartels_mesh_plan plan);
 
 namespace {
 
-constexpr int kDenseNodes = 24;   // coarsest level solved densely up to 24 nodes (144 DOFs)
+constexpr int kDenseNodes = 64;   // coarsest level solved densely up to 64 nodes (384 DOFs)
 constexpr int kPowerIters = 10;   // power iterations for each smoother's largest eigenvalue
 constexpr int kCoarsestDeg = 6;   // Chebyshev steps on a coarsest level that is neither dense nor block diagonal
 
@@ -279,6 +281,154 @@ int dalloc_n(MgHierarchy *mg, T **dst, size_t count) {
 
 }  // namespace
 
+constexpr int kClThreads = 512;  // threads per CTA of the coarse-cycle cluster
+__global__ void k_mgc_cluster(const __grid_constant__ MgClArgs a, const PcgState *__restrict__ st);
+
+namespace {
+
+// launch configuration of one cluster of `ctas` CTAs
+cudaLaunchConfig_t cluster_config(bartels_ctx ctx, int ctas, int threads, int smem, cudaLaunchAttribute *at) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Node ranges of a level for `ctas` CTAs, balanced by stored blocks (a dense
+// level: by nodes, so that 4 CTAs hold the inverse of kDenseNodes nodes).
+void cluster_split(const HostLevel &h, bool dense, int ctas, int *split) {
+  if (dense) {
+    const int per = (h.n + ctas - 1) / ctas;
+    for (int q = 0; q <= ctas; ++q) split[q] = std::min(h.n, q * per);
+    return;
+  }
+  const int64_t total = h.rp[h.n];
+  for (int q = 0; q <= ctas; ++q) {
+    const int64_t want = total * q / ctas;
+    split[q] = (int)(std::lower_bound(h.rp.begin(), h.rp.end(), want) - h.rp.begin());
+  }
+  split[0] = 0;
+  split[ctas] = h.n;
+}
+
+// Shared-memory layout of levels first .. last for a cluster of a.ctas CTAs;
+// returns the bytes each CTA needs.
+int64_t cluster_layout(MgClArgs &a) {
+  int64_t off = 0;
+  auto take = [&](int64_t bytes) {
+    const int64_t o = off;
+    off += (bytes + 15) & ~int64_t(15);
+    return (int)std::min<int64_t>(o, INT_MAX);
+  };
+  for (int l = 0; l < a.nlev; ++l) {
+    MgClLevel &L = a.lv[l];
+    const bool last = l + 1 == a.nlev, dense = last && a.last_mode == kMgLastDense;
+    int64_t rows = 0, blocks = 0, mems = 0;
+    for (int q = 0; q < a.ctas; ++q) {
+      rows = std::max<int64_t>(rows, L.split[q + 1] - L.split[q]);
+      blocks = std::max<int64_t>(blocks, L.bsplit[q + 1] - L.bsplit[q]);
+      mems = std::max<int64_t>(mems, L.msplit[q + 1] - L.msplit[q]);
+    }
+    if (dense) {
+      L.o_val = take(sizeof(float) * 6 * rows * a.nd);
+    } else {
+      L.o_val = take(72 * blocks);
+      L.o_ci = take(4 * blocks);
+      L.o_rp = take(4 * (rows + 1));
+      L.o_dinv = take(144 * rows);
+    }
+    if (!last) {
+      L.o_Q = take(144 * rows);
+      L.o_agg = take(4 * rows);
+    }
+    if (l > 0) {
+      L.o_mptr = take(4 * (rows + 1));
+      L.o_mem = take(4 * mems);
+    }
+    if (!dense) {
+      L.o_b = take(24 * rows);
+      L.o_x = take(24 * rows);
+      L.o_r = take(24 * rows);
+      L.o_d = take(24 * rows);
+    }
+  }
+  if (a.last_mode == kMgLastDense) a.o_db = take(sizeof(float) * a.nd);
+  return off;
+}
+
+// The coarse part of the hierarchy as one cluster launch (k_mgc_cluster):
+// levels from the finest one that fits the cluster's shared memory down to the
+// coarsest. Leaves cl.ctas = 0 (the per-level launches) when not even the
+// coarsest level fits or the device cannot host the cluster.
+int build_cluster(bartels_ctx ctx, MgHierarchy *mg, const std::vector<HostLevel> &H) {
+  constexpr int kSmem = 220 * 1024;
+  const int L = (int)H.size();
+  const int want = env_int("BARTELS_MG_CLUSTER", kMgClusterMax, 4, kMgClusterMax);
+  mg->cl = MgClArgs();
+  BT_CUDA(cudaFuncSetAttribute(k_mgc_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  BT_CUDA(cudaFuncSetAttribute(k_mgc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (int first = std::max(1, L - kMgClusterLevels); first < L; ++first) {
+    MgClArgs a;
+    a.first = first;
+    a.nlev = L - first;
+    a.last_mode = mg->dense ? kMgLastDense : (mg->coarse_blockdiag ? kMgLastExact : kMgLastCheb);
+    a.nd = mg->nd;
+    a.ainv = mg->ainv;
+    a.coef = mg->coef;
+    a.ctas = want;
+    for (int l = 0; l < a.nlev; ++l) {
+      const HostLevel &h = H[first + l];
+      MgClLevel &c = a.lv[l];
+      cluster_split(h, mg->dense && l + 1 == a.nlev, a.ctas, c.split);
+      for (int q = 0; q <= a.ctas; ++q) {
+        c.bsplit[q] = h.rp[c.split[q]];
+        c.msplit[q] = l > 0 ? H[first + l - 1].mptr[c.split[q]] : 0;
+      }
+    }
+    const int64_t smem = cluster_layout(a);
+    if (smem > kSmem) continue;
+    a.smem = (int)smem;
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = cluster_config(ctx, a.ctas, kClThreads, a.smem, at);
+    int fit = 0;
+    BT_CUDA(cudaOccupancyMaxActiveClusters(&fit, k_mgc_cluster, &cfg));
+    if (fit < 1) return fail(BARTELS_E_UNSUPPORTED, "multigrid: the device cannot host the coarse-cycle cluster");
+    for (int l = 0; l < a.nlev; ++l) {
+      const MgLevel &d = mg->lv[first + l];
+      MgClLevel &c = a.lv[l];
+      c.deg = d.deg;
+      c.rp = d.rp;
+      c.ci = d.ci;
+      c.agg = d.agg;
+      c.val16 = d.val16;
+      c.dinv = d.dinv;
+      c.Q = d.Q;
+      c.gb = d.b;
+      c.gx = d.x;
+      c.gd = d.d;
+      c.gd2 = d.d2;
+      c.gres = l + 1 < a.nlev ? d.x2 : d.x;  // as level_result
+      if (l > 0) {
+        c.mptr = mg->lv[first + l - 1].mptr;
+        c.midx = mg->lv[first + l - 1].midx;
+      }
+    }
+    mg->cl = a;
+    return BARTELS_OK;
+  }
+  if (mg->dense) return fail(BARTELS_E_DEVICE, "multigrid: the dense level does not fit the cluster");
+  return BARTELS_OK;
+}
+
+}  // namespace
+
 MgHierarchy::~MgHierarchy() {
   for (void *p : allocs) cudaFree(p);
 }
@@ -365,11 +515,15 @@ int mg_prepare(bartels_ctx ctx, bartels_mesh_plan plan) {
   const int deg0 = env_int("BARTELS_MG_DEG0", 1, 1, 1);
   // Chebyshev degrees: level 1 (the largest coarse level; its one step is
   // fused into the restriction) and the levels below it, whose steps are
-  // cheap and cut the PCG iterations. n = 96, one multigrid solve: level 1 at
-  // 3 with 3 / 4 / 5 / 6 below gives 70 / 66 / 63 / 62 iterations and 50.4 /
-  // 49.5 / 49.1 / 50.1 ms; with 5 below, level 1 at 1 / 2 / 3 / 4 gives
-  // 47.1 / 48.2 / 48.8 / 50.2 ms.
+  // cheap and cut the PCG iterations. n = 96, a multigrid solve to 1e-9: level
+  // 1 at 1 with 3 / 4 / 5 / 6 below gives 59.8 / 57.6 / 56.4 / 55.7 ms (n = 48,
+  // learned smoother: 14.0 / 13.7 / 13.7 / 13.9), level 1 at 2 with 4 / 5 below
+  // 59.4 / 58.5.
   const int degc = env_int("BARTELS_MG_DEGC", 1, 1, (kMgCoef - 1) / 2 + 1);
+  // level 1 inside the cluster launch, where a step is cheap (24^3 Newton step:
+  // 1 / 2 / 3 / 4 / 5 give 12.5 / 11.6 / 11.4 / 11.5 / 11.8 ms, smaller solves
+  // are best at 2)
+  const int degcl = env_int("BARTELS_MG_DEGCL", 2, 1, (kMgCoef - 1) / 2 + 1);
   const int degc2 = env_int("BARTELS_MG_DEGC2", 5, 1, (kMgCoef - 1) / 2 + 1);
   mg->lv.resize(H.size());
   for (size_t l = 0; l < H.size(); ++l) {
@@ -439,12 +593,15 @@ int mg_prepare(bartels_ctx ctx, bartels_mesh_plan plan) {
   if (mg->dense) {
     mg->nd = 6 * mg->lv.back().n;
     BT_CHECK(dalloc_n(mg, &mg->ainv, (size_t)mg->nd * mg->nd));
+    BT_CHECK(dalloc_n(mg, &mg->panel, 2 * 6 * (size_t)mg->nd));
   }
   BT_CHECK(dalloc_n(mg, &mg->coef, (size_t)kMgMaxLevels * kMgCoef));
   BT_CHECK(dalloc_n(mg, &mg->norms, 2 * (size_t)kMgMaxLevels));
   mg->nparts = 4096;
   BT_CHECK(dalloc_n(mg, &mg->part, (size_t)mg->nparts));
   BT_CUDA(cudaMemset(mg->coef, 0, sizeof(float) * kMgMaxLevels * kMgCoef));
+  BT_CHECK(build_cluster(ctx, mg, H));
+  if (mg->cl.ctas && mg->cl.first == 1 && H.size() > 2) mg->lv[1].deg = mg->cl.lv[0].deg = degcl;
   return BARTELS_OK;
 }
 
@@ -624,64 +781,94 @@ __global__ void k_mg_inv6(int n, const int *__restrict__ dpos, const float *__re
   }
 }
 
-// Dense inverse of the coarsest level (nd = 6 x nodes <= 144): the level's
-// blocks scattered into shared memory, in-place Gauss-Jordan (no pivoting, the
-// matrix is SPD), dead DOFs as in k_mg_inv6. One CTA.
-__global__ void __launch_bounds__(1024)
-k_mg_dense_inv(int nodes, const int *__restrict__ rp, const int *__restrict__ ci, const float *__restrict__ val,
-               float *__restrict__ ainv) {
-  extern __shared__ float sA[];
-  __shared__ float s_p;
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Dense inverse of the coarsest level (nd = 6 x nodes <= 384, symmetrised) by
+// in-place block Gauss-Jordan without pivoting (the matrix is SPD). Dead DOFs
+// as in k_mg_inv6. One thread-block cluster; each CTA keeps the rows of its
+// own nodes (split) in shared memory. Per node K: the owner eliminates within
+// the node's 6 rows and publishes them (panel, double-buffered), then every
+// CTA updates its other rows. One cluster barrier per node: 8 / 64 nodes take
+// ~16 / ~130 us; a single CTA with a barrier per scalar pivot took 58 us for
+// 8 and 552 us for 18.
+struct MgInvArgs {
+  int nodes = 0, split[kMgClusterMax + 1] = {};
+  const int *rp = nullptr, *ci = nullptr, *rev = nullptr, *dpos = nullptr;
+  const float *val = nullptr;
+  float *panel = nullptr, *ainv = nullptr;
+};
+constexpr int kInvThreads = 512;
+__global__ void __launch_bounds__(kInvThreads, 1)
+k_mg_dense_inv(const __grid_constant__ MgInvArgs a) {
+  extern __shared__ __align__(16) float sA[];  // own rows (6 x own nodes) x nd, then the panel 6 x nd
   __shared__ unsigned char dead[6 * kDenseNodes];
-  const int nd = 6 * nodes;
-  for (int i = threadIdx.x; i < nd * nd; i += blockDim.x) sA[i] = 0.f;
+  const int rank = cl_rank(), n0 = a.split[rank], n1 = a.split[rank + 1], rows = 6 * (n1 - n0), nd = 6 * a.nodes;
+  float *sP = sA + rows * nd;
+  for (int i = threadIdx.x; i < nd; i += blockDim.x) dead[i] = !(a.val[36ll * a.dpos[i / 6] + 7 * (i % 6)] != 0.f);
+  for (int e = threadIdx.x; e < rows * nd; e += blockDim.x) sA[e] = 0.f;
   __syncthreads();
-  for (int I = 0; I < nodes; ++I)
-    for (int k = rp[I]; k < rp[I + 1]; ++k) {
-      const int J = ci[k];
-      for (int e = threadIdx.x; e < 36; e += blockDim.x) {
-        const int a = e / 6, b = e - 6 * (e / 6);
-        sA[(6 * I + a) * nd + 6 * J + b] = val[36ll * k + e];
+  for (int I = n0; I < n1; ++I)
+    for (int e = threadIdx.x; e < 36 * (a.rp[I + 1] - a.rp[I]); e += blockDim.x) {
+      const int k = a.rp[I] + e / 36, r = (e % 36) / 6, c = e % 6, i = 6 * I + r, j = 6 * a.ci[k] + c;
+      const float t = 0.5f * (a.val[36ll * k + 6 * r + c] + a.val[36ll * a.rev[k] + 6 * c + r]);
+      sA[(i - 6 * n0) * nd + j] = (dead[i] || dead[j]) ? 0.f : t;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows; i += blockDim.x)
+    if (dead[6 * n0 + i]) sA[i * nd + 6 * n0 + i] = 1.f;
+  __syncthreads();
+  for (int K = 0; K < a.nodes; ++K) {
+    float *pan = a.panel + (K & 1) * 6 * nd;
+    if (K >= n0 && K < n1) {
+      float *R = sA + 6 * (K - n0) * nd;  // the node's 6 rows
+      for (int k = 0; k < 6; ++k) {
+        const int kk = 6 * K + k;
+        const float piv = R[k * nd + kk], p = piv > 0.f ? 1.f / piv : 0.f;
+        float f[6];
+#pragma unroll
+        for (int r = 0; r < 6; ++r) f[r] = R[r * nd + kk];
+        __syncthreads();
+        for (int j = threadIdx.x; j < nd; j += blockDim.x) {
+          const float t = j == kk ? p : R[k * nd + j] * p;
+#pragma unroll
+          for (int r = 0; r < 6; ++r) {
+            if (r == k) R[r * nd + j] = t;
+            else R[r * nd + j] = j == kk ? -f[r] * p : R[r * nd + j] - f[r] * t;
+          }
+        }
+        __syncthreads();
+      }
+      for (int e = threadIdx.x; e < 6 * nd; e += blockDim.x) pan[e] = R[e];
+    }
+    cl_barrier();
+    for (int e = threadIdx.x; e < 6 * nd; e += blockDim.x) sP[e] = __ldcg(pan + e);
+    __syncthreads();
+    // one warp per row: row -= f . panel, f the row's entries in the node's columns
+    for (int i = threadIdx.x >> 5; i < rows; i += blockDim.x >> 5) {
+      if (n0 + i / 6 == K) continue;
+      float *row = sA + i * nd, f[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) f[k] = row[6 * K + k];
+      __syncwarp();
+      for (int j = threadIdx.x & 31; j < nd; j += 32) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += f[k] * sP[k * nd + j];
+        row[j] = (j >= 6 * K && j < 6 * K + 6) ? -s : row[j] - s;
       }
     }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nd; i += blockDim.x) dead[i] = !(sA[i * nd + i] != 0.f);
-  __syncthreads();
-  for (int e = threadIdx.x; e < nd * nd; e += blockDim.x) {
-    const int i = e / nd, j = e - nd * (e / nd);
-    if (dead[i] || dead[j]) sA[e] = (i == j) ? 1.f : 0.f;
-    else if (i > j) sA[e] = 0.5f * (sA[e] + sA[j * nd + i]);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < nd * nd; e += blockDim.x) {
-    const int i = e / nd, j = e - nd * (e / nd);
-    if (i < j) sA[e] = sA[j * nd + i];
-  }
-  __syncthreads();
-  for (int k = 0; k < nd; ++k) {
-    if (threadIdx.x == 0) {
-      const float piv = sA[k * nd + k];
-      s_p = (piv > 0.f) ? 1.f / piv : 0.f;
-    }
-    __syncthreads();
-    const float p = s_p;
-    for (int j = threadIdx.x; j < nd; j += blockDim.x)
-      if (j != k) sA[k * nd + j] *= p;
-    __syncthreads();
-    for (int e = threadIdx.x; e < nd * nd; e += blockDim.x) {
-      const int i = e / nd, j = e - nd * (e / nd);
-      if (i != k && j != k) sA[e] -= sA[i * nd + k] * sA[k * nd + j];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nd; i += blockDim.x) {
-      if (i != k) sA[i * nd + k] *= -p;
-      else sA[k * nd + k] = p;
-    }
     __syncthreads();
   }
-  for (int e = threadIdx.x; e < nd * nd; e += blockDim.x) {
-    const int i = e / nd, j = e - nd * (e / nd);
-    ainv[e] = (dead[i] || dead[j]) ? 0.f : sA[e];
+  for (int e = threadIdx.x; e < rows * nd; e += blockDim.x) {
+    const int i = 6 * n0 + e / nd, j = e % nd;
+    a.ainv[6ll * n0 * nd + e] = (dead[i] || dead[j]) ? 0.f : sA[e];
   }
 }
 
@@ -1226,20 +1413,298 @@ k_mgc_MA(int n, const int *__restrict__ rp, const int *__restrict__ ci, const __
   BT_CROW_LOOP_END
 }
 
-// coarsest level, dense: x = Ainv b (one CTA)
-__global__ void __launch_bounds__(256)
-k_mg_dense_apply(int nd, const float *__restrict__ ainv, const float *__restrict__ b, float *__restrict__ x,
-                 const PcgState *__restrict__ st) {
+// ==================================== coarse levels in one cluster launch ===
+// The coarse part of the V-cycle (every level from cl.first down to the
+// coarsest and back) as one kernel of one thread-block cluster. Each CTA owns
+// a contiguous range of every level's nodes and keeps their BF16 blocks,
+// inverse diagonal blocks, transfer blocks and own vector entries in shared
+// memory. A step gathers its neighbours' vector entries through L2 and ends in
+// one hardware cluster barrier.
+//
+// Why: as launches these levels are 27 dependent kernels of 1 - 42 CTAs per
+// V-cycle, each bound by its launch and by a chain of three L2 latencies (row
+// pointer -> column -> vector), 4 - 9 us apiece. Here a step is one barrier
+// (~500 cycles, plus the flush of the step's stores) and one L2 latency (~460);
+// measured after its wait, the coarse part takes 42 us on the 96^3-cell cube
+// (1,331 + 64 nodes; ~150 us as launches) and 12 us at 24^3 (670 + 27). The
+// operators are staged before the wait on the previous kernel, i.e. while that
+// one is still running. 16 CTAs beat 8 (12.5 against 13.0 ms for a 24^3 Newton
+// step, 56.5 against 60.4 ms for a 96^3 solve): a step's row products are
+// bound by the shared-memory and issue rate of the CTAs that hold the level. Gathering
+// through distributed shared memory instead was measured and is slower: a
+// single load takes ~500 cycles, and scattered 24-byte entries from 1024
+// threads ~8,000.
+__device__ __forceinline__ void ldcg6(const float *v, int node, float x[6]) {
+  const float2 *p = reinterpret_cast<const float2 *>(v + 6 * node);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float2 t = __ldcg(p + q);
+    x[2 * q] = t.x;
+    x[2 * q + 1] = t.y;
+  }
+}
+
+// d = a * b + c on two packed FP32 values
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(d)
+      : "l"(*reinterpret_cast<unsigned long long *>(&a)), "l"(*reinterpret_cast<unsigned long long *>(&b)),
+        "l"(*reinterpret_cast<unsigned long long *>(&c)));
+  return *reinterpret_cast<float2 *>(&d);
+}
+
+// s = (A v)_i of the CTA's own row i, over a group of G lanes (all lanes end with the sum)
+template <int G>
+__device__ __forceinline__ void cl_row(const char *sm, const MgClLevel &L, const float *v, int i, bool active, int sl,
+                                       float s[6]) {
+  float2 s2[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) s2[c] = make_float2(0.f, 0.f);
+  if (active) {
+    const int *rp = reinterpret_cast<const int *>(sm + L.o_rp);
+    const int *ci = reinterpret_cast<const int *>(sm + L.o_ci);
+    const int k0 = rp[0], k1 = rp[i + 1] - k0;
+#pragma unroll 2
+    for (int k = rp[i] - k0 + sl; k < k1; k += G) {
+      float2 x[3];
+      const float2 *xp = reinterpret_cast<const float2 *>(v) + 3 * ci[k];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) x[q] = __ldcg(xp + q);
+      const uint2 *a2 = reinterpret_cast<const uint2 *>(sm + L.o_val) + 9 * k;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const uint2 t = a2[q];  // entries 4q .. 4q + 3 of the row-major block: pairs 2q and 2q + 1 of its 18
+        s2[(2 * q) / 3] = fma2(make_float2(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u)),
+                               x[(2 * q) % 3], s2[(2 * q) / 3]);
+        s2[(2 * q + 1) / 3] = fma2(make_float2(__uint_as_float(t.y << 16), __uint_as_float(t.y & 0xFFFF0000u)),
+                                   x[(2 * q + 1) % 3], s2[(2 * q + 1) / 3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 6; ++c) s[c] = s2[c].x + s2[c].y;
+  group_reduce6<G>(s);
+}
+
+// One smoothing step of the CTA's own rows: r -= A v (kStepPost: r = b - A v,
+// v = x), then with z = Dinv r
+//   kStepCheb:  d = c1 d + c2 z, acc += d
+//   kStepPost:  d = c2 z, acc = x + d  (acc is the b area: b is read for the last time here)
+//   kStepResid: d = Q^T r, the node's share of the restriction
+// and out = d for the other CTAs, or acc on the level's final step. A row's
+// group holds the whole sum in every lane; its lanes share the components of
+// the 6x6 product.
+enum { kStepCheb = 0, kStepPost = 1, kStepResid = 2 };
+template <int G>
+__device__ __forceinline__ void cl_step_g(char *sm, const MgClLevel &L, int r0, int rows, int mode, const float *v,
+                                          float *out, int o_acc, bool final, float c1, float c2) {
+  const int sl = threadIdx.x % G, g = threadIdx.x / G;
+  const float *rr = reinterpret_cast<const float *>(sm + (mode == kStepPost ? L.o_b : L.o_r));
+  float *rw = reinterpret_cast<float *>(sm + L.o_r), *d = reinterpret_cast<float *>(sm + L.o_d);
+  float *x = reinterpret_cast<float *>(sm + L.o_x), *acc = reinterpret_cast<float *>(sm + o_acc);
+  const float *M = reinterpret_cast<const float *>(sm + (mode == kStepResid ? L.o_Q : L.o_dinv));
+  for (int i0 = 0; i0 < rows; i0 += blockDim.x / G) {
+    const int i = i0 + g;
+    const bool active = i < rows;
+    float s[6];
+    cl_row<G>(sm, L, v, i, active, sl, s);
+    float rn[6];
+    if (active)
+#pragma unroll
+      for (int c = 0; c < 6; ++c) rn[c] = rr[6 * i + c] - s[c];
+    __syncwarp();
+    if (active)
+#pragma unroll
+    for (int a = sl; a < 6; a += G) {
+      const float *m = M + 36 * i + (mode == kStepResid ? a : 6 * a);  // column a of Q, row a of Dinv
+      const int st = mode == kStepResid ? 6 : 1;
+      float z = 0.f, mine = rn[0];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) z += m[st * c] * rn[c];
+#pragma unroll
+      for (int c = 1; c < 6; ++c) mine = a == c ? rn[c] : mine;
+      const int e = 6 * i + a;
+      float o = z;
+      if (mode != kStepResid) {
+        rw[e] = mine;
+        const float dk = mode == kStepCheb ? c1 * d[e] + c2 * z : c2 * z;
+        const float ak = (mode == kStepCheb ? acc[e] : x[e]) + dk;
+        d[e] = dk;
+        acc[e] = ak;
+        o = final ? ak : dk;
+      }
+      out[6 * r0 + e] = o;
+    }
+  }
+}
+__device__ __forceinline__ void cl_step(char *sm, const MgClLevel &L, int r0, int rows, int mode, const float *v,
+                                        float *out, int o_acc, bool final, float c1, float c2) {
+  // as many lanes per row as keep the CTA's threads busy in one pass
+  if (rows <= kClThreads / 16) cl_step_g<16>(sm, L, r0, rows, mode, v, out, o_acc, final, c1, c2);
+  else if (rows <= kClThreads / 8) cl_step_g<8>(sm, L, r0, rows, mode, v, out, o_acc, final, c1, c2);
+  else cl_step_g<4>(sm, L, r0, rows, mode, v, out, o_acc, final, c1, c2);
+}
+
+// asynchronous global -> shared copies of n 4-byte words (8: n even, both ends 8-byte aligned)
+__device__ __forceinline__ void cl_stage8(unsigned dst, const void *src, int n) {
+  const char *s = static_cast<const char *>(src);
+  for (int i = threadIdx.x; i < n / 2; i += blockDim.x)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8 * i), "l"(s + 8ll * i) : "memory");
+}
+__device__ __forceinline__ void cl_stage4(unsigned dst, const void *src, int n) {
+  const char *s = static_cast<const char *>(src);
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * i), "l"(s + 4ll * i) : "memory");
+}
+
+__global__ void __launch_bounds__(kClThreads, 1)
+k_mgc_cluster(const __grid_constant__ MgClArgs a, const PcgState *__restrict__ st) {
+  extern __shared__ __align__(16) char sm[];
+  __shared__ float s_coef[kMgClusterLevels * kMgCoef];
+  const unsigned rank = cl_rank();
+  const unsigned smb = (unsigned)__cvta_generic_to_shared(sm);
+  const int last = a.nlev - 1;
+  // Stage the operators. They were written by the set-up launches, which are
+  // complete: this kernel starts at the earliest when its predecessor's own
+  // wait has returned.
+  for (int i = threadIdx.x; i < a.nlev * kMgCoef; i += blockDim.x) s_coef[i] = a.coef[kMgCoef * a.first + i];
+  for (int l = 0; l < a.nlev; ++l) {
+    const MgClLevel &L = a.lv[l];
+    const int r0 = L.split[rank], nr = L.split[rank + 1] - r0, k0 = L.bsplit[rank], nk = L.bsplit[rank + 1] - k0;
+    if (l == last && a.last_mode == kMgLastDense) {
+      cl_stage8(smb + L.o_val, a.ainv + 6ll * r0 * a.nd, 6 * nr * a.nd);
+    } else {
+      cl_stage8(smb + L.o_val, L.val16 + 36ll * k0, 18 * nk);
+      cl_stage8(smb + L.o_dinv, L.dinv + 36ll * r0, 36 * nr);
+      cl_stage4(smb + L.o_ci, L.ci + k0, nk);
+      cl_stage4(smb + L.o_rp, L.rp + r0, nr + 1);
+    }
+    if (l < last) {
+      cl_stage8(smb + L.o_Q, L.Q + 36ll * r0, 36 * nr);
+      cl_stage4(smb + L.o_agg, L.agg + r0, nr);
+    }
+    if (l > 0) {
+      const int m0 = L.msplit[rank];
+      cl_stage4(smb + L.o_mptr, L.mptr + r0, nr + 1);
+      cl_stage4(smb + L.o_mem, L.midx + m0, L.msplit[rank + 1] - m0);
+    }
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
   pdl_wait();
   pdl_trigger();
-  if (st && st->done) return;
-  __shared__ float sb[6 * kDenseNodes];
-  for (int i = threadIdx.x; i < nd; i += blockDim.x) sb[i] = __ldcg(b + i);
-  __syncthreads();
-  for (int i = threadIdx.x; i < nd; i += blockDim.x) {
-    float s = 0.f;
-    for (int j = 0; j < nd; ++j) s += __ldg(ainv + (int64_t)i * nd + j) * sb[j];
-    x[i] = s;
+  if (st && st->done) return;  // the same for every CTA: nothing writes the flag while this kernel runs
+
+  auto F = [&](int o) { return reinterpret_cast<float *>(sm + o); };
+  const int lane = threadIdx.x & 31;
+  // ---- down
+  const float *t_fine = nullptr;  // the finer level's shares of the restriction
+  for (int l = 0; l <= last; ++l) {
+    const MgClLevel &L = a.lv[l];
+    const int r0 = L.split[rank], rows = L.split[rank + 1] - r0;
+    const bool dense = l == last && a.last_mode == kMgLastDense;
+    const bool exact = l == last && a.last_mode == kMgLastExact;
+    const float *cf = s_coef + kMgCoef * l;
+    // right-hand side and first step from x = 0: x = d = c0 Dinv b, r = b. One warp per node.
+    for (int i = threadIdx.x >> 5; i < rows; i += blockDim.x >> 5) {
+      const int c = lane & 7;
+      float bv = 0.f;
+      if (l == 0) {
+        if (c < 6) bv = __ldcg(L.gb + 6 * (r0 + i) + c);
+      } else {
+        const int *mp = reinterpret_cast<const int *>(sm + L.o_mptr);
+        const int *mem = reinterpret_cast<const int *>(sm + L.o_mem);
+        if (c < 6)
+#pragma unroll 4
+          for (int m = mp[i] - mp[0] + (lane >> 3); m < mp[i + 1] - mp[0]; m += 4)
+            bv += __ldcg(t_fine + 6 * mem[m] + c);
+        bv += __shfl_xor_sync(0xffffffffu, bv, 8);
+        bv += __shfl_xor_sync(0xffffffffu, bv, 16);
+      }
+      float bb[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) bb[k] = __shfl_sync(0xffffffffu, bv, k);
+      if (lane < 6) {
+        const int e = 6 * i + lane;
+        if (dense) {
+          L.gb[6 * r0 + e] = bv;
+        } else {
+          const float *m = F(L.o_dinv) + 36 * i + 6 * lane;
+          float z = 0.f;
+#pragma unroll
+          for (int k = 0; k < 6; ++k) z += m[k] * bb[k];
+          const float xv = exact ? z : cf[0] * z;
+          F(L.o_b)[e] = bv;
+          F(L.o_x)[e] = xv;
+          F(L.o_r)[e] = bv;
+          F(L.o_d)[e] = xv;
+          (l == last && (exact || L.deg == 1) ? L.gres : L.gd)[6 * r0 + e] = xv;
+        }
+      }
+    }
+    cl_barrier();
+    if (dense) {
+      // x = Ainv b: every CTA gathers b, then one warp per row of its own nodes
+      float *db = F(a.o_db);
+      for (int j = threadIdx.x; j < a.nd; j += blockDim.x) db[j] = __ldcg(L.gb + j);
+      __syncthreads();
+      for (int i = threadIdx.x >> 5; i < 6 * rows; i += blockDim.x >> 5) {
+        const float *m = F(L.o_val) + i * a.nd;
+        float s = 0.f;
+        for (int j = lane; j < a.nd; j += 32) s += m[j] * db[j];
+        s = warp_sumf(s);
+        if (lane == 0) L.gres[6 * r0 + i] = s;
+      }
+      cl_barrier();
+      break;
+    }
+    if (exact) break;
+    float *din = L.gd, *dout = L.gd2;
+    for (int j = 1; j < L.deg; ++j) {
+      const bool fin = l == last && j + 1 == L.deg;
+      cl_step(sm, L, r0, rows, kStepCheb, din, fin ? L.gres : dout, L.o_x, fin, cf[2 * j - 1], cf[2 * j]);
+      cl_barrier();
+      float *t = din;
+      din = dout;
+      dout = t;
+    }
+    if (l < last) {
+      cl_step(sm, L, r0, rows, kStepResid, din, dout, L.o_x, false, 0.f, 0.f);
+      t_fine = dout;
+      cl_barrier();
+    }
+  }
+  // ---- up
+  for (int l = last - 1; l >= 0; --l) {
+    const MgClLevel &L = a.lv[l];
+    const int r0 = L.split[rank], rows = L.split[rank + 1] - r0;
+    const float *cf = s_coef + kMgCoef * l;
+    const int *agg = reinterpret_cast<const int *>(sm + L.o_agg);
+    const float *xc = a.lv[l + 1].gres;
+    for (int e = threadIdx.x; e < 6 * rows; e += blockDim.x) {  // x += Q x_c
+      float c[6];
+      ldcg6(xc, agg[e / 6], c);
+      const float *q = F(L.o_Q) + 6 * e;
+      float s = 0.f;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s += q[k] * c[k];
+      s += F(L.o_x)[e];
+      F(L.o_x)[e] = s;
+      L.gx[6 * r0 + e] = s;
+    }
+    cl_barrier();
+    cl_step(sm, L, r0, rows, kStepPost, L.gx, L.deg == 1 ? L.gres : L.gd, L.o_b, L.deg == 1, 0.f, cf[0]);
+    float *din = L.gd, *dout = L.gd2;
+    for (int j = 1; j < L.deg; ++j) {
+      cl_barrier();
+      const bool fin = j + 1 == L.deg;
+      cl_step(sm, L, r0, rows, kStepCheb, din, fin ? L.gres : dout, L.o_b, fin, cf[2 * j - 1], cf[2 * j]);
+      float *t = din;
+      din = dout;
+      dout = t;
+    }
+    if (l > 0) cl_barrier();
   }
 }
 
@@ -1370,7 +1835,7 @@ int restrict_into(bartels_ctx ctx, MgHierarchy *mg, const MgLevel &f, const floa
                   bool *first_done) {
   MgLevel &c = mg->lv[l];
   const bool last = l + 1 == (int)mg->lv.size();
-  const bool fuse = !(last && mg->dense);
+  const bool fuse = !(mg->cl.ctas && l == mg->cl.first);  // the cluster kernel takes the first step itself
   const bool exact = last && mg->coarse_blockdiag;  // x = Dinv b
   const float *coef = exact ? nullptr : mg->coef + kMgCoef * l;
   const int g = grid_rows(ctx, (c.n + 3) / 4, 32);
@@ -1384,14 +1849,27 @@ int restrict_into(bartels_ctx ctx, MgHierarchy *mg, const MgLevel &f, const floa
   return BARTELS_OK;
 }
 
+int launch_cluster(bartels_ctx ctx, MgHierarchy *mg, const PcgState *st) {
+  const MgClArgs &a = mg->cl;
+  cudaLaunchAttribute at[2];
+  cudaLaunchConfig_t cfg = cluster_config(ctx, a.ctas, kClThreads, a.smem, at);
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mgc_cluster, a, st);
+  ctx->launches++;
+  if (e != cudaSuccess) return fail(BARTELS_E_DEVICE, std::string("launch k_mgc_cluster: ") + cudaGetErrorString(e));
+  return BARTELS_OK;
+}
+
 int enqueue_coarse(bartels_ctx ctx, MgHierarchy *mg, int l, bool first_done, const PcgState *st) {
+  if (mg->cl.ctas && l == mg->cl.first) return launch_cluster(ctx, mg, st);
   MgLevel &c = mg->lv[l];
   const float *coef = mg->coef + kMgCoef * l;
   const int last = (int)mg->lv.size() - 1;
   if (l == last) {
-    if (mg->dense) {
-      BT_LAUNCH_PDL(ctx, k_mg_dense_apply, 1, 256, 0, mg->nd, mg->ainv, c.b, c.x, st);
-    } else if (mg->coarse_blockdiag) {
+    // (a dense coarsest level is always part of the cluster launch)
+    if (mg->coarse_blockdiag) {
       if (!first_done)
         BT_LAUNCH_PDL(ctx, k_mgc_first, grid_n(ctx, c.n), 256, 0, c.n, c.dinv, c.b, c.x, (float *)nullptr,
                   (float *)nullptr, (const float *)nullptr, st);
@@ -1503,9 +1981,24 @@ int mg_setup_numeric(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
   }
   if (mg->dense) {
     const MgLevel &c = mg->lv[L - 1];
-    const size_t smem = sizeof(float) * mg->nd * mg->nd;
-    BT_CUDA(cudaFuncSetAttribute(k_mg_dense_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    BT_LAUNCH(ctx, k_mg_dense_inv, 1, 1024, smem, c.n, c.rp, c.ci, c.val, mg->ainv);
+    MgInvArgs ia;
+    ia.nodes = c.n;
+    ia.rp = c.rp;
+    ia.ci = c.ci;
+    ia.rev = c.rev;
+    ia.dpos = c.dpos;
+    ia.val = c.val;
+    ia.panel = mg->panel;
+    ia.ainv = mg->ainv;
+    const int ctas = std::min(c.n, 8), per = (c.n + ctas - 1) / ctas;
+    for (int q = 0; q <= kMgClusterMax; ++q) ia.split[q] = std::min(c.n, q * per);
+    const int smem = (int)sizeof(float) * (6 * per + 6) * mg->nd;
+    BT_CUDA(cudaFuncSetAttribute(k_mg_dense_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = cluster_config(ctx, ctas, kInvThreads, smem, at);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mg_dense_inv, ia);
+    ctx->launches++;
+    if (e != cudaSuccess) return fail(BARTELS_E_DEVICE, std::string("launch k_mg_dense_inv: ") + cudaGetErrorString(e));
   }
   // largest eigenvalue of M A on every smoothed level (power iteration; per
   // segment on the finest level of a packed plan)

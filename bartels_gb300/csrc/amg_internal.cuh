@@ -42,6 +42,35 @@ struct MgLevel {
 
 constexpr int kMgMaxLevels = 12;
 constexpr int kMgCoef = 16;  // per level: 1/theta, then (c1, c2) per further Chebyshev step
+constexpr int kMgClusterMax = 16;  // CTAs of the coarse-cycle cluster
+
+constexpr int kMgClusterLevels = 8;
+
+// One level as the coarse-cycle kernel sees it: its nodes split into
+// contiguous ranges, one per CTA of the cluster (split: first node, bsplit:
+// first block, msplit: first member-list entry of each range). The o_* are
+// byte offsets of the level's areas in a CTA's shared memory, sized for the
+// largest range; g* are the level's vectors in global memory, for the entries
+// that other CTAs read.
+struct MgClLevel {
+  int deg = 1;
+  int split[kMgClusterMax + 1] = {}, bsplit[kMgClusterMax + 1] = {}, msplit[kMgClusterMax + 1] = {};
+  const int *rp = nullptr, *ci = nullptr;
+  const int *mptr = nullptr, *midx = nullptr;  // members (finer nodes) of each node, none on the first level
+  const int *agg = nullptr;                    // aggregate of each node (none on the last level)
+  const __nv_bfloat16 *val16 = nullptr;
+  const float *dinv = nullptr, *Q = nullptr;
+  float *gb = nullptr, *gx = nullptr, *gd = nullptr, *gd2 = nullptr, *gres = nullptr;
+  int o_val = 0, o_ci = 0, o_rp = 0, o_dinv = 0, o_Q = 0, o_agg = 0, o_mptr = 0, o_mem = 0;
+  int o_b = 0, o_x = 0, o_r = 0, o_d = 0;
+};
+enum { kMgLastDense = 0, kMgLastExact = 1, kMgLastCheb = 2 };
+struct MgClArgs {
+  int nlev = 0, first = 0, ctas = 0, last_mode = 0, nd = 0, smem = 0;
+  int o_db = 0;  // the coarsest right-hand side gathered by every CTA (dense)
+  const float *ainv = nullptr, *coef = nullptr;
+  MgClLevel lv[kMgClusterLevels];  // lv[0] is hierarchy level `first`
+};
 
 struct MgHierarchy {
   std::vector<MgLevel> lv;
@@ -49,6 +78,7 @@ struct MgHierarchy {
   int nd = 0;             // dense size (6 x nodes of the coarsest level)
   int coarse_blockdiag = 0;  // coarsest level is block diagonal: its block-Jacobi solve is exact
   float *ainv = nullptr;  // nd x nd
+  float *panel = nullptr; // 2 x 6 x nd: pivot rows of the dense inversion
   float *coef = nullptr;  // kMgMaxLevels x kMgCoef Chebyshev coefficients (device)
   double *norms = nullptr;  // 2 per level: squared norms of the last two power iterates
   double *part = nullptr;   // reduction partials
@@ -65,6 +95,8 @@ struct MgHierarchy {
   // one 8-byte load.
   __nv_bfloat16 *a16 = nullptr;
   int *a16_off = nullptr;
+  // levels first .. last as one kernel of one thread-block cluster (ctas == 0: not used)
+  MgClArgs cl;
   std::vector<void *> allocs;
   ~MgHierarchy();
 };
