@@ -37,14 +37,13 @@
 // below). The smoother of level 0 is block-Jacobi or the learned factor
 // M = G^T G (the network's output on the Hessian's lower block pattern). The
 // smoothing passes read exactly symmetric BF16 copies of the operators (the
-// fine one in padded rows); the Galerkin products use the FP32 values. The
+// fine one in the sliced-ELL layout); the Galerkin products use the FP32 values. The
 // levels that fit the shared memory of one thread-block cluster run as one
 // kernel (k_mgc_cluster). Every kernel becomes a no-op once the PCG's
 // convergence flag is set, so fixed-length CUDA graphs of PCG iterations can
 // contain it.
 #include <algorithm>
 #include <climits>
-#include <type_traits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -52,6 +51,7 @@
 #include "amg_internal.cuh"
 #include "lpcg_internal.cuh"
 #include "pcg_common.cuh"
+#include "sell.cuh"
 
 namespace bartels {
 
@@ -579,16 +579,9 @@ int mg_prepare(bartels_ctx ctx, bartels_mesh_plan plan) {
     if (l > 0) BT_CHECK(dalloc_n(mg, &d.d2, nv));
   }
   if (env_int("BARTELS_MG_FINE_BF16", 1, 0, 1)) {
-    std::vector<int> off(plan->nV + 1, 0);
-    for (int v = 0; v < plan->nV; ++v) {
-      const int64_t next = off[v] + 3ll * padded_row(plan->h_brp[v + 1] - plan->h_brp[v]);
-      if (next > INT_MAX) return fail(BARTELS_E_UNSUPPORTED, "multigrid: BF16 copy larger than 2^31 entries");
-      off[v + 1] = (int)next;
-    }
-    BT_CHECK(upload(mg, &mg->a16_off, off));
-    BT_CHECK(dalloc_n(mg, &mg->a16, (size_t)off[plan->nV] + 4));
-    // the pads stay zero (the conversion writes only the entries)
-    BT_CUDA(cudaMemset(mg->a16, 0, sizeof(__nv_bfloat16) * ((size_t)off[plan->nV] + 4)));
+    SellPattern *sp;
+    BT_CHECK(plan_sell(plan, &sp));
+    BT_CHECK(dalloc_n(mg, &mg->a16, 288 * (size_t)std::max<int64_t>(sp->groups, 1)));
   }
   if (mg->dense) {
     mg->nd = 6 * mg->lv.back().n;
@@ -1031,111 +1024,67 @@ k_mg0_update(int nV, const float *__restrict__ pa, const float *__restrict__ pb,
   }
 }
 
-// BF16 copy of the finest level's values for the V-cycle's SpMVs, exactly
-// symmetric: entry (3v+k, 3w+l) of block p = (v, w) and entry (3w+l, 3v+k) of
-// its transpose q = rev[p] both take bf16((A_p(k,l) + A_q(l,k)) / 2). One warp
-// per vertex row, one lane per block.
-__global__ void __launch_bounds__(256)
-k_mg0_to_bf16(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const int *__restrict__ rev,
-              const float *__restrict__ val, const int *__restrict__ a16_off, __nv_bfloat16 *__restrict__ a16) {
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int v = warp; v < nV; v += nwarps) {
-    const int rb = brp[v], nb = brp[v + 1] - rb, rs = 3 * nb, rsp = padded_row(nb);
-    __nv_bfloat16 *out = a16 + __ldg(a16_off + v);
-    for (int j = lane; j < nb; j += 32) {
-      const int w = __ldg(bcol + rb + j);
-      const int q = __ldg(rev + rb + j);
-      const int rbw = __ldg(brp + w), rsw = 3 * (__ldg(brp + w + 1) - rbw), jq = q - rbw;
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          const float a = __ldg(val + 9ll * rb + k * rs + 3 * j + l);
-          const float t = __ldg(val + 9ll * rbw + l * rsw + 3 * jq + k);
-          out[k * rsp + 3 * j + l] = __float2bfloat16_rn(0.5f * (a + t));
-        }
-    }
-  }
-}
-
-// One row of the finest level: the FP32 values in the plan's layout
-// (off == nullptr), or the padded BF16 copy (4 values per 8-byte load).
-template <int G, class VT, class XV>
-__device__ __forceinline__ void row0_acc(int v, int sl, const int *__restrict__ brp, const int *__restrict__ bcol,
-                                         const VT *__restrict__ val, const int *__restrict__ off, XV &&xval,
-                                         float &s0, float &s1, float &s2) {
-  if constexpr (std::is_same<VT, __nv_bfloat16>::value) {
-    const int rb = __ldg(brp + v), nb = __ldg(brp + v + 1) - rb;
-    tri_row_acc4<G>(sl, bcol + rb, val + __ldg(off + v), 3 * nb, padded_row(nb), xval, s0, s1, s2);
-  } else {
-    spmv_row_acc<G>(v, sl, brp, bcol, val, xval, s0, s1, s2);
-  }
-}
-
 // out = b - A x, or A x without b (rows of pinned vertices give 0)
-template <int G, class VT>
+__device__ __forceinline__ void mg0_resid_row(int v, const float *s, const float *b, float *out,
+                                              const unsigned char *pinned) {
+  const bool pin = pinned && pinned[v];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float t = b ? __ldcg(b + 3 * v + k) - s[k] : s[k];
+    out[3 * v + k] = pin ? 0.f : t;
+  }
+}
+
+// over the values' own layout, G lanes per row
+template <int G>
 __global__ void __launch_bounds__(256)
-k_mg0_resid(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const VT *__restrict__ val,
-            const int *__restrict__ off, const float *__restrict__ b, const float *__restrict__ x,
-            float *__restrict__ out, const unsigned char *__restrict__ pinned, const PcgState *__restrict__ st) {
+k_mg0_resid(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const float *__restrict__ val,
+            const float *__restrict__ b, const float *__restrict__ x, float *__restrict__ out,
+            const unsigned char *__restrict__ pinned, const PcgState *__restrict__ st) {
   pdl_wait();
   pdl_trigger();
   if (st && st->done) return;
   BT_ROW_LOOP_BEGIN(G)
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  if (active) row0_acc<G>(v, sl, brp, bcol, val, off, [&](int c) { return __ldcg(x + c); }, s0, s1, s2);
-  group_reduce<G>(s0, s1, s2);
-  if (active && sl == 0) {
-    if (b) {
-      s0 = __ldcg(b + 3 * v) - s0;
-      s1 = __ldcg(b + 3 * v + 1) - s1;
-      s2 = __ldcg(b + 3 * v + 2) - s2;
-    }
-    if (pinned && pinned[v]) s0 = s1 = s2 = 0.f;
-    out[3 * v] = s0;
-    out[3 * v + 1] = s1;
-    out[3 * v + 2] = s2;
-  }
+  float s[3] = {0.f, 0.f, 0.f};
+  if (active) spmv_row_acc<G>(v, sl, brp, bcol, val, [&](int c) { return __ldcg(x + c); }, s[0], s[1], s[2]);
+  group_reduce<G>(s[0], s[1], s[2]);
+  if (active && sl == 0) mg0_resid_row(v, s, b, out, pinned);
   BT_ROW_LOOP_END
+}
+
+// over the sliced-ELL BF16 copy (bound by HBM: 18 B of values and 4 B of column per block)
+template <int S>
+__global__ void __launch_bounds__(256)
+k_mg0_resid_sell(SellView sv, const uint2 *__restrict__ val, const float *__restrict__ b, const float *x,
+                 float *__restrict__ out, const unsigned char *__restrict__ pinned, const PcgState *__restrict__ st) {
+  pdl_wait();
+  pdl_trigger();
+  if (st && st->done) return;
+  sell_pass<S>(sv, val, x, [&](int v, float *s) { mg0_resid_row(v, s, b, out, pinned); });
 }
 
 // Final step of the V-cycle with the block-Jacobi smoother:
 // z = x + c Dinv (b - A x), partial sums of b.z; the last block stores r.z
 // and beta = r.z / r.z_old in the PCG state.
-template <int G, class VT>
-__global__ void __launch_bounds__(256)
-k_mg0_post_bj(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const VT *__restrict__ val,
-              const int *__restrict__ off, const float *__restrict__ minv, const float *__restrict__ b,
-              const float *__restrict__ x, float *__restrict__ z, const unsigned char *__restrict__ pinned,
-              const float *__restrict__ coef, double *__restrict__ part, PcgState *__restrict__ st) {
-  pdl_wait();
-  pdl_trigger();
-  if (st->done) return;
-  const float c = coef[0];
-  float acc = 0.f;
-  BT_ROW_LOOP_BEGIN(G)
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  if (active) row0_acc<G>(v, sl, brp, bcol, val, off, [&](int cc) { return __ldcg(x + cc); }, s0, s1, s2);
-  group_reduce<G>(s0, s1, s2);
-  if (active && sl == 0) {
-    float bv[3], rv[3], zv[3];
+__device__ __forceinline__ float mg0_post_row(int v, const float *s, const float *minv, const float *b, const float *x,
+                                              float *z, const unsigned char *pinned, float c) {
+  float bv[3], rv[3], zv[3], acc = 0.f;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) bv[k] = __ldcg(b + 3 * v + k);
-    rv[0] = bv[0] - s0;
-    rv[1] = bv[1] - s1;
-    rv[2] = bv[2] - s2;
-    apply_minv(minv, v, rv, zv);
-    const bool pin = pinned && pinned[v];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float zk = pin ? 0.f : __ldcg(x + 3 * v + k) + c * zv[k];
-      z[3 * v + k] = zk;
-      acc += bv[k] * zk;
-    }
+  for (int k = 0; k < 3; ++k) {
+    bv[k] = __ldcg(b + 3 * v + k);
+    rv[k] = bv[k] - s[k];
   }
-  BT_ROW_LOOP_END
+  apply_minv(minv, v, rv, zv);
+  const bool pin = pinned && pinned[v];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float zk = pin ? 0.f : __ldcg(x + 3 * v + k) + c * zv[k];
+    z[3 * v + k] = zk;
+    acc += bv[k] * zk;
+  }
+  return acc;
+}
+__device__ __forceinline__ void finish_rz(float acc, double *__restrict__ part, PcgState *__restrict__ st) {
   double s = cta_sum_f(acc);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
   if (last_block(&st->count)) {
@@ -1146,6 +1095,39 @@ k_mg0_post_bj(int nV, const int *__restrict__ brp, const int *__restrict__ bcol,
       st->count = 0;
     }
   }
+}
+template <int G>
+__global__ void __launch_bounds__(256)
+k_mg0_post_bj(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const float *__restrict__ val,
+              const float *__restrict__ minv, const float *__restrict__ b, const float *__restrict__ x,
+              float *__restrict__ z, const unsigned char *__restrict__ pinned, const float *__restrict__ coef,
+              double *__restrict__ part, PcgState *__restrict__ st) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->done) return;
+  const float c = coef[0];
+  float acc = 0.f;
+  BT_ROW_LOOP_BEGIN(G)
+  float s[3] = {0.f, 0.f, 0.f};
+  if (active) spmv_row_acc<G>(v, sl, brp, bcol, val, [&](int cc) { return __ldcg(x + cc); }, s[0], s[1], s[2]);
+  group_reduce<G>(s[0], s[1], s[2]);
+  if (active && sl == 0) acc += mg0_post_row(v, s, minv, b, x, z, pinned, c);
+  BT_ROW_LOOP_END
+  finish_rz(acc, part, st);
+}
+template <int S>
+__global__ void __launch_bounds__(256)
+k_mg0_post_bj_sell(SellView sv, const uint2 *__restrict__ val, const float *__restrict__ minv,
+                   const float *__restrict__ b, const float *x, float *__restrict__ z,
+                   const unsigned char *__restrict__ pinned, const float *__restrict__ coef,
+                   double *__restrict__ part, PcgState *__restrict__ st) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->done) return;
+  const float c = coef[0];
+  float acc = 0.f;
+  sell_pass<S>(sv, val, x, [&](int v, float *s) { acc += mg0_post_row(v, s, minv, b, x, z, pinned, c); });
+  finish_rz(acc, part, st);
 }
 
 // y = G r (learned factor, lower rows; pinned rows give 0)
@@ -1209,17 +1191,7 @@ k_mg0_fac_upper(int nV, const int4 *__restrict__ meta, const int *__restrict__ b
     }
   }
   BT_ROW_LOOP_END
-  if (!part) return;
-  double s = cta_sum_f(acc);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-  if (last_block(&st->count)) {
-    const double rz = sum_partials(part, gridDim.x);
-    if (threadIdx.x == 0) {
-      st->beta = (float)(rz / st->rz);
-      st->rz = rz;
-      st->count = 0;
-    }
-  }
+  if (part) finish_rz(acc, part, st);
 }
 
 // BF16 copy of a coarse level, exactly symmetric: block k gets
@@ -1931,19 +1903,17 @@ int fac_upper(bartels_ctx ctx, bartels_mesh_plan plan, const MgSmoother &sm, con
 // out = b - A x on the finest level, with the V-cycle's BF16 copy of A when it has one
 int resid0(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const float *b, const float *x, float *out,
            const PcgState *st) {
-  using B16 = __nv_bfloat16;
-  const B16 *a16 = plan->mg ? plan->mg->a16 : nullptr;
+  const uint2 *a16 = plan->mg ? plan->mg->a16 : nullptr;
   if (a16) {
-    // padded BF16 rows: the factor passes' lane count (4 values per lane step)
-    const int G = plan_lanes_tri(ctx, plan);
-    const int g = grid_rows(ctx, plan->nV, G);
-    BT_MG_G(G, BT_LAUNCH_PDL(ctx, (k_mg0_resid<GL, B16>), g, 256, 0, plan->nV, plan->brp, plan->bcol, a16,
-                             (const int *)plan->mg->a16_off, b, x, out, plan->pinned, st));
+    const SellView sv = plan->sell->view();
+    const int S = sell_split(ctx, sv.nslices), g = sell_grid(ctx, sv.nslices, S);
+    if (S == 1) BT_LAUNCH_PDL(ctx, k_mg0_resid_sell<1>, g, 256, 0, sv, a16, b, x, out, plan->pinned, st);
+    else BT_LAUNCH_PDL(ctx, k_mg0_resid_sell<4>, g, 256, 0, sv, a16, b, x, out, plan->pinned, st);
   } else {
     const int G = plan_lanes_spmv(ctx, plan);
     const int g = grid_rows(ctx, plan->nV, G);
-    BT_MG_G(G, BT_LAUNCH_PDL(ctx, (k_mg0_resid<GL, float>), g, 256, 0, plan->nV, plan->brp, plan->bcol, values,
-                             (const int *)nullptr, b, x, out, plan->pinned, st));
+    BT_MG_G(G, BT_LAUNCH_PDL(ctx, k_mg0_resid<GL>, g, 256, 0, plan->nV, plan->brp, plan->bcol, values, b, x, out,
+                             plan->pinned, st));
   }
   return BARTELS_OK;
 }
@@ -1965,8 +1935,7 @@ int mg_setup_numeric(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
   if (mg->a16) {
     FactorPattern *fp = nullptr;
     BT_CHECK(plan_factor_pattern(plan, &fp));
-    BT_LAUNCH(ctx, k_mg0_to_bf16, grid_rows(ctx, plan->nV, 32), 256, 0, plan->nV, plan->brp, plan->bcol, fp->rev,
-              values, (const int *)mg->a16_off, mg->a16);
+    BT_CHECK(sell_fill_bf16(ctx, plan, values, fp->rev, mg->a16));
   }
   for (int l = 0; l + 1 < L; ++l) {
     MgLevel &f = mg->lv[l], &c = mg->lv[l + 1];
@@ -2075,18 +2044,19 @@ int mg_enqueue_apply(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
     BT_CHECK(fac_lower(ctx, plan, sm, l0.r, y, st));
     BT_CHECK(fac_upper(ctx, plan, sm, y, l0.x, z, c0, r, part, st));
   } else {
-    using B16 = __nv_bfloat16;
     if (mg->a16) {
-      const int G = plan_lanes_tri(ctx, plan);
-      const int g = grid_rows(ctx, nV, G);
-      BT_MG_G(G, BT_LAUNCH_PDL(ctx, (k_mg0_post_bj<GL, B16>), g, 256, 0, nV, plan->brp, plan->bcol,
-                               (const B16 *)mg->a16, (const int *)mg->a16_off, sm.minv, r, l0.x, z, plan->pinned, c0,
-                               part, st));
+      const SellView sv = plan->sell->view();
+      const int S = sell_split(ctx, sv.nslices), g = sell_grid(ctx, sv.nslices, S);
+      const uint2 *a16 = mg->a16;
+      if (S == 1)
+        BT_LAUNCH_PDL(ctx, k_mg0_post_bj_sell<1>, g, 256, 0, sv, a16, sm.minv, r, l0.x, z, plan->pinned, c0, part, st);
+      else
+        BT_LAUNCH_PDL(ctx, k_mg0_post_bj_sell<4>, g, 256, 0, sv, a16, sm.minv, r, l0.x, z, plan->pinned, c0, part, st);
     } else {
       const int G = plan_lanes_spmv(ctx, plan);
       const int g = grid_rows(ctx, nV, G);
-      BT_MG_G(G, BT_LAUNCH_PDL(ctx, (k_mg0_post_bj<GL, float>), g, 256, 0, nV, plan->brp, plan->bcol, values,
-                               (const int *)nullptr, sm.minv, r, l0.x, z, plan->pinned, c0, part, st));
+      BT_MG_G(G, BT_LAUNCH_PDL(ctx, k_mg0_post_bj<GL>, g, 256, 0, nV, plan->brp, plan->bcol, values, sm.minv, r, l0.x, z,
+                               plan->pinned, c0, part, st));
     }
   }
   return BARTELS_OK;

@@ -88,13 +88,9 @@ struct MgHierarchy {
   PcgState *st_once = nullptr;  // state for a single application outside PCG
   double *segn = nullptr;       // per-segment norms of the finest level's last two power iterates
   int segn_n = 0;
-  // BF16 copy of the finest level's values, made exactly symmetric, for the
-  // V-cycle's own SpMVs (nullptr: the FP32 values are used). Vertex v's three
-  // scalar rows start at a16_off[v] and are each padded with zeros to
-  // padded_row(nb) entries (a multiple of 4), so a lane reads 4 values with
-  // one 8-byte load.
-  __nv_bfloat16 *a16 = nullptr;
-  int *a16_off = nullptr;
+  // BF16 copy of the finest level's values in the sliced-ELL layout, made exactly
+  // symmetric, for the V-cycle's own SpMVs (nullptr: the FP32 values are used)
+  uint2 *a16 = nullptr;
   // levels first .. last as one kernel of one thread-block cluster (ctas == 0: not used)
   MgClArgs cl;
   std::vector<void *> allocs;

@@ -93,6 +93,7 @@ static_assert(sizeof(TetRec64) == 128, "TetRec64 must be 128 bytes");
 struct FactorPattern;  // lower / upper block storage maps (learned preconditioner)
 struct LpcgPlanState;  // per-plan buffers of the learned preconditioner
 struct MgHierarchy;    // aggregation multigrid hierarchy of a plan
+struct SellPattern;    // sliced-ELL layout of a plan's block rows
 
 // Packed meshes: the plan's vertices and tets as independent segments
 // (instances), each with its own PCG scalars and line-search step.
@@ -178,11 +179,9 @@ struct bartels_mesh_plan_s {
   int nchunks = 0;
   // half-size chunks (<= 64 vertices, 32 KB), made when the tuning asks for them
   int *chunk_v64 = nullptr;
-  // padded copy of the FP32 values for the PCG loop's SpMV: vertex v's three
-  // scalar rows start at pad_off[v] (pad_total entries in all), each padded
-  // with zeros to a multiple of 4 entries; w_vpad holds the copy
-  int *pad_off = nullptr;
-  int64_t pad_total = 0;
+  // sliced-ELL layout of the block rows (built on the first solve); w_sell holds
+  // the FP32 values in it for the PCG loop's SpMV
+  bartels::SellPattern *sell = nullptr;
   int nchunks64 = 0;
   // Hessian tuning: vertices per assembly CTA (128, or 64 with chunk_v64) and
   // threads per CTA of the PSD pre-pass kernels (64, 128 or 256)
@@ -209,7 +208,7 @@ struct bartels_mesh_plan_s {
   // packed-mesh segments (nullptr: one system)
   bartels::SegInfo *seg = nullptr;
   // solver workspace
-  bartels::DevBuf w_values, w_minv, w_vec, w_grad_e, w_energy, w_u, w_pcg, w_psd, w_spmv, w_vpad;
+  bartels::DevBuf w_values, w_minv, w_vec, w_grad_e, w_energy, w_u, w_pcg, w_psd, w_spmv, w_sell;
 };
 
 namespace bartels {

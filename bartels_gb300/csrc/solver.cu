@@ -25,6 +25,7 @@
 #include "amg_internal.cuh"
 #include "lpcg_internal.cuh"
 #include "pcg_common.cuh"
+#include "sell.cuh"
 
 namespace bartels {
 
@@ -230,40 +231,8 @@ k_pcg_dir(int n, const float *__restrict__ z, float *__restrict__ pa, float *__r
     p_new[i] = z[i] + beta * p_old[i];
 }
 
-// ap = A p (block layout), partials of p.Ap; alpha in the last block. PAD:
-// val is the padded copy of the values (rows at off[v], 4 per 16-byte load),
-// otherwise the plan's own layout.
-template <int G, bool PAD>
-__global__ void __launch_bounds__(256)
-k_pcg_spmv_blk(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const float *__restrict__ val,
-               const int *__restrict__ off, const float *__restrict__ pa, const float *__restrict__ pb,
-               float *__restrict__ ap, const unsigned char *__restrict__ pinned, double *__restrict__ part,
-               PcgState *__restrict__ st) {
-  pdl_wait();
-  pdl_trigger();
-  if (st->done) return;
-  const float *p = (st->it & 1) ? pb : pa;
-  float acc = 0.f;
-  BT_ROW_LOOP_BEGIN(G)
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  if (active) {
-    if constexpr (PAD) {
-      const int rb = __ldg(brp + v), nb = __ldg(brp + v + 1) - rb;
-      row_acc4f<G>(sl, bcol + rb, val + __ldg(off + v), 3 * nb, padded_row(nb), [&](int c) { return __ldcg(p + c); },
-                   s0, s1, s2);
-    } else {
-      spmv_row_acc<G>(v, sl, brp, bcol, val, [&](int c) { return __ldcg(p + c); }, s0, s1, s2);
-    }
-  }
-  group_reduce<G>(s0, s1, s2);
-  if (active && sl == 0) {
-    if (pinned && pinned[v]) s0 = s1 = s2 = 0.f;
-    ap[3 * v] = s0;
-    ap[3 * v + 1] = s1;
-    ap[3 * v + 2] = s2;
-    acc += __ldcg(p + 3 * v) * s0 + __ldcg(p + 3 * v + 1) * s1 + __ldcg(p + 3 * v + 2) * s2;
-  }
-  BT_ROW_LOOP_END
+// alpha = r.z / p.Ap from the CTAs' partial sums of p.Ap, in the last CTA
+__device__ __forceinline__ void finish_pap(float acc, double *__restrict__ part, PcgState *__restrict__ st) {
   double s = cta_sum_f(acc);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
   if (last_block(&st->count)) {
@@ -276,22 +245,53 @@ k_pcg_spmv_blk(int nV, const int *__restrict__ brp, const int *__restrict__ bcol
   }
 }
 
-// Copy of the values into the padded layout (warp per vertex row); the pads
-// are zeroed when the buffer is allocated and never written.
+// ap = A p over the values' own layout (G lanes per vertex row), partials of p.Ap
+template <int G>
 __global__ void __launch_bounds__(256)
-k_pad_values(int nV, const int *__restrict__ brp, const int *__restrict__ off, const float *__restrict__ val,
-             float *__restrict__ vpad) {
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int v = warp; v < nV; v += nwarps) {
-    const int rb = brp[v], nb = brp[v + 1] - rb, rs = 3 * nb, rsp = padded_row(nb);
-    const float *src = val + 9ll * rb;
-    float *dst = vpad + off[v];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      for (int e = lane; e < rs; e += 32) dst[k * rsp + e] = __ldcs(src + k * rs + e);
+k_pcg_spmv_blk(int nV, const int *__restrict__ brp, const int *__restrict__ bcol, const float *__restrict__ val,
+               const float *__restrict__ pa, const float *__restrict__ pb, float *__restrict__ ap,
+               const unsigned char *__restrict__ pinned, double *__restrict__ part, PcgState *__restrict__ st) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->done) return;
+  const float *p = (st->it & 1) ? pb : pa;
+  float acc = 0.f;
+  BT_ROW_LOOP_BEGIN(G)
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+  if (active) spmv_row_acc<G>(v, sl, brp, bcol, val, [&](int c) { return __ldcg(p + c); }, s0, s1, s2);
+  group_reduce<G>(s0, s1, s2);
+  if (active && sl == 0) {
+    if (pinned && pinned[v]) s0 = s1 = s2 = 0.f;
+    ap[3 * v] = s0;
+    ap[3 * v + 1] = s1;
+    ap[3 * v + 2] = s2;
+    acc += __ldcg(p + 3 * v) * s0 + __ldcg(p + 3 * v + 1) * s1 + __ldcg(p + 3 * v + 2) * s2;
   }
+  BT_ROW_LOOP_END
+  finish_pap(acc, part, st);
+}
+
+// The PCG loop's SpMV, ap = A p over the sliced-ELL copy of the values, and the
+// partials of p.Ap. Bound by HBM (36 B of values and 4 B of column per block).
+template <int S>
+__global__ void __launch_bounds__(256)
+k_pcg_spmv_sell(SellView sv, const float4 *__restrict__ val, const float *pa, const float *pb, float *__restrict__ ap,
+                const unsigned char *__restrict__ pinned, double *__restrict__ part, PcgState *__restrict__ st) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->done) return;
+  const float *p = (st->it & 1) ? pb : pa;
+  float acc = 0.f;
+  sell_pass<S>(sv, val, p, [&](int v, float *s) {
+    const bool pin = pinned && pinned[v];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float t = pin ? 0.f : s[k];
+      ap[3 * v + k] = t;
+      acc += p[3 * v + k] * t;
+    }
+  });
+  finish_pap(acc, part, st);
 }
 
 // ap = A p for a generic scalar CSR (one warp per row), partials of p.Ap.
@@ -738,8 +738,7 @@ struct PcgOperator {
   // block layout (plan)
   bartels_mesh_plan plan = nullptr;
   const float *values = nullptr;
-  const float *vpad = nullptr;    // padded copy of values for the loop's SpMV (nullptr: values' own layout)
-  const int *pad_off = nullptr;
+  const float4 *vsell = nullptr;  // sliced-ELL copy of values for the loop's SpMV (nullptr: values' own layout)
   const unsigned char *pinned = nullptr;
   // generic CSR
   int n = 0;
@@ -813,19 +812,26 @@ static int pcg_enqueue_mg(bartels_ctx ctx, const PcgOperator &op, const PcgWork 
   return BARTELS_OK;
 }
 
-static int pcg_spmv_blk(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w, int lanes, int gs) {
-#define BT_K0(G, PAD, VAL, OFF)                                                                                 \
-  BT_LAUNCH_PDL(ctx, (k_pcg_spmv_blk<G, PAD>), gs, 256, 0, op.plan->nV, op.plan->brp, op.plan->bcol, VAL, OFF, \
-                w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st)
-  if (op.vpad) {
-    if (lanes == 4) BT_K0(4, true, op.vpad, op.pad_off);
-    else if (lanes == 16) BT_K0(16, true, op.vpad, op.pad_off);
-    else BT_K0(8, true, op.vpad, op.pad_off);
-  } else {
-    if (lanes == 4) BT_K0(4, false, op.values, (const int *)nullptr);
-    else if (lanes == 16) BT_K0(16, false, op.values, (const int *)nullptr);
-    else BT_K0(8, false, op.values, (const int *)nullptr);
+// the loop's SpMV: over the sliced-ELL copy, or the values' own layout
+static int pcg_spmv_blk(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w) {
+  const bartels_mesh_plan plan = op.plan;
+  if (op.vsell) {
+    const SellView sv = plan->sell->view();
+    const int S = sell_split(ctx, sv.nslices), g = sell_grid(ctx, sv.nslices, S);
+    if (S == 1)
+      BT_LAUNCH_PDL(ctx, k_pcg_spmv_sell<1>, g, 256, 0, sv, op.vsell, w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st);
+    else
+      BT_LAUNCH_PDL(ctx, k_pcg_spmv_sell<4>, g, 256, 0, sv, op.vsell, w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st);
+    return BARTELS_OK;
   }
+  const int lanes = lanes_spmv(ctx, plan);
+  const int gs = grid_spmv(ctx, (int64_t)plan->nV * lanes / 32 + 1);
+#define BT_K0(G)                                                                                               \
+  BT_LAUNCH_PDL(ctx, k_pcg_spmv_blk<G>, gs, 256, 0, plan->nV, plan->brp, plan->bcol, op.values, w.pa, w.pb, w.ap, \
+                op.pinned, w.part_a, w.st)
+  if (lanes == 4) BT_K0(4);
+  else if (lanes == 16) BT_K0(16);
+  else BT_K0(8);
 #undef BT_K0
   return BARTELS_OK;
 }
@@ -833,14 +839,13 @@ static int pcg_spmv_blk(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w
 static int pcg_enqueue_iters(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w, int n, int nb, int iters) {
   const bool blk = op.plan != nullptr;
   const bool fac = blk && op.gl != nullptr;
-  const int lanes = blk ? lanes_spmv(ctx, op.plan) : 0;
-  const int gs = blk ? grid_spmv(ctx, (int64_t)op.plan->nV * lanes / 32 + 1) : grid_spmv(ctx, n);
+  const int gs = grid_spmv(ctx, n);
   const int gu = grid_vec(ctx, (nb + 3) / 4);
   const int gd = grid_vec(ctx, (n + 3) / 4);
   for (int i = 0; i < iters; ++i) {
     if (op.mg) {
       // p was formed at the end of the previous iteration (or at the start of the solve)
-      BT_CHECK(pcg_spmv_blk(ctx, op, w, lanes, gs));
+      BT_CHECK(pcg_spmv_blk(ctx, op, w));
       if (op.sm.gl) {
         BT_LAUNCH_PDL(ctx, k_pcg_update_f, gd, 256, 0, n, w.pa, w.pb, w.ap, w.x, w.r, w.part_b, w.st);
       } else {
@@ -852,7 +857,7 @@ static int pcg_enqueue_iters(bartels_ctx ctx, const PcgOperator &op, const PcgWo
     // with the factor preconditioner the direction is formed by k_pcg_prec_upper
     if (!fac) BT_LAUNCH_PDL(ctx, k_pcg_dir, gd, 256, 0, n, w.z, w.pa, w.pb, w.st);
     if (blk) {
-      BT_CHECK(pcg_spmv_blk(ctx, op, w, lanes, gs));
+      BT_CHECK(pcg_spmv_blk(ctx, op, w));
     } else {
       BT_LAUNCH_PDL(ctx, k_pcg_spmv_csr, gs, 256, 0, n, op.rp, op.ci, op.values, w.pa, w.pb, w.ap, w.part_a, w.st);
     }
@@ -1313,11 +1318,9 @@ static SegPtrs seg_ptrs(const SegInfo *sg) {
 static int seg_enqueue_iters(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w, const SegPtrs &sp, int iters) {
   const bartels_mesh_plan plan = op.plan;
   const int nV = plan->nV;
-  const int lanes = lanes_spmv(ctx, plan);
-  const int gs = grid_spmv(ctx, (int64_t)nV * lanes / 32 + 1);
   const int gv = grid_vec(ctx, nV);
   for (int i = 0; i < iters; ++i) {
-    BT_CHECK(pcg_spmv_blk(ctx, op, w, lanes, gs));
+    BT_CHECK(pcg_spmv_blk(ctx, op, w));
     BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegPap>, sp.nseg, 256, 0, sp, (const float *)nullptr, w.ap,
                   (const float *)nullptr, (const float *)nullptr, w.pa, w.pb, 0.0, 0, w.st);
     BT_LAUNCH_PDL(ctx, k_seg_update, gv, 256, 0, nV, sp.vseg, sp.alpha, w.pa, w.pb, w.ap, w.x, w.r, w.z,
@@ -1553,10 +1556,8 @@ int plan_set_segments(bartels_mesh_plan plan, int nseg, const int *voff, const i
   return BARTELS_OK;
 }
 
-// The PCG loop's SpMV reads a padded copy of the values (three scalar rows
-// per vertex, each padded with zeros to a multiple of 4 entries, so that a
-// lane reads 4 values with one 16-byte load); the copy is made once per
-// linear solve. BARTELS_PCG_PADDED=0 keeps the values' own layout.
+// The PCG loop's SpMV reads a copy of the values in the sliced-ELL layout, made
+// once per linear solve. BARTELS_PCG_PADDED=0 keeps the values' own layout.
 static bool padded_spmv_enabled() {
   static const bool on = [] {
     const char *e = std::getenv("BARTELS_PCG_PADDED");
@@ -1565,33 +1566,15 @@ static bool padded_spmv_enabled() {
   return on;
 }
 
-static int plan_pad_offsets(bartels_mesh_plan plan) {
-  if (plan->pad_off) return BARTELS_OK;
-  std::vector<int> off(plan->nV + 1, 0);
-  for (int v = 0; v < plan->nV; ++v) {
-    const int64_t next = off[v] + 3ll * padded_row(plan->h_brp[v + 1] - plan->h_brp[v]);
-    if (next > INT_MAX) return fail(BARTELS_E_UNSUPPORTED, "padded values larger than 2^31 entries");
-    off[v + 1] = (int)next;
-  }
-  BT_CUDA(cudaMalloc(&plan->pad_off, sizeof(int) * off.size()));
-  BT_CUDA(cudaMemcpy(plan->pad_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
-  plan->pad_total = off[plan->nV];
-  return BARTELS_OK;
-}
-
-// *out = the padded copy of values (nullptr when the padded SpMV is off)
-static int plan_padded_values(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const float **out) {
+// *out = the sliced-ELL copy of values (nullptr when it is off)
+static int plan_sell_values(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const float4 **out) {
   *out = nullptr;
   if (!padded_spmv_enabled() || !values) return BARTELS_OK;
-  BT_CHECK(plan_pad_offsets(plan));
-  const size_t bytes = sizeof(float) * ((size_t)plan->pad_total + 4);
-  if (plan->w_vpad.bytes < bytes) {
-    BT_CHECK(plan->w_vpad.ensure(bytes));
-    BT_CUDA(cudaMemsetAsync(plan->w_vpad.p, 0, plan->w_vpad.bytes, ctx->stream));
-  }
-  BT_LAUNCH(ctx, k_pad_values, grid_spmv(ctx, plan->nV), 256, 0, plan->nV, plan->brp, (const int *)plan->pad_off,
-            values, plan->w_vpad.as<float>());
-  *out = plan->w_vpad.as<float>();
+  SellPattern *sp;
+  BT_CHECK(plan_sell(plan, &sp));
+  BT_CHECK(plan->w_sell.ensure(sizeof(float4) * 288 * (size_t)std::max<int64_t>(sp->groups, 1)));
+  BT_CHECK(sell_fill_f32(ctx, plan, values, plan->w_sell.as<float4>()));
+  *out = plan->w_sell.as<float4>();
   return BARTELS_OK;
 }
 
@@ -1615,8 +1598,7 @@ static int plan_pcg_impl(bartels_ctx ctx, bartels_mesh_plan plan, const float *v
   op.plan = plan;
   op.values = values;
   op.pinned = plan->pinned;
-  BT_CHECK(plan_padded_values(ctx, plan, values, &op.vpad));
-  op.pad_off = plan->pad_off;
+  BT_CHECK(plan_sell_values(ctx, plan, values, &op.vsell));
   if (fallback) *fallback = 0;
   const bool mg_learned = plan->precond == BARTELS_PRECOND_LEARNED_MULTIGRID && plan->lpcg_net;
   if (plan->precond == BARTELS_PRECOND_MULTIGRID || mg_learned) {
@@ -1967,14 +1949,13 @@ int advance_implicit_euler(bartels_ctx ctx, bartels_mesh_plan plan, double dt, c
   return BARTELS_OK;
 }
 
-// y = A x with the PCG loop's own SpMV kernel (k_pcg_spmv_blk, which also
-// forms the partial sums of x.Ax), on a scratch state of the plan, so that
-// timing this entry point times the SpMV the solves run. The state is zeroed
+// y = A x over the values' own layout (k_pcg_spmv_blk, which also forms the
+// partial sums of x.Ax), on a scratch state of the plan. The state is zeroed
 // once when its buffer is made; the kernel's last block resets its counter.
 int plan_spmv(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const float *x, float *y) {
   const int lanes = lanes_spmv(ctx, plan);
   const int g = grid_spmv(ctx, (int64_t)plan->nV * lanes / 32 + 1);
-  const size_t o_st = (sizeof(double) * g + 255) & ~size_t(255);
+  const size_t o_st = sizeof(double) * 4096;  // room for the partials of any grid
   const size_t need = o_st + sizeof(PcgState);
   if (plan->w_spmv.bytes < need) {
     BT_CHECK(plan->w_spmv.ensure(need));
@@ -1983,8 +1964,8 @@ int plan_spmv(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, cons
   double *part = plan->w_spmv.as<double>();
   PcgState *st = reinterpret_cast<PcgState *>(plan->w_spmv.as<char>() + o_st);
 #define BT_SPMV(G)                                                                                               \
-  BT_LAUNCH_PDL(ctx, (k_pcg_spmv_blk<G, false>), g, 256, 0, plan->nV, plan->brp, plan->bcol, values, (const int *)nullptr, \
-                x, x, y, plan->pinned, part, st)
+  BT_LAUNCH_PDL(ctx, k_pcg_spmv_blk<G>, g, 256, 0, plan->nV, plan->brp, plan->bcol, values, x, x, y, plan->pinned, \
+                part, st)
   if (lanes == 4) BT_SPMV(4);
   else if (lanes == 16) BT_SPMV(16);
   else BT_SPMV(8);
@@ -1992,47 +1973,36 @@ int plan_spmv(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, cons
   return BARTELS_OK;
 }
 
-// The PCG loop's SpMV kernel on these values (over the padded copy when the
+// The PCG loop's SpMV kernel on these values (over the sliced-ELL copy when the
 // loop uses one, made once here), y = A x: 3 warm-up launches, then reps
 // launches timed with CUDA events on the context's stream; *us = microseconds
 // per launch.
 int plan_pcg_spmv_time(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const float *x, float *y,
                        int reps, double *us) {
-  const int lanes = lanes_spmv(ctx, plan);
-  const int g = grid_spmv(ctx, (int64_t)plan->nV * lanes / 32 + 1);
-  const size_t o_st = (sizeof(double) * g + 255) & ~size_t(255);
+  const size_t o_st = sizeof(double) * 4096;
   const size_t need = o_st + sizeof(PcgState);
   if (plan->w_spmv.bytes < need) {
     BT_CHECK(plan->w_spmv.ensure(need));
     BT_CUDA(cudaMemsetAsync(plan->w_spmv.p, 0, plan->w_spmv.bytes, ctx->stream));
   }
-  double *part = plan->w_spmv.as<double>();
-  PcgState *st = reinterpret_cast<PcgState *>(plan->w_spmv.as<char>() + o_st);
-  const float *vpad = nullptr;
-  BT_CHECK(plan_padded_values(ctx, plan, values, &vpad));
-  const int *poff = plan->pad_off;
-  const int nV = plan->nV;
-  auto launch = [&]() {
-#define BT_TL(GG)                                                                                                  \
-  do {                                                                                                             \
-    if (vpad)                                                                                                      \
-      k_pcg_spmv_blk<GG, true><<<g, 256, 0, ctx->stream>>>(nV, plan->brp, plan->bcol, vpad, poff, x, x, y,         \
-                                                           plan->pinned, part, st);                                \
-    else                                                                                                           \
-      k_pcg_spmv_blk<GG, false><<<g, 256, 0, ctx->stream>>>(nV, plan->brp, plan->bcol, values, nullptr, x, x, y,   \
-                                                            plan->pinned, part, st);                               \
-  } while (0)
-    if (lanes == 4) BT_TL(4);
-    else if (lanes == 16) BT_TL(16);
-    else BT_TL(8);
-#undef BT_TL
-  };
+  PcgOperator op;
+  op.plan = plan;
+  op.values = values;
+  op.pinned = plan->pinned;
+  BT_CHECK(plan_sell_values(ctx, plan, values, &op.vsell));
+  PcgWork w{};
+  w.pa = w.pb = const_cast<float *>(x);  // read only
+  w.ap = y;
+  w.part_a = plan->w_spmv.as<double>();
+  w.st = reinterpret_cast<PcgState *>(plan->w_spmv.as<char>() + o_st);
   cudaEvent_t e0, e1;
   BT_CUDA(cudaEventCreate(&e0));
   BT_CUDA(cudaEventCreate(&e1));
-  for (int k = 0; k < 3; ++k) launch();
-  cudaEventRecord(e0, ctx->stream);
-  for (int k = 0; k < reps; ++k) launch();
+  int status = BARTELS_OK;
+  for (int k = 0; k < 3 + reps && status == BARTELS_OK; ++k) {
+    if (k == 3) cudaEventRecord(e0, ctx->stream);
+    status = pcg_spmv_blk(ctx, op, w);
+  }
   cudaEventRecord(e1, ctx->stream);
   cudaError_t e = cudaEventSynchronize(e1);
   float ms = 0.f;
@@ -2040,8 +2010,8 @@ int plan_pcg_spmv_time(bartels_ctx ctx, bartels_mesh_plan plan, const float *val
   if (e == cudaSuccess) e = cudaGetLastError();
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (status != BARTELS_OK) return status;
   if (e != cudaSuccess) return fail(BARTELS_E_DEVICE, std::string("SpMV timing: ") + cudaGetErrorString(e));
-  ctx->launches += 3 + reps;
   *us = 1e3 * ms / reps;
   return BARTELS_OK;
 }
@@ -2127,8 +2097,8 @@ int plan_set_hessian_tuning(bartels_mesh_plan plan, int chunk, int block) {
   return BARTELS_OK;
 }
 
-// Autotuner: time the PCG loop's block-row SpMV with 4, 8 and 16 lanes per
-// vertex row and the factor passes with 4 and 8 lanes on this plan (CUDA
+// Autotuner: time the block-row SpMV over the values' own layout with 4, 8 and 16
+// lanes per vertex row and the factor passes with 4 and 8 lanes on this plan (CUDA
 // events on the context's stream, 3 warm-up + 10 timed launches each, best of
 // three rounds over the candidates), keep the fastest in
 // the plan and in the context's cache for the plan's size bucket
@@ -2181,13 +2151,6 @@ int plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, 
     cudaMemsetAsync(gl, 0, 2 * (size_t)fp->lsize + 16, ctx->stream);
     cudaMemsetAsync(st, 0, sizeof(PcgState), ctx->stream);
     const int nV = plan->nV;
-    const float *vpad = nullptr;
-    const int ps = plan_padded_values(ctx, plan, values, &vpad);
-    if (ps != BARTELS_OK) {
-      cleanup();
-      return ps;  // with plan_padded_values' message
-    }
-    const int *poff = plan->pad_off;
     // three rounds over the candidates, each candidate's best time kept (the
     // clocks may still be ramping up when a plan is set up)
     constexpr int kRounds = 3;
@@ -2198,17 +2161,10 @@ int plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, 
     for (int ci = 0; ci < 3; ++ci) {
       const int G = cand_s[ci];
       const int g = grid_spmv(ctx, (int64_t)nV * G / 32 + 1);
-      // the PCG loop's own SpMV (A p and the partials of p.Ap) on a scratch state
+      // A p over the values' own layout and the partials of p.Ap on a scratch state
       const float ms = timed([&] {
-#define BT_TS(GG)                                                                                             \
-  do {                                                                                                        \
-    if (vpad)                                                                                                 \
-      k_pcg_spmv_blk<GG, true><<<g, 256, 0, ctx->stream>>>(nV, plan->brp, plan->bcol, vpad, poff, x, x, y,    \
-                                                           plan->pinned, part, st);                           \
-    else                                                                                                      \
-      k_pcg_spmv_blk<GG, false><<<g, 256, 0, ctx->stream>>>(nV, plan->brp, plan->bcol, values, nullptr, x, x, \
-                                                            y, plan->pinned, part, st);                       \
-  } while (0)
+#define BT_TS(GG) \
+  k_pcg_spmv_blk<GG><<<g, 256, 0, ctx->stream>>>(nV, plan->brp, plan->bcol, values, x, x, y, plan->pinned, part, st)
         if (G == 4) BT_TS(4);
         else if (G == 8) BT_TS(8);
         else BT_TS(16);
