@@ -110,6 +110,13 @@ struct SegInfo {
   double *rz = nullptr, *rr = nullptr, *tol2 = nullptr, *abs2 = nullptr, *red = nullptr, *red2 = nullptr;
   float *alpha = nullptr, *beta = nullptr;
   int *done = nullptr, *iters = nullptr;
+  // the segments' DOFs cut into pieces, one CTA of a per-segment reduction each:
+  // {segment, first DOF, end, unused}
+  int npieces = 0;
+  int4 *piece = nullptr;
+  int *piece_ptr = nullptr;      // nseg + 1: pieces of each segment
+  double *piece_sum = nullptr;   // 2 per piece
+  unsigned int *piece_count = nullptr;  // nseg: pieces finished (reset by the last)
   double *alpha64 = nullptr;     // line-search steps
   double *et = nullptr, *ev = nullptr;  // per-tet and per-vertex energy-difference terms
   std::vector<int> last_iters;   // PCG iterations per segment of the last solve (host)

@@ -1123,6 +1123,10 @@ struct SegPtrs {
   double *rz, *rr, *tol2, *abs2, *red;
   float *alpha, *beta;
   int *done, *iters;
+  const int4 *piece;
+  const int *piece_ptr;
+  double *piece_sum;
+  unsigned int *piece_count;
 };
 
 enum { kSegNorm = 0, kSegInit = 1, kSegPap = 2, kSegRzRr = 3 };
@@ -1136,6 +1140,12 @@ enum { kSegNorm = 0, kSegInit = 1, kSegPap = 2, kSegRzRr = 3 };
 // kSegInit and kSegRzRr end with the last CTA setting the global state (all
 // segments done, or the iteration cap) that the shared kernels and the loop
 // condition read.
+//
+// One CTA per piece of at most kSegPiece DOFs; the last piece of a segment adds
+// the segment's partial sums in order. With one CTA per segment the two
+// reductions of an iteration took 42 + 48 us of 200 on 24 meshes of 8 - 22
+// cells a side: 24 CTAs, the largest with 36,501 entries.
+constexpr int kSegPiece = 2048;
 template <int MODE>
 __global__ void __launch_bounds__(256)
 k_seg_scalars(SegPtrs sp, const float *__restrict__ a, const float *__restrict__ b, const float *__restrict__ c,
@@ -1145,15 +1155,37 @@ k_seg_scalars(SegPtrs sp, const float *__restrict__ a, const float *__restrict__
   pdl_trigger();
   if ((MODE == kSegPap || MODE == kSegRzRr) && st->done) return;
   if (MODE == kSegPap) a = (st->it & 1) ? pb : pa;
-  const int s = blockIdx.x;
-  const int i0 = 3 * sp.voff[s], i1 = 3 * sp.voff[s + 1];
+  const int4 pc = sp.piece[blockIdx.x];
+  const int s = pc.x;
   float acc1 = 0.f, acc2 = 0.f;
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+#pragma unroll 4
+  for (int i = pc.y + threadIdx.x; i < pc.z; i += blockDim.x) {
     acc1 += __ldcg(a + i) * __ldcg(b + i);
     if (c) acc2 += __ldcg(c + i) * __ldcg(d + i);
   }
-  const double s1 = cta_sum_f(acc1);
-  const double s2 = c ? cta_sum_f(acc2) : 0.0;
+  const double p1 = cta_sum_f(acc1);
+  const double p2 = c ? cta_sum_f(acc2) : 0.0;
+  if (threadIdx.x == 0) {
+    sp.piece_sum[2 * blockIdx.x] = p1;
+    sp.piece_sum[2 * blockIdx.x + 1] = p2;
+  }
+  const int q0 = sp.piece_ptr[s], q1 = sp.piece_ptr[s + 1];
+  {
+    __shared__ bool seg_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) seg_last = atomicAdd(sp.piece_count + s, 1u) == (unsigned)(q1 - q0 - 1);
+    __syncthreads();
+    if (!seg_last) return;
+  }
+  double s1 = 0.0, s2 = 0.0;
+  for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    s1 += __ldcg(sp.piece_sum + 2 * q);
+    s2 += __ldcg(sp.piece_sum + 2 * q + 1);
+  }
+  s1 = cta_sum(s1);
+  s2 = c ? cta_sum(s2) : 0.0;
+  if (threadIdx.x == 0) sp.piece_count[s] = 0;
   if (threadIdx.x == 0) {
     if (MODE == kSegNorm) {
       sp.red[s] = s1;
@@ -1180,7 +1212,12 @@ k_seg_scalars(SegPtrs sp, const float *__restrict__ a, const float *__restrict__
     }
   }
   if (MODE == kSegInit || MODE == kSegRzRr) {
-    if (last_block(&st->count)) {
+    __shared__ bool all_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) all_last = atomicAdd(&st->count, 1u) == (unsigned)(sp.nseg - 1);
+    __syncthreads();
+    if (all_last) {
       int all = 1;
       for (int q = threadIdx.x; q < sp.nseg; q += blockDim.x)
         if (!__ldcg(sp.done + q)) all = 0;
@@ -1311,6 +1348,10 @@ static SegPtrs seg_ptrs(const SegInfo *sg) {
   sp.beta = sg->beta;
   sp.done = sg->done;
   sp.iters = sg->iters;
+  sp.piece = sg->piece;
+  sp.piece_ptr = sg->piece_ptr;
+  sp.piece_sum = sg->piece_sum;
+  sp.piece_count = sg->piece_count;
   return sp;
 }
 
@@ -1321,12 +1362,12 @@ static int seg_enqueue_iters(bartels_ctx ctx, const PcgOperator &op, const PcgWo
   const int gv = grid_vec(ctx, nV);
   for (int i = 0; i < iters; ++i) {
     BT_CHECK(pcg_spmv_blk(ctx, op, w));
-    BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegPap>, sp.nseg, 256, 0, sp, (const float *)nullptr, w.ap,
+    BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegPap>, op.plan->seg->npieces, 256, 0, sp, (const float *)nullptr, w.ap,
                   (const float *)nullptr, (const float *)nullptr, w.pa, w.pb, 0.0, 0, w.st);
     BT_LAUNCH_PDL(ctx, k_seg_update, gv, 256, 0, nV, sp.vseg, sp.alpha, w.pa, w.pb, w.ap, w.x, w.r, w.z,
                   op.mg ? (const float *)nullptr : w.minv, w.st);
     if (op.mg) BT_CHECK(mg_enqueue_apply(ctx, plan, op.values, op.sm, w.r, w.z, w.ap, w.part_b, w.st, false));
-    BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegRzRr>, sp.nseg, 256, 0, sp, w.r, w.z, w.r, w.r, (const float *)nullptr,
+    BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegRzRr>, op.plan->seg->npieces, 256, 0, sp, w.r, w.z, w.r, w.r, (const float *)nullptr,
                   (const float *)nullptr, 0.0, 0, w.st);
     BT_LAUNCH_PDL(ctx, k_seg_dir, gv, 256, 0, nV, sp.vseg, sp.beta, w.z, w.pa, w.pb, w.st);
   }
@@ -1409,7 +1450,7 @@ static int seg_pcg_solve(bartels_ctx ctx, const PcgOperator &op, const double *b
     }
     BT_LAUNCH(ctx, k_resid_blk_ff<lanes_r>, gs, 256, 0, nV, plan->brp, plan->bcol, op.values, w.xh, w.xl, w.bh,
               w.bl, w.rres, op.pinned, w.part_a);
-    BT_LAUNCH(ctx, k_seg_scalars<kSegNorm>, nseg, 256, 0, sp, w.rres, w.rres, (const float *)nullptr,
+    BT_LAUNCH(ctx, k_seg_scalars<kSegNorm>, sg->npieces, 256, 0, sp, w.rres, w.rres, (const float *)nullptr,
               (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, 0.0, 0, w.st);
     BT_CUDA(cudaMemcpyAsync(rr.data(), sg->red, sizeof(double) * nseg, cudaMemcpyDeviceToHost, ctx->stream));
     BT_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1443,7 +1484,7 @@ static int seg_pcg_solve(bartels_ctx ctx, const PcgOperator &op, const double *b
     BT_LAUNCH_PDL(ctx, k_seg_init, gv, 256, 0, nV, sg->vseg, sg->done, w.rres, op.mg ? (const float *)nullptr : w.minv,
                   w.x, w.r, w.z, w.pa, w.pb, w.st);
     if (op.mg) BT_CHECK(mg_enqueue_apply(ctx, plan, op.values, op.sm, w.r, w.z, w.ap, w.part_b, w.st, false));
-    BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegInit>, nseg, 256, 0, sp, w.r, w.z, w.r, w.r, (const float *)nullptr,
+    BT_LAUNCH_PDL(ctx, k_seg_scalars<kSegInit>, sg->npieces, 256, 0, sp, w.r, w.z, w.r, w.r, (const float *)nullptr,
                   (const float *)nullptr, prm.inner_rel_tol * prm.inner_rel_tol, prm.max_iters - rep->iterations,
                   w.st);
     BT_LAUNCH_PDL(ctx, k_seg_dir, gv, 256, 0, nV, sg->vseg, sg->beta, w.z, w.pa, w.pb, w.st);
@@ -1549,6 +1590,26 @@ int plan_set_segments(bartels_mesh_plan plan, int nseg, const int *voff, const i
   BT_CHECK(alloc((void **)&sg->iters, sizeof(int) * nseg));
   BT_CHECK(alloc((void **)&sg->et, sizeof(double) * plan->nT));
   BT_CHECK(alloc((void **)&sg->ev, sizeof(double) * plan->nV));
+  // pieces: every segment has at least one, so that an empty one still gets its scalars
+  std::vector<int4> piece;
+  std::vector<int> pptr(nseg + 1, 0);
+  for (int q = 0; q < nseg; ++q) {
+    const int i0 = 3 * voff[q], i1 = 3 * voff[q + 1];
+    int i = i0;
+    do {
+      piece.push_back(make_int4(q, i, std::min(i + kSegPiece, i1), 0));
+      i += kSegPiece;
+    } while (i < i1);
+    pptr[q + 1] = (int)piece.size();
+  }
+  sg->npieces = (int)piece.size();
+  BT_CHECK(alloc((void **)&sg->piece, sizeof(int4) * piece.size()));
+  BT_CHECK(alloc((void **)&sg->piece_ptr, sizeof(int) * (nseg + 1)));
+  BT_CHECK(alloc((void **)&sg->piece_sum, sizeof(double) * 2 * piece.size()));
+  BT_CHECK(alloc((void **)&sg->piece_count, sizeof(unsigned int) * nseg));
+  BT_CUDA(cudaMemcpy(sg->piece, piece.data(), sizeof(int4) * piece.size(), cudaMemcpyHostToDevice));
+  BT_CUDA(cudaMemcpy(sg->piece_ptr, pptr.data(), sizeof(int) * (nseg + 1), cudaMemcpyHostToDevice));
+  BT_CUDA(cudaMemset(sg->piece_count, 0, sizeof(unsigned int) * nseg));
   BT_CUDA(cudaMemcpy(sg->voff, voff, sizeof(int) * (nseg + 1), cudaMemcpyHostToDevice));
   BT_CUDA(cudaMemcpy(sg->toff, toff, sizeof(int64_t) * (nseg + 1), cudaMemcpyHostToDevice));
   BT_CUDA(cudaMemcpy(sg->vseg, vseg.data(), sizeof(int) * plan->nV, cudaMemcpyHostToDevice));
