@@ -786,9 +786,9 @@ __device__ __forceinline__ void cl_barrier() {
 // Dense inverse of the coarsest level (nd = 6 x nodes <= 384, symmetrised) by
 // in-place block Gauss-Jordan without pivoting (the matrix is SPD). Dead DOFs
 // as in k_mg_inv6. One thread-block cluster; each CTA keeps the rows of its
-// own nodes (split) in shared memory. Per node K: the owner eliminates within
-// the node's 6 rows and publishes them (panel, double-buffered), then every
-// CTA updates its other rows. One cluster barrier per node: 8 / 64 nodes take
+// own nodes (split) in shared memory. Per node K: the owner inverts the 6x6 pivot
+// block, scales the node's 6 rows with it and publishes them (panel, double-
+// buffered), then every CTA updates its other rows. One cluster barrier per node: 8 / 64 nodes take
 // ~16 / ~130 us; a single CTA with a barrier per scalar pivot took 58 us for
 // 8 and 552 us for 18.
 struct MgInvArgs {
@@ -802,6 +802,7 @@ __global__ void __launch_bounds__(kInvThreads, 1)
 k_mg_dense_inv(const __grid_constant__ MgInvArgs a) {
   extern __shared__ __align__(16) float sA[];  // own rows (6 x own nodes) x nd, then the panel 6 x nd
   __shared__ unsigned char dead[6 * kDenseNodes];
+  __shared__ float sPiv[36];
   const int rank = cl_rank(), n0 = a.split[rank], n1 = a.split[rank + 1], rows = 6 * (n1 - n0), nd = 6 * a.nodes;
   float *sP = sA + rows * nd;
   for (int i = threadIdx.x; i < nd; i += blockDim.x) dead[i] = !(a.val[36ll * a.dpos[i / 6] + 7 * (i % 6)] != 0.f);
@@ -821,24 +822,40 @@ k_mg_dense_inv(const __grid_constant__ MgInvArgs a) {
     float *pan = a.panel + (K & 1) * 6 * nd;
     if (K >= n0 && K < n1) {
       float *R = sA + 6 * (K - n0) * nd;  // the node's 6 rows
-      for (int k = 0; k < 6; ++k) {
-        const int kk = 6 * K + k;
-        const float piv = R[k * nd + kk], p = piv > 0.f ? 1.f / piv : 0.f;
-        float f[6];
+      if (threadIdx.x < 32) {
+        // P = inverse of the 6x6 pivot block: lane r < 6 holds its row r
+        const int r = min((int)threadIdx.x, 5);
+        float w[6];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) f[r] = R[r * nd + kk];
-        __syncthreads();
-        for (int j = threadIdx.x; j < nd; j += blockDim.x) {
-          const float t = j == kk ? p : R[k * nd + j] * p;
+        for (int c = 0; c < 6; ++c) w[c] = R[r * nd + 6 * K + c];
 #pragma unroll
-          for (int r = 0; r < 6; ++r) {
-            if (r == k) R[r * nd + j] = t;
-            else R[r * nd + j] = j == kk ? -f[r] * p : R[r * nd + j] - f[r] * t;
+        for (int k = 0; k < 6; ++k) {
+          const float piv = __shfl_sync(0xffffffffu, w[k], k), p = piv > 0.f ? 1.f / piv : 0.f, f = w[k];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            const float t = (c == k ? 1.f : __shfl_sync(0xffffffffu, w[c], k)) * p;
+            w[c] = r == k ? t : (c == k ? -f * t : w[c] - f * t);
           }
         }
-        __syncthreads();
+        if (threadIdx.x < 6)
+#pragma unroll
+          for (int c = 0; c < 6; ++c) sPiv[6 * r + c] = w[c];
       }
-      for (int e = threadIdx.x; e < 6 * nd; e += blockDim.x) pan[e] = R[e];
+      __syncthreads();
+      for (int j = threadIdx.x; j < nd; j += blockDim.x) {
+        float v[6];
+        const int jj = j - 6 * K;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) v[c] = jj >= 0 && jj < 6 ? (c == jj ? 1.f : 0.f) : R[c * nd + j];
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
+          float t = 0.f;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) t += sPiv[6 * r + c] * v[c];
+          R[r * nd + j] = t;
+          pan[r * nd + j] = t;
+        }
+      }
     }
     cl_barrier();
     for (int e = threadIdx.x; e < 6 * nd; e += blockDim.x) sP[e] = __ldcg(pan + e);
