@@ -936,7 +936,7 @@ BT_HD void tridiag_qr(T *d, T *e, T *Z, T eps) {
 // eigenvectors the columns of Z (column-major 9x9). Householder reduction to
 // tridiagonal form, the reflectors multiplied out, then implicit QR. Every
 // index is a compile-time constant, so the arrays stay in registers. The
-// entries are expected to be of order one (psd_eig_N scales them); an off-
+// entries are expected to be of order one (psd_eig_K scales them); an off-
 // diagonal is negligible at one rounding of that order.
 //
 // Bound by issue: two to three QR steps per eigenvalue, ~64 instructions per
@@ -1004,13 +1004,16 @@ BT_HD void eig9p(T *A, T *d, T *Z) {
   tridiag_qr<8>(d, e, Z, sizeof(T) == 4 ? T(6e-8) : T(1e-16));
 }
 
-// Slow path, step 1 (once per element): N = W max(L, tol) W^T (packed, 45)
-// with M = (R (x) I) S (R^T (x) I) = W L W^T.
+// Slow path, step 1 (once per element): the projected blocks K_ab of nodes a, b =
+// 1 .. 3 (packed symmetric 9x9, rows 3 (a - 1) + k), without the tol/4
+// translation term. With M = (R (x) I) S (R^T (x) I) = W L W^T the projection is
+// (Q (x) I) W max(L, tol) W^T (Q^T (x) I); the eigenvectors are taken to the
+// nodes first. Node 0 follows from the null translations (psd_row_from_K).
 template <class Law, class T>
-BT_HD_NOINLINE void psd_eig_N(const Law &law, const T (*phi)[3], T tol, T *N) {
-  T M[45];
+BT_HD_NOINLINE void psd_eig_K(const Law &law, const T (*phi)[3], T tol, T *K) {
+  T M[45], Q[4][3];
   {
-    T S[45], Q[4][3], Rm[9];
+    T S[45], Rm[9];
     law_matrix9p(law, S);
     qr_phi(phi, Q, Rm);
     // M[(k + 3c), (l + 3d)] = sum_{i,j} R[c][i] R[d][j] S[(k + 3i), (l + 3j)]  (R upper triangular)
@@ -1045,6 +1048,15 @@ BT_HD_NOINLINE void psd_eig_N(const Law &law, const T (*phi)[3], T tol, T *N) {
   const T floor_ = tol * up;
 #pragma unroll
   for (int i = 0; i < 9; ++i) lam[i] = (lam[i] < floor_ ? floor_ : lam[i]) * down;
+  // Y = (Q (x) I) W for nodes 1 .. 3, in place
+#pragma unroll
+  for (int e = 0; e < 9; ++e)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const T w0 = W[k + 9 * e], w1 = W[3 + k + 9 * e], w2 = W[6 + k + 9 * e];
+#pragma unroll
+      for (int a = 1; a < 4; ++a) W[3 * (a - 1) + k + 9 * e] = Q[a][0] * w0 + Q[a][1] * w1 + Q[a][2] * w2;
+    }
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     T wl[9];
@@ -1055,38 +1067,35 @@ BT_HD_NOINLINE void psd_eig_N(const Law &law, const T (*phi)[3], T tol, T *N) {
       T acc = T(0);
 #pragma unroll
       for (int k = 0; k < 9; ++k) acc += wl[k] * W[j + 9 * k];
-      N[p9(i, j)] = acc;
+      K[p9(i, j)] = acc;
     }
   }
 }
 
-// Slow path, step 2 (per incidence): blocks K_ab (b = 0..3) of row a from the
-// projected N (packed), without the tol/4 translation term.
+// Slow path, step 2 (per incidence): blocks K_ab (b = 0 .. 3) of row a from the
+// packed K. The projected element matrix keeps the translations in its null
+// space, so K_0b = -(K_1b + K_2b + K_3b) and K_a0 = -(K_a1 + K_a2 + K_a3).
 template <class T>
-BT_HD void psd_blocks_from_N(const T *N, const T (*phi)[3], int a, T (*out)[9]) {
-  T Q[4][3], Rm[9];
-  qr_phi(phi, Q, Rm);
+BT_HD void psd_row_from_K(const T *K, int a, T (*out)[9]) {
 #pragma unroll
-  for (int b = 0; b < 4; ++b)
+  for (int b = 1; b < 4; ++b)
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
       for (int l = 0; l < 3; ++l) {
-        T acc = T(0);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int d = 0; d < 3; ++d) acc += Q[a][c] * Q[b][d] * N[p9(k + 3 * c, l + 3 * d)];
-        out[b][3 * k + l] = acc;
+        const T r1 = K[p9(k, 3 * (b - 1) + l)], r2 = K[p9(3 + k, 3 * (b - 1) + l)], r3 = K[p9(6 + k, 3 * (b - 1) + l)];
+        out[b][3 * k + l] = a == 0 ? -(r1 + r2 + r3) : a == 1 ? r1 : a == 2 ? r2 : r3;
       }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) out[0][i] = -(out[1][i] + out[2][i] + out[3][i]);
 }
 
 // Both steps (used by host tests and by callers without a pre-pass)
 template <class Law, class T>
 BT_HD void psd_row_slow(const Law &law, const T (*phi)[3], T tol, int a, T (*out)[9]) {
-  T N[45];
-  psd_eig_N(law, phi, tol, N);
-  psd_blocks_from_N(N, phi, a, out);
+  T K[45];
+  psd_eig_K(law, phi, tol, K);
+  psd_row_from_K(K, a, out);
 }
 
 }  // namespace bartels

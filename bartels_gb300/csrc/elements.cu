@@ -499,13 +499,13 @@ k_psd_test(int nT, const TetRec32 *__restrict__ rec, const float4 *__restrict__ 
   }
 }
 
-// PSD pre-pass, part 2, one thread per flagged tet: the projected 9x9 N
-// (packed, 45 floats) of simple_psd_fix.
+// PSD pre-pass, part 2, one thread per flagged tet: the blocks of nodes 1 .. 3 of
+// the matrix that simple_psd_fix projects (packed, 45 floats in a slot of 48).
 template <int MODEL>
 __global__ void __launch_bounds__(256)
 k_psd_eig(const int *__restrict__ list, const int *__restrict__ count, const TetRec32 *__restrict__ rec,
           const float4 *__restrict__ u, const float4 *__restrict__ ul, int add_identity, float tol, int corot_exact,
-          float *__restrict__ Nbuf) {
+          float *__restrict__ Kbuf) {
   const int n = *count;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int t = __ldg(list + i);
@@ -516,11 +516,12 @@ k_psd_eig(const int *__restrict__ list, const int *__restrict__ count, const Tet
     float F[9];
     elem_F<MODEL>(r, u, ul, add_identity, F);
     with_law<MODEL>(F, r.pv, corot_exact, [&](const auto &law) {
-      float N[45];
-      psd_eig_N(law, phi, tol, N);
-      float *o = Nbuf + 45ll * t;
+      float K[48];
+      K[45] = K[46] = K[47] = 0.f;
+      psd_eig_K(law, phi, tol, K);
+      float4 *o = reinterpret_cast<float4 *>(Kbuf + 48ll * t);
 #pragma unroll
-      for (int k = 0; k < 45; ++k) o[k] = N[k];
+      for (int k = 0; k < 12; ++k) o[k] = make_float4(K[4 * k], K[4 * k + 1], K[4 * k + 2], K[4 * k + 3]);
     });
   }
 }
@@ -581,18 +582,21 @@ __device__ __forceinline__ void load_inc_x(const float4 *__restrict__ u, const f
 // so K_a0 = -(K_a1 + K_a2 + K_a3) and only three blocks are evaluated.
 template <int MODEL, bool PSD>
 __device__ __forceinline__ void hess_inc(const HessInc &h, float *row, int rs, float *D, int add_identity, float cK,
-                                         float cM, float tol, int corot_exact, const float *__restrict__ Nbuf) {
+                                         float cM, float tol, int corot_exact, const float *__restrict__ Kbuf) {
   const int a = h.a;
   float phi[4][3];
   phi4(h.r.dphi, phi);
   float K[4][9];
   if constexpr (MODEL >= 0) {
     if (PSD && h.slow) {
-      float N[45];
-      const float *src = Nbuf + 45ll * h.t;
+      float P[48];
+      const float4 *src = reinterpret_cast<const float4 *>(Kbuf + 48ll * h.t);
 #pragma unroll
-      for (int i = 0; i < 45; ++i) N[i] = __ldg(src + i);
-      psd_blocks_from_N(N, phi, a, K);
+      for (int i = 0; i < 12; ++i) {
+        const float4 q = __ldg(src + i);
+        P[4 * i] = q.x; P[4 * i + 1] = q.y; P[4 * i + 2] = q.z; P[4 * i + 3] = q.w;
+      }
+      psd_row_from_K(P, a, K);
 #pragma unroll
       for (int b = 0; b < 4; ++b)
 #pragma unroll
@@ -669,7 +673,7 @@ __global__ void __launch_bounds__(kChunkMaxVerts)
 k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *__restrict__ inc_ptr,
        const int *__restrict__ inc_tet, const uint32_t *__restrict__ inc_pos, const TetRec32 *__restrict__ rec,
        const float4 *__restrict__ u, const float4 *__restrict__ ul, int add_identity, float cK, float cM, float tol,
-       int corot_exact, const float4 *__restrict__ fslot, const float *__restrict__ Nbuf, float *__restrict__ values) {
+       int corot_exact, const float4 *__restrict__ fslot, const float *__restrict__ Kbuf, float *__restrict__ values) {
   constexpr bool PRE = PSD && MODEL >= 0;
   extern __shared__ float sbuf[];
   const int v0 = chunk_v[blockIdx.x], v1 = chunk_v[blockIdx.x + 1];
@@ -695,8 +699,8 @@ k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *
       load_inc_x<PRE>(u, ul, h0);
       load_inc_x<PRE>(u, ul, h1);
       jd = (h0.pos >> (8 * h0.a)) & 255;
-      hess_inc<MODEL, PSD>(h0, row, rs, D, add_identity, cK, cM, tol, corot_exact, Nbuf);
-      if (two) hess_inc<MODEL, PSD>(h1, row, rs, D, add_identity, cK, cM, tol, corot_exact, Nbuf);
+      hess_inc<MODEL, PSD>(h0, row, rs, D, add_identity, cK, cM, tol, corot_exact, Kbuf);
+      if (two) hess_inc<MODEL, PSD>(h1, row, rs, D, add_identity, cK, cM, tol, corot_exact, Kbuf);
     }
     if (k1 > k0) {
 #pragma unroll
@@ -979,25 +983,25 @@ static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *
   }
   const int pb = plan->psd_block;
   float4 *fslot = nullptr;
-  float *nbuf = nullptr;
+  float *kbuf = nullptr;
   const float4 *ul = u + plan->nV;  // lo parts of the displacement pairs follow the hi parts
   if constexpr (PSD && MODEL >= 0) {
     const size_t nT = (size_t)plan->nT;
-    // F + flag slots (12 floats per tet), N (45 floats per tet), the slow-tet list and its count
-    BT_CHECK(plan->w_psd.ensure(nT * (57 * sizeof(float) + sizeof(int)) + 512));
+    // F + flag slots (12 floats per tet), projected blocks (48 floats per tet), the slow-tet list and its count
+    BT_CHECK(plan->w_psd.ensure(nT * (60 * sizeof(float) + sizeof(int)) + 512));
     fslot = plan->w_psd.as<float4>();
-    nbuf = reinterpret_cast<float *>(fslot + 3 * nT);
-    int *list = reinterpret_cast<int *>(nbuf + 45 * nT);
+    kbuf = reinterpret_cast<float *>(fslot + 3 * nT);
+    int *list = reinterpret_cast<int *>(kbuf + 48 * nT);
     int *count = list + nT;
     BT_CUDA(cudaMemsetAsync(count, 0, sizeof(int), ctx->stream));
     BT_LAUNCH(ctx, k_psd_test<MODEL>, grid_for(ctx, plan->nT, pb), pb, 0, plan->nT, plan->rec32, u, ul,
               add_identity, tol, corot_exact, fslot, list, count);
     BT_LAUNCH(ctx, k_psd_eig<MODEL>, grid_for(ctx, plan->nT, pb), pb, 0, list, count, plan->rec32, u, ul,
-              add_identity, tol, corot_exact, nbuf);
+              add_identity, tol, corot_exact, kbuf);
   }
   BT_LAUNCH(ctx, (k_hess<MODEL, PSD>), small ? plan->nchunks64 : plan->nchunks, small ? 64 : kChunkMaxVerts, smem,
             small ? plan->chunk_v64 : plan->chunk_v, plan->brp, plan->inc_ptr, plan->inc_tet, plan->inc_pos,
-            plan->rec32, u, ul, add_identity, cK, cM, tol, corot_exact, fslot, nbuf, values);
+            plan->rec32, u, ul, add_identity, cK, cM, tol, corot_exact, fslot, kbuf, values);
   return BARTELS_OK;
 }
 
