@@ -419,13 +419,6 @@ __global__ void k_grad_gather(int nV, const int *__restrict__ inc_ptr, const int
 }
 
 // ------------------------------------------------- fused FP32 Hessian -------
-// One CTA per chunk of consecutive vertices, one thread per vertex. The thread
-// walks its incidences in tet order, evaluates the 3x12 slab (row block a) of
-// the element Hessian B^T d2psi B vol (PSD-projected if asked), and adds the
-// four 3x3 blocks into its CSR rows staged in shared memory at the positions
-// precomputed in inc_pos. Every entry is therefore summed over its tets in tet
-// order, as the reference's setFromTriplets does. The chunk's values are then
-// written out with coalesced stores.
 // F of a tet from its vertices' displacement pairs (x = hi, l = lo): the edge
 // differences are (hi_a - hi_0) + (lo_a - lo_0).
 template <int MODEL>
@@ -573,20 +566,17 @@ __device__ __forceinline__ void load_inc_x(const float4 *__restrict__ u, const f
   }
 }
 
-// Row block a of one element Hessian: the off-diagonal blocks (b != a) are
-// added into the thread's staged CSR rows, the diagonal block (b == a, always
-// the thread's own diagonal position) into the registers D.
+// Row block a of one element Hessian, K_ab for b = 0 .. 3.
 //
 // Unprojected elements: every law is linear in its parameters (K cK =
 // K(cK pv)) and bilinear in (pa, pb) with phi_0 = -(phi_1 + phi_2 + phi_3),
 // so K_a0 = -(K_a1 + K_a2 + K_a3) and only three blocks are evaluated.
 template <int MODEL, bool PSD>
-__device__ __forceinline__ void hess_inc(const HessInc &h, float *row, int rs, float *D, int add_identity, float cK,
-                                         float cM, float tol, int corot_exact, const float *__restrict__ Kbuf) {
+__device__ __forceinline__ void hess_slab(const HessInc &h, float (*K)[9], int add_identity, float cK, float cM,
+                                          float tol, int corot_exact, const float *__restrict__ Kbuf) {
   const int a = h.a;
   float phi[4][3];
   phi4(h.r.dphi, phi);
-  float K[4][9];
   if constexpr (MODEL >= 0) {
     if (PSD && h.slow) {
       float P[48];
@@ -644,36 +634,48 @@ __device__ __forceinline__ void hess_inc(const HessInc &h, float *row, int rs, f
       K[b][8] += m;
     }
   }
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    if (b == a) {
-#pragma unroll
-      for (int i = 0; i < 9; ++i) D[i] += K[b][i];
-    } else {
-      const int j = (h.pos >> (8 * b)) & 255;
-#pragma unroll
-      for (int kk = 0; kk < 3; ++kk)
-#pragma unroll
-        for (int ll = 0; ll < 3; ++ll) row[kk * rs + 3 * j + ll] += K[b][3 * kk + ll];
-    }
-  }
 }
 
-// One CTA per chunk of consecutive vertices, one thread per vertex. The thread
-// walks its incidences in tet order, evaluates the 3x12 slab (row block a) of
-// the element Hessian B^T d2psi B vol (PSD-projected if asked, from the
-// pre-pass), and adds the four 3x3 blocks into its CSR rows staged in shared
-// memory at the positions precomputed in inc_pos. Every entry is therefore
-// summed over its tets in tet order, as the reference's setFromTriplets does.
-// Incidences are loaded two at a time (both load chains, incidence -> tet
-// record -> vertex positions, in flight together) and added in order. The
-// chunk's values are then written out with coalesced stores.
-template <int MODEL, bool PSD>
-__global__ void __launch_bounds__(kChunkMaxVerts)
+// Adds one 3x3 block at block position j of the row. The nine addresses are
+// distinct: all are read before the first is written, so that the block costs
+// one shared-memory latency and not nine.
+__device__ __forceinline__ void hess_add_block(float *row, int rs, int j, const float *K) {
+  float *p = row + 3 * j, t[9];
+#pragma unroll
+  for (int kk = 0; kk < 3; ++kk)
+#pragma unroll
+    for (int ll = 0; ll < 3; ++ll) t[3 * kk + ll] = p[kk * rs + ll];
+#pragma unroll
+  for (int kk = 0; kk < 3; ++kk)
+#pragma unroll
+    for (int ll = 0; ll < 3; ++ll) p[kk * rs + ll] = t[3 * kk + ll] + K[3 * kk + ll];
+}
+
+// One CTA per chunk of consecutive vertices, G lanes per vertex. The lanes take
+// the vertex's incidences G at a time in tet order, evaluate the 3x12 slabs (row
+// block a) of the element Hessian B^T d2psi B vol at the same time
+// (PSD-projected if asked, from the pre-pass), and add the off-diagonal blocks
+// one lane after the other into the vertex's CSR rows staged in shared memory,
+// at the positions precomputed in inc_pos. Every off-diagonal entry is therefore
+// summed over its tets in tet order, as the reference's setFromTriplets does;
+// the diagonal block is summed per lane and then over the lanes, in a fixed
+// order. The chunk's values are then written out with coalesced stores.
+//
+// Bound by the L1 / shared-memory pipe (fully divergent 16-byte record loads and
+// the staged rows' read-modify-writes) and, on small meshes, by a lane's chain
+// of evaluations. n = 96 without projection: one lane per vertex 855 us (12
+// warps per SM, 78% of the pipe), two lanes 760 us, four 1,094 (the adds are
+// issued once per lane of the group); 1.05M tets with projection 375 / 274 /
+// 354. On 135k tets (25k vertices): 101 / 62 / 82, on 15.6k vertices two lanes
+// 39, four 34. So two lanes, and four where the chunks leave most SMs short of
+// work (launch_hess_t).
+template <int MODEL, bool PSD, int G>
+__global__ void __launch_bounds__(kChunkMaxVerts * G, 4 / G)
 k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *__restrict__ inc_ptr,
-       const int *__restrict__ inc_tet, const uint32_t *__restrict__ inc_pos, const TetRec32 *__restrict__ rec,
-       const float4 *__restrict__ u, const float4 *__restrict__ ul, int add_identity, float cK, float cM, float tol,
-       int corot_exact, const float4 *__restrict__ fslot, const float *__restrict__ Kbuf, float *__restrict__ values) {
+             const int *__restrict__ inc_tet, const uint32_t *__restrict__ inc_pos, const TetRec32 *__restrict__ rec,
+             const float4 *__restrict__ u, const float4 *__restrict__ ul, int add_identity, float cK, float cM,
+             float tol, int corot_exact, const float4 *__restrict__ fslot, const float *__restrict__ Kbuf,
+             float *__restrict__ values) {
   constexpr bool PRE = PSD && MODEL >= 0;
   extern __shared__ float sbuf[];
   const int v0 = chunk_v[blockIdx.x], v1 = chunk_v[blockIdx.x + 1];
@@ -681,34 +683,47 @@ k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *
   const int len = 9 * (brp[v1] - b0);
   for (int i = threadIdx.x; i < len; i += blockDim.x) sbuf[i] = 0.f;
   __syncthreads();
-  const int v = v0 + threadIdx.x;
+  const int v = v0 + threadIdx.x / G, sl = threadIdx.x % G;
+  int k0 = 0, k1 = 0, rs = 0;
+  float *row = sbuf;
   if (v < v1) {
     const int rb = brp[v];
-    const int rs = 3 * (brp[v + 1] - rb);
-    float *row = sbuf + 9 * (rb - b0);
-    const int k0 = inc_ptr[v], k1 = inc_ptr[v + 1];
-    float D[9];
+    rs = 3 * (brp[v + 1] - rb);
+    row = sbuf + 9 * (rb - b0);
+    k0 = inc_ptr[v];
+    k1 = inc_ptr[v + 1];
+  }
+  float D[9];  // this lane's share of the diagonal block
 #pragma unroll
-    for (int i = 0; i < 9; ++i) D[i] = 0.f;
-    int jd = 0;  // the diagonal block's position in the row
-    for (int k = k0; k < k1; k += 2) {
-      const bool two = k + 1 < k1;
-      HessInc h0, h1;
-      load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k, h0);
-      load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, two ? k + 1 : k, h1);
-      load_inc_x<PRE>(u, ul, h0);
-      load_inc_x<PRE>(u, ul, h1);
-      jd = (h0.pos >> (8 * h0.a)) & 255;
-      hess_inc<MODEL, PSD>(h0, row, rs, D, add_identity, cK, cM, tol, corot_exact, Kbuf);
-      if (two) hess_inc<MODEL, PSD>(h1, row, rs, D, add_identity, cK, cM, tol, corot_exact, Kbuf);
+  for (int i = 0; i < 9; ++i) D[i] = 0.f;
+  int jd = 0;
+  for (int k = k0 + sl; __any_sync(0xffffffffu, k - sl < k1); k += G) {
+    const bool have = k < k1;
+    HessInc h;
+    float K[4][9];
+    if (have) {
+      load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k, h);
+      load_inc_x<PRE>(u, ul, h);
+      hess_slab<MODEL, PSD>(h, K, add_identity, cK, cM, tol, corot_exact, Kbuf);
+      jd = (h.pos >> (8 * h.a)) & 255;
+#pragma unroll
+      for (int i = 0; i < 9; ++i)
+        D[i] += h.a == 0 ? K[0][i] : h.a == 1 ? K[1][i] : h.a == 2 ? K[2][i] : K[3][i];
     }
-    if (k1 > k0) {
 #pragma unroll
-      for (int kk = 0; kk < 3; ++kk)
+    for (int g = 0; g < G; ++g) {
+      if (have && sl == g)
 #pragma unroll
-        for (int ll = 0; ll < 3; ++ll) row[kk * rs + 3 * jd + ll] += D[3 * kk + ll];
+        for (int b = 0; b < 4; ++b)
+          if (b != h.a) hess_add_block(row, rs, (h.pos >> (8 * b)) & 255, K[b]);
+      __syncwarp();
     }
   }
+#pragma unroll
+  for (int o = 1; o < G; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < 9; ++i) D[i] += __shfl_xor_sync(0xffffffffu, D[i], o);
+  if (sl == 0 && k1 > k0) hess_add_block(row, rs, jd, D);
   __syncthreads();
   float *out = values + 9ll * b0;
   for (int i = threadIdx.x; i < len; i += blockDim.x) out[i] = sbuf[i];
@@ -973,11 +988,13 @@ int gradient(bartels_ctx ctx, bartels_mesh_plan plan, int model, const Objective
 template <int MODEL, bool PSD>
 static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *u, int add_identity, float cK,
                          float cM, float tol, int corot_exact, float *values) {
-  const bool small = plan->hess_chunk == 64 && plan->chunk_v64;
+  const bool small = plan->hess_chunk == 64;
   const int smem = (small ? kChunkFloats / 2 : kChunkFloats) * (int)sizeof(float);
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
-    BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kChunkFloats * (int)sizeof(float)));
+    BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kChunkFloats * (int)sizeof(float)));
     attr_set = true;
   }
@@ -999,9 +1016,15 @@ static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *
     BT_LAUNCH(ctx, k_psd_eig<MODEL>, grid_for(ctx, plan->nT, pb), pb, 0, list, count, plan->rec32, u, ul,
               add_identity, tol, corot_exact, kbuf);
   }
-  BT_LAUNCH(ctx, (k_hess<MODEL, PSD>), small ? plan->nchunks64 : plan->nchunks, small ? 64 : kChunkMaxVerts, smem,
-            small ? plan->chunk_v64 : plan->chunk_v, plan->brp, plan->inc_ptr, plan->inc_tet, plan->inc_pos,
-            plan->rec32, u, ul, add_identity, cK, cM, tol, corot_exact, fslot, kbuf, values);
+  const int chunks = small ? plan->nchunks64 : plan->nchunks, verts = small ? 64 : kChunkMaxVerts;
+  const int *chunk_v = small ? plan->chunk_v64 : plan->chunk_v;
+#define BT_HG(G)                                                                                                  \
+  BT_LAUNCH(ctx, (k_hess<MODEL, PSD, G>), chunks, verts * G, smem, chunk_v, plan->brp, plan->inc_ptr,            \
+            plan->inc_tet, plan->inc_pos, plan->rec32, u, ul, add_identity, cK, cM, tol, corot_exact, fslot, kbuf, \
+            values)
+  if (plan->nV <= 128 * ctx->num_sms) BT_HG(4);  // at most two 64-vertex chunks per SM
+  else BT_HG(2);
+#undef BT_HG
   return BARTELS_OK;
 }
 

@@ -184,7 +184,7 @@ struct bartels_mesh_plan_s {
   // assembly chunks (consecutive vertex ranges whose values fit in shared memory)
   int *chunk_v = nullptr;     // nchunks + 1
   int nchunks = 0;
-  // half-size chunks (<= 64 vertices, 32 KB), made when the tuning asks for them
+  // half-size chunks (<= 64 vertices, 32 KB)
   int *chunk_v64 = nullptr;
   // sliced-ELL layout of the block rows (built on the first solve); w_sell holds
   // the FP32 values in it for the PCG loop's SpMV
@@ -192,7 +192,7 @@ struct bartels_mesh_plan_s {
   int nchunks64 = 0;
   // Hessian tuning: vertices per assembly CTA (128, or 64 with chunk_v64) and
   // threads per CTA of the PSD pre-pass kernels (64, 128 or 256)
-  int hess_chunk = 128, psd_block = 128;
+  int hess_chunk = 64, psd_block = 128;
   std::vector<int> h_brp, h_bcol, h_chunk_v;  // host copies
   // lazily built scalar CSR pattern (device)
   int *csr_rp = nullptr, *csr_col = nullptr;

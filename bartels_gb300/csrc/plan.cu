@@ -195,6 +195,7 @@ int plan_build(bartels_mesh_plan plan, const double *V, const int *E) {
     BT_CHECK(plan_refresh_records(plan));
   }
   plan->dphi_matches_rest = true;
+  BT_CHECK(plan_chunks64(plan));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
   return BARTELS_OK;
 }
@@ -257,7 +258,8 @@ void FactorPattern::release() {
 // Lower / upper storage maps of a triangular factor on the plan's block
 // pattern (rows are sorted, so the lower part of a row is a prefix of it).
 // Chunks of at most 64 consecutive vertices whose values fit in 32 KB: the
-// assembly's smaller CTA shape (more CTAs per SM, less shared memory each).
+// assembly's smaller and default CTA shape (more CTAs per SM, less shared memory
+// each; 789 against 871 us at n = 96).
 int plan_chunks64(bartels_mesh_plan plan) {
   if (plan->chunk_v64) return BARTELS_OK;
   constexpr int kVerts = 64, kFloats = kChunkFloats / 2;
