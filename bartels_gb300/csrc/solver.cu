@@ -25,6 +25,7 @@
 #include "amg_internal.cuh"
 #include "lpcg_internal.cuh"
 #include "pcg_common.cuh"
+#include "pcg_small.cuh"
 #include "sell.cuh"
 
 namespace bartels {
@@ -744,6 +745,7 @@ struct PcgOperator {
   int n = 0;
   const int *rp = nullptr, *ci = nullptr;
   const double *values64 = nullptr;  // exact values for the FP64 refinement residual
+  const int *h_rp = nullptr;         // host copy of rp
   // factor preconditioner z = G^T G r (block layout only): lower and upper storage
   const __nv_bfloat16 *gl = nullptr, *gu = nullptr;
   const FactorPattern *fp = nullptr;
@@ -981,6 +983,18 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
                o_pb = take(4ull * n), o_ap = take(4ull * n), o_minv = take(24ull * nb), o_rres = take(4ull * n),
                o_xh = take(4ull * n), o_xl = take(4ull * n), o_bh = take(4ull * n), o_bl = take(4ull * n),
                o_pa8 = take(8ull * nparts), o_pb8 = take(8ull * nparts), o_st = take(sizeof(PcgState));
+  // small block-Jacobi systems: the inner solve as one cluster launch
+  PcgSmall small;
+  std::vector<int> small_off, small_rp;
+  const int *h_rp = op.h_rp;
+  if (blk && !op.mg && !op.gl && (int64_t)n <= 65536) {
+    small_rp.assign(n + 1, 0);
+    for (int i = 0; i < n; ++i)
+      small_rp[i + 1] = small_rp[i] + 3 * (op.plan->h_brp[i / 3 + 1] - op.plan->h_brp[i / 3]);
+    h_rp = small_rp.data();
+  }
+  bool is_small = !op.mg && !op.gl && h_rp && pcg_small_plan(n, h_rp, small, small_off);
+  const size_t o_small = take(is_small ? pcg_small_bytes(small) : 0);
   BT_CHECK(wbuf.ensure(off));
   char *base = wbuf.as<char>();
   PcgWork w;
@@ -1023,14 +1037,26 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     return rep->converged ? BARTELS_OK : fail(BARTELS_E_NONFINITE, "non-finite right-hand side");
   }
   const double target = prm.rel_tol * bnorm;
+  // its sums are float pairs: keep the squares well inside the float range
+  is_small = is_small && bnorm < 1e12 && bnorm > 1e-9 && target > 1e-18;
   // CUDA graph of a fixed number of PCG iterations (kernels no-op once done)
   const int chunk = op.mg ? 8 : 16;  // fixed-length fallback only
   cudaGraphExec_t exec = nullptr;
   int64_t graph_launches = 0;
   bool device_loop = false;
-  BT_CHECK(build_loop_graph(
-      ctx, w.st, [&](int k) { return pcg_enqueue_iters(ctx, op, w, n, nb, k); }, chunk, &exec, &graph_launches,
-      &device_loop));
+  if (is_small) {
+    const int *rp = op.rp, *ci = op.ci;
+    if (blk) {
+      BT_CHECK(plan_build_csr_pattern(op.plan));
+      rp = op.plan->csr_rp;
+      ci = op.plan->csr_col;
+    }
+    BT_CHECK(pcg_small_fill(ctx, small, base + o_small, small_off, rp, ci, op.values, op.pinned));
+  } else {
+    BT_CHECK(build_loop_graph(
+        ctx, w.st, [&](int k) { return pcg_enqueue_iters(ctx, op, w, n, nb, k); }, chunk, &exec, &graph_launches,
+        &device_loop));
+  }
   int status = BARTELS_OK;
   double rel = 0.0;
   PcgState hs{};
@@ -1070,7 +1096,12 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     const double abs2 = (0.5 * target) * (0.5 * target);
     const int cont = (pass > 0 && !prm.restart) ? 1 : 0;
     const int it0 = cont ? hs.it : 0;
-    if (op.mg) {
+    if (is_small) {
+      BT_CHECK(pcg_small_run(ctx, small, w.rres, w.minv, w.x, w.pa, w.st, prm.inner_rel_tol * prm.inner_rel_tol, abs2,
+                             prm.max_iters - rep->iterations, cont));
+      BT_CUDA(cudaMemcpyAsync(&hs, w.st, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx->stream));
+      BT_CUDA(cudaStreamSynchronize(ctx->stream));
+    } else if (op.mg) {
       BT_LAUNCH_PDL(ctx, k_pcg_init_f, gv, 256, 0, n, w.rres, w.x, w.r, w.pa, w.pb, w.part_a, w.st,
                 prm.inner_rel_tol * prm.inner_rel_tol, abs2, prm.max_iters - rep->iterations, cont);
       BT_CHECK(pcg_enqueue_mg(ctx, op, w, n, false));
@@ -1082,7 +1113,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
       BT_LAUNCH_PDL(ctx, k_pcg_init, gv, 256, 0, nb, n, w.rres, w.minv, w.x, w.r, w.z, w.pa, w.pb, w.part_a, w.part_b,
                 w.st, prm.inner_rel_tol * prm.inner_rel_tol, abs2, prm.max_iters - rep->iterations, cont);
     }
-    for (;;) {
+    while (!is_small) {
       BT_CUDA(cudaGraphLaunch(exec, ctx->stream));
       BT_CUDA(cudaMemcpyAsync(&hs, w.st, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx->stream));
       BT_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1100,7 +1131,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     rep->iterations += hs.it - it0;
     BT_LAUNCH(ctx, k_axpy64, grid_vec(ctx, n), 256, 0, n, w.x, x, w.xh, w.xl);
   }
-  cudaGraphExecDestroy(exec);
+  if (exec) cudaGraphExecDestroy(exec);
   return status;
 }
 
@@ -2313,6 +2344,7 @@ int csr_search_direction(bartels_ctx ctx, int n, const int *rp, const int *ci, c
   op.ci = dci;
   op.values = dv32;
   op.values64 = dv64;
+  op.h_rp = rp;
   int s = pcg_solve(ctx, op, n, db, dx, ctx->stage_d, prm, rep);
   BT_CUDA(cudaMemcpyAsync(d, dx, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
