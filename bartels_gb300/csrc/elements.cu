@@ -651,6 +651,53 @@ __device__ __forceinline__ void hess_add_block(float *row, int rs, int j, const 
     for (int ll = 0; ll < 3; ++ll) p[kk * rs + ll] = t[3 * kk + ll] + K[3 * kk + ll];
 }
 
+// One unprojected incidence of the one-lane form: the off-diagonal blocks into
+// the staged rows, the diagonal block into D.
+template <int MODEL>
+__device__ __forceinline__ void hess_inc(const HessInc &h, float *row, int rs, float *D, int add_identity, float cK,
+                                         float cM, int corot_exact) {
+  const int a = h.a;
+  float phi[4][3], K[4][9], F[9], pa[3];
+  phi4(h.r.dphi, phi);
+  elem_F_from<MODEL>(h.r, h.x[0], h.x[1], h.x[2], h.x[3], h.xl[0], h.xl[1], h.xl[2], h.xl[3], add_identity, F);
+  const float pv[2] = {cK * h.r.pv[0], cK * h.r.pv[1]};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) pa[d] = a == 0 ? phi[0][d] : a == 1 ? phi[1][d] : a == 2 ? phi[2][d] : phi[3][d];
+  with_law<MODEL>(F, pv, corot_exact, [&](const auto &law) {
+#pragma unroll
+    for (int b = 1; b < 4; ++b) law.block(pa, phi[b], K[b]);
+  });
+#pragma unroll
+  for (int i = 0; i < 9; ++i) K[0][i] = -(K[1][i] + K[2][i] + K[3][i]);
+  if (cM != 0.f) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float m = cM * h.r.mass * (a == b ? 0.1f : 0.05f);
+      K[b][0] += m;
+      K[b][4] += m;
+      K[b][8] += m;
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    if (b == a) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) D[i] += K[b][i];
+    } else {
+      const int j = (h.pos >> (8 * b)) & 255;
+#pragma unroll
+      for (int kk = 0; kk < 3; ++kk)
+#pragma unroll
+        for (int ll = 0; ll < 3; ++ll) row[kk * rs + 3 * j + ll] += K[b][3 * kk + ll];
+    }
+  }
+}
+
+// Laws without an SVD, unprojected: few registers and few instructions per incidence.
+constexpr bool hess_cheap(int model, bool psd) {
+  return !psd && model >= 0 && model != MODEL_COROT && model != MODEL_ARAP;
+}
+
 // One CTA per chunk of consecutive vertices, G lanes per vertex. The lanes take
 // the vertex's incidences G at a time in tet order, evaluate the 3x12 slabs (row
 // block a) of the element Hessian B^T d2psi B vol at the same time
@@ -664,11 +711,10 @@ __device__ __forceinline__ void hess_add_block(float *row, int rs, int j, const 
 // Bound by the L1 / shared-memory pipe (fully divergent 16-byte record loads and
 // the staged rows' read-modify-writes) and, on small meshes, by a lane's chain
 // of evaluations. n = 96 without projection: one lane per vertex 855 us (12
-// warps per SM, 78% of the pipe), two lanes 760 us, four 1,094 (the adds are
-// issued once per lane of the group); 1.05M tets with projection 375 / 274 /
-// 354. On 135k tets (25k vertices): 101 / 62 / 82, on 15.6k vertices two lanes
-// 39, four 34. So two lanes, and four where the chunks leave most SMs short of
-// work (launch_hess_t).
+// warps per SM, 78% of the pipe), two lanes 720 us, four 940 (the adds are issued
+// once per lane of the group); 1.05M tets with projection 375 / 270 / 300.
+// 18-KB chunks of 32 vertices: 757 us per call, 789 with 64 vertices, 871 with
+// 128. launch_hess_t chooses the lanes.
 template <int MODEL, bool PSD, int G>
 __global__ void __launch_bounds__(kChunkMaxVerts * G, 4 / G)
 k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *__restrict__ inc_ptr,
@@ -697,26 +743,51 @@ k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *
 #pragma unroll
   for (int i = 0; i < 9; ++i) D[i] = 0.f;
   int jd = 0;
-  for (int k = k0 + sl; __any_sync(0xffffffffu, k - sl < k1); k += G) {
-    const bool have = k < k1;
-    HessInc h;
-    float K[4][9];
-    if (have) {
-      load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k, h);
-      load_inc_x<PRE>(u, ul, h);
-      hess_slab<MODEL, PSD>(h, K, add_identity, cK, cM, tol, corot_exact, Kbuf);
-      jd = (h.pos >> (8 * h.a)) & 255;
-#pragma unroll
-      for (int i = 0; i < 9; ++i)
-        D[i] += h.a == 0 ? K[0][i] : h.a == 1 ? K[1][i] : h.a == 2 ? K[2][i] : K[3][i];
+  if constexpr (G == 1) {
+    // one lane: two incidences' load chains in flight, added in order
+    for (int k = k0; k < k1; k += 2) {
+      HessInc h0, h1;
+      const bool two = k + 1 < k1;
+      load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k, h0);
+      load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, two ? k + 1 : k, h1);
+      load_inc_x<PRE>(u, ul, h0);
+      load_inc_x<PRE>(u, ul, h1);
+      jd = (h0.pos >> (8 * h0.a)) & 255;
+      hess_inc<MODEL>(h0, row, rs, D, add_identity, cK, cM, corot_exact);
+      if (two) hess_inc<MODEL>(h1, row, rs, D, add_identity, cK, cM, corot_exact);
     }
+  } else {
+    // where the registers allow it the next incidence's record is loaded while this one is evaluated
+    constexpr bool AHEAD = G == 2 && hess_cheap(MODEL, PSD);
+    HessInc next;
+    if constexpr (AHEAD) {
+      if (k0 + sl < k1) load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k0 + sl, next);
+    }
+    for (int k = k0 + sl; __any_sync(0xffffffffu, k - sl < k1); k += G) {
+      const bool have = k < k1;
+      HessInc h;
+      float K[4][9];
+      if constexpr (AHEAD) h = next;
+      if (have) {
+        if constexpr (!AHEAD) load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k, h);
+        load_inc_x<PRE>(u, ul, h);
+        if constexpr (AHEAD) {
+          if (k + G < k1) load_inc_head<PRE>(inc_tet, inc_pos, rec, fslot, k + G, next);
+        }
+        hess_slab<MODEL, PSD>(h, K, add_identity, cK, cM, tol, corot_exact, Kbuf);
+        jd = (h.pos >> (8 * h.a)) & 255;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (have && sl == g)
+        for (int i = 0; i < 9; ++i)
+          D[i] += h.a == 0 ? K[0][i] : h.a == 1 ? K[1][i] : h.a == 2 ? K[2][i] : K[3][i];
+      }
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if (b != h.a) hess_add_block(row, rs, (h.pos >> (8 * b)) & 255, K[b]);
-      __syncwarp();
+      for (int g = 0; g < G; ++g) {
+        if (have && sl == g)
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+            if (b != h.a) hess_add_block(row, rs, (h.pos >> (8 * b)) & 255, K[b]);
+        __syncwarp();
+      }
     }
   }
 #pragma unroll
@@ -989,13 +1060,16 @@ template <int MODEL, bool PSD>
 static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *u, int add_identity, float cK,
                          float cM, float tol, int corot_exact, float *values) {
   const bool small = plan->hess_chunk == 64;
-  const int smem = (small ? kChunkFloats / 2 : kChunkFloats) * (int)sizeof(float);
+  const int smem = (small ? kSmallFloats : kChunkFloats) * (int)sizeof(float);
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
     BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kChunkFloats * (int)sizeof(float)));
     BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kChunkFloats * (int)sizeof(float)));
+    if constexpr (hess_cheap(MODEL, PSD))
+      BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   kChunkFloats * (int)sizeof(float)));
     attr_set = true;
   }
   const int pb = plan->psd_block;
@@ -1016,13 +1090,29 @@ static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *
     BT_LAUNCH(ctx, k_psd_eig<MODEL>, grid_for(ctx, plan->nT, pb), pb, 0, list, count, plan->rec32, u, ul,
               add_identity, tol, corot_exact, kbuf);
   }
-  const int chunks = small ? plan->nchunks64 : plan->nchunks, verts = small ? 64 : kChunkMaxVerts;
+  const int chunks = small ? plan->nchunks64 : plan->nchunks, verts = small ? kSmallVerts : kChunkMaxVerts;
   const int *chunk_v = small ? plan->chunk_v64 : plan->chunk_v;
 #define BT_HG(G)                                                                                                  \
   BT_LAUNCH(ctx, (k_hess<MODEL, PSD, G>), chunks, verts * G, smem, chunk_v, plan->brp, plan->inc_ptr,            \
             plan->inc_tet, plan->inc_pos, plan->rec32, u, ul, add_identity, cK, cM, tol, corot_exact, fslot, kbuf, \
             values)
-  if (plan->nV <= 128 * ctx->num_sms) BT_HG(4);  // at most two 64-vertex chunks per SM
+  // Four lanes while a vertex's pair of lanes would leave most SMs short of work
+  // (15.6k vertices: 31 us, two lanes 38). The cheap laws' one-lane form runs in
+  // one wave of three 128-vertex chunks per SM, so its time hardly grows up to
+  // there; the two-lane form's second wave starts at ~190 vertices per SM on a
+  // mesh numbered without locality. Shuffled balls, one lane / two: 27.6k
+  // vertices 66 / 60 us, 30.1k 67 / 72, 37.5k 67 / 78, 56.2k 94 / 112, 63.4k (a
+  // second wave) 153 / 128; boxes: 35.9k 52 / 43, 50.7k 64 / 69, 59.3k 96 / 72.
+  const int64_t nV = plan->nV, sms = ctx->num_sms;
+  if constexpr (hess_cheap(MODEL, PSD)) {
+    if (nV > 190 * sms && plan->nchunks <= 3 * sms) {
+      BT_LAUNCH(ctx, (k_hess<MODEL, PSD, 1>), plan->nchunks, kChunkMaxVerts, kChunkFloats * (int)sizeof(float),
+                plan->chunk_v, plan->brp, plan->inc_ptr, plan->inc_tet, plan->inc_pos, plan->rec32, u, ul,
+                add_identity, cK, cM, tol, corot_exact, fslot, kbuf, values);
+      return BARTELS_OK;
+    }
+  }
+  if (nV <= 128 * sms) BT_HG(4);
   else BT_HG(2);
 #undef BT_HG
   return BARTELS_OK;

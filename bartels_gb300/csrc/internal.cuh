@@ -184,7 +184,7 @@ struct bartels_mesh_plan_s {
   // assembly chunks (consecutive vertex ranges whose values fit in shared memory)
   int *chunk_v = nullptr;     // nchunks + 1
   int nchunks = 0;
-  // half-size chunks (<= 64 vertices, 32 KB)
+  // the small shape's chunks (kSmallVerts)
   int *chunk_v64 = nullptr;
   // sliced-ELL layout of the block rows (built on the first solve); w_sell holds
   // the FP32 values in it for the PCG loop's SpMV
@@ -222,11 +222,14 @@ namespace bartels {
 
 constexpr int kChunkFloats = 16384;  // 64 KB of shared memory per assembly CTA
 constexpr int kChunkMaxVerts = 128;
+// the small shape: 18 KB, 32 vertices of the usual 14 - 15 blocks
+constexpr int kSmallFloats = 4608;
+constexpr int kSmallVerts = 32;
 
 
 // Kernel-side entry points implemented in the .cu files.
 int plan_build(bartels_mesh_plan plan, const double *V_host, const int *E_host);
-// the half-size assembly chunks (built once, on first use)
+// the small shape's assembly chunks (built once, on first use)
 int plan_chunks64(bartels_mesh_plan plan);
 int plan_refresh_records(bartels_mesh_plan plan);
 int plan_build_csr_pattern(bartels_mesh_plan plan);

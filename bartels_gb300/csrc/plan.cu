@@ -257,18 +257,17 @@ void FactorPattern::release() {
 
 // Lower / upper storage maps of a triangular factor on the plan's block
 // pattern (rows are sorted, so the lower part of a row is a prefix of it).
-// Chunks of at most 64 consecutive vertices whose values fit in 32 KB: the
-// assembly's smaller and default CTA shape (more CTAs per SM, less shared memory
-// each; 789 against 871 us at n = 96).
+// Chunks of at most kSmallVerts consecutive vertices whose values fit in
+// kSmallFloats: the assembly's smaller and default CTA shape (the tuning's "64").
 int plan_chunks64(bartels_mesh_plan plan) {
   if (plan->chunk_v64) return BARTELS_OK;
-  constexpr int kVerts = 64, kFloats = kChunkFloats / 2;
+  constexpr int kVerts = kSmallVerts, kFloats = kSmallFloats;
   std::vector<int> chunks{0};
   int start = 0;
   int64_t floats = 0;
   for (int v = 0; v < plan->nV; ++v) {
     const int64_t need = 9ll * (plan->h_brp[v + 1] - plan->h_brp[v]);
-    if (need > kFloats) return fail(BARTELS_E_UNSUPPORTED, "vertex row too long for the half-size chunks");
+    if (need > kFloats) return fail(BARTELS_E_UNSUPPORTED, "vertex row too long for the small chunks");
     if (v - start >= kVerts || floats + need > kFloats) {
       chunks.push_back(v);
       start = v;

@@ -2111,12 +2111,12 @@ int plan_pcg_spmv_time(bartels_ctx ctx, bartels_mesh_plan plan, const float *val
 // Hessian autotuner: time the fused PSD-projected assembly at positions q
 // (3 warm-up + 5 timed calls, CUDA events on the context's stream, best of
 // three rounds over the candidates) for every
-// pair of assembly CTA shape (128 vertices / 64 KB or 64 vertices / 32 KB of
-// shared memory) and PSD pre-pass block size (64, 128, 256 threads); keep the
+// pair of assembly CTA shape (128 vertices / 64 KB or, named 64, the small shape's
+// 32 vertices / 18 KB of shared memory) and PSD pre-pass block size (64, 128, 256 threads); keep the
 // fastest in the plan and in the context's cache for the size bucket
 // floor(log2 nV), which later plans of that bucket take without timing. The
-// assembled values do not depend on the choice (each entry is still summed by
-// its row's thread in tet order).
+// assembled values do not depend on the choice (each entry is summed in
+// the same order under both shapes).
 int plan_autotune_hessian(bartels_ctx ctx, bartels_mesh_plan plan, int model, const double *q, int force,
                           int *chunk_out, int *block_out) {
   int bucket = 0;
@@ -2127,7 +2127,7 @@ int plan_autotune_hessian(bartels_ctx ctx, bartels_mesh_plan plan, int model, co
     plan->hess_chunk = hit->second.first;
     plan->psd_block = hit->second.second;
   } else {
-    // the half-size chunks exist unless a vertex row needs more than their shared memory
+    // the small shape's chunks exist unless a vertex row needs more than their shared memory
     const bool have64 = plan_chunks64(plan) == BARTELS_OK;
     BT_CHECK(plan->w_u.ensure(2 * sizeof(float4) * (size_t)plan->nV));
     BT_CHECK(plan->w_values.ensure(sizeof(float) * 9 * (size_t)plan->nnzb));

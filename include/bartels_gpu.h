@@ -469,8 +469,9 @@ int bartels_plan_pcg_spmv_time_d(bartels_ctx ctx, bartels_mesh_plan plan, const 
                                  float *y_d, int reps, double *us_per_launch);
 
 /* Hessian autotuner: times the fused simple_psd_fix-projected assembly of the
- * plan at device positions q_d for the assembly's CTA shapes (128 vertices
- * per CTA with 64 KB of shared memory, or 64 vertices with 32 KB) and the PSD
+ * plan at device positions q_d for the assembly's CTA shapes (128: 128 vertices
+ * per CTA with 64 KB of shared memory; 64: the small shape, 32 vertices with
+ * 18 KB) and the PSD
  * pre-pass block sizes (64, 128, 256 threads), keeps the fastest pair for the
  * plan's Hessians and caches it in the context per size bucket floor(log2 nV)
  * (reused by later plans of that bucket unless force != 0). The assembled

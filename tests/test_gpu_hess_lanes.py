@@ -1,7 +1,8 @@
-"""The assembly kernel with two and four lanes per vertex, against the oracle.
+"""The assembly kernel with one, two and four lanes per vertex, against the oracle.
 
-Mesh sizes on both sides of the rule that picks the lane count (four while the
-vertices fit two 64-vertex chunks per SM), around a chunk's 64 vertices, and a
+Mesh sizes on all sides of the rule that picks the lane count (four up to 128
+vertices per SM, one for the cheap laws from 190 up to three chunks per SM, two
+elsewhere; on 152 SMs 22.0k is above the first line, 42.9k between the others), and a
 shuffled numbering with uneven incidence counts; with and without projection,
 and under both CTA shapes (whose values must be the same bits)."""
 import numpy as np
@@ -25,7 +26,7 @@ def _mesh(kind):
     return V, E, 1.0 / n
 
 
-@pytest.mark.parametrize("kind", ["cube1", "cube3", "shuf4", "shuf12", "cube27"])
+@pytest.mark.parametrize("kind", ["cube1", "cube3", "shuf4", "shuf12", "cube27", "shuf34"])
 @pytest.mark.parametrize("psd", [None, 1e-6])
 def test_values_match_the_oracle(kind, psd):
     import bartels_gb300 as bg
