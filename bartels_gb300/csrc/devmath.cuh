@@ -514,6 +514,142 @@ __device__ __forceinline__ void with_law64(int model, const double *F, const dou
 }
 #endif
 
+// Rotation of the polar decomposition F = R C (the R = U V^T of the rotation-
+// variant SVD) for det F > 0 and singular values within a factor of 10; false
+// otherwise, and nothing is said about R. An SVD's FP64 sweeps cost ~800
+// operations on a unit that runs 1/64 of the FP32 rate, and neither the energy
+// nor the stress of the corotational law needs U, S and V apart. So: F V / S V^T
+// in FP32 (off by ~1e-6), taken to FP64 through its quaternion, which makes R
+// orthonormal to rounding; then Newton steps R <- exp([w]) R on the symmetry of
+// F R^T, (tr(F R^T) I - F R^T) w = sum_j r_j x f_j, whose right-hand side is
+// FP64 and whose matrix and solution are FP32: each step gains a factor of
+// ~1e-5, so one leaves R off by ~1e-11 (the energy is stationary in R: second
+// order in that) and two by rounding. ~110 and ~135 FP64 operations.
+template <int STEPS>
+BT_HD bool polar_rot(const double *F, double *R) {
+  float f[9], A[9], V[9], B[9];
+  for (int i = 0; i < 9; ++i) {
+    f[i] = (float)F[i];
+    V[i] = (i % 4 == 0) ? 1.f : 0.f;
+  }
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j)
+      A[i + 3 * j] = f[3 * i] * f[3 * j] + f[1 + 3 * i] * f[1 + 3 * j] + f[2 + 3 * i] * f[2 + 3 * j];
+  for (int s = 0; s < 6; ++s) {
+    const float off = A[3] * A[3] + A[6] * A[6] + A[7] * A[7];
+    const float dia = A[0] * A[0] + A[4] * A[4] + A[8] * A[8];
+    if (off <= 1e-14f * dia) break;
+    jacobi_rot(A, V, 0, 1);
+    jacobi_rot(A, V, 0, 2);
+    jacobi_rot(A, V, 1, 2);
+  }
+  float n[3];
+  for (int j = 0; j < 3; ++j) {
+    for (int i = 0; i < 3; ++i) B[i + 3 * j] = f[i] * V[3 * j] + f[i + 3] * V[1 + 3 * j] + f[i + 6] * V[2 + 3 * j];
+    n[j] = B[3 * j] * B[3 * j] + B[1 + 3 * j] * B[1 + 3 * j] + B[2 + 3 * j] * B[2 + 3 * j];
+  }
+  const float big = bt_max(n[0], bt_max(n[1], n[2])), small = -bt_max(-n[0], bt_max(-n[1], -n[2]));
+  if (!(det3(f) > 0.f && big > 1e-12f && big < 1e12f && small > 0.01f * big)) return false;
+  float r[9];
+  for (int j = 0; j < 3; ++j) {
+    const float q = 1.f / bt_sqrt(n[j]);
+    for (int i = 0; i < 3; ++i) B[i + 3 * j] *= q;
+  }
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) r[i + 3 * j] = B[i] * V[j] + B[i + 3] * V[j + 3] + B[i + 6] * V[j + 6];
+  // quaternion of r up to its scale
+  const float tr = r[0] + r[4] + r[8], a0 = r[5] - r[7], a1 = r[6] - r[2], a2 = r[1] - r[3];
+  float qw, qx, qy, qz;
+  if (tr > 0.f) {
+    qw = 1.f + tr, qx = a0, qy = a1, qz = a2;
+  } else if (r[0] >= r[4] && r[0] >= r[8]) {
+    qw = a0, qx = 1.f + r[0] - r[4] - r[8], qy = r[1] + r[3], qz = r[2] + r[6];
+  } else if (r[4] >= r[8]) {
+    qw = a1, qx = r[1] + r[3], qy = 1.f + r[4] - r[0] - r[8], qz = r[5] + r[7];
+  } else {
+    qw = a2, qx = r[2] + r[6], qy = r[5] + r[7], qz = 1.f + r[8] - r[0] - r[4];
+  }
+  const double w = qw, x = qx, y = qy, z = qz;
+  const double s = 2.0 / (w * w + x * x + y * y + z * z);
+  const double X = s * x, Y = s * y, Z = s * z;
+  R[0] = 1.0 - (y * Y + z * Z);
+  R[4] = 1.0 - (x * X + z * Z);
+  R[8] = 1.0 - (x * X + y * Y);
+  const double xy = x * Y, xz = x * Z, yz = y * Z;
+  R[1] = xy + w * Z;
+  R[3] = xy - w * Z;
+  R[6] = xz + w * Y;
+  R[2] = xz - w * Y;
+  R[5] = yz + w * X;
+  R[7] = yz - w * X;
+  // inverse of tr(N) I - N, N the symmetric part of F R^T
+  float N[6];  // 00 11 22 01 02 12
+  for (int i = 0; i < 3; ++i) N[i] = f[i] * r[i] + f[i + 3] * r[i + 3] + f[i + 6] * r[i + 6];
+  for (int e = 0; e < 3; ++e) {
+    const int i = e == 2 ? 1 : 0, j = e == 0 ? 1 : 2;
+    N[3 + e] = -0.5f * (f[i] * r[j] + f[i + 3] * r[j + 3] + f[i + 6] * r[j + 6] + f[j] * r[i] + f[j + 3] * r[i + 3] +
+                        f[j + 6] * r[i + 6]);
+  }
+  const float d0 = N[1] + N[2], d1 = N[0] + N[2], d2 = N[0] + N[1];
+  const float c00 = d1 * d2 - N[5] * N[5], c01 = N[4] * N[5] - N[3] * d2, c02 = N[3] * N[5] - N[4] * d1;
+  const float c11 = d0 * d2 - N[4] * N[4], c12 = N[3] * N[4] - N[5] * d0, c22 = d0 * d1 - N[3] * N[3];
+  const float di = 1.f / (d0 * c00 + N[3] * c01 + N[4] * c02);
+  for (int it = 0; it < STEPS; ++it) {
+    double g[3] = {0.0, 0.0, 0.0};
+    for (int j = 0; j < 3; ++j) {
+      const double *p = R + 3 * j, *q = F + 3 * j;
+      g[0] += p[1] * q[2] - p[2] * q[1];
+      g[1] += p[2] * q[0] - p[0] * q[2];
+      g[2] += p[0] * q[1] - p[1] * q[0];
+    }
+    const float g0 = (float)g[0] * di, g1 = (float)g[1] * di, g2 = (float)g[2] * di;
+    const double w0 = c00 * g0 + c01 * g1 + c02 * g2, w1 = c01 * g0 + c11 * g1 + c12 * g2,
+                 w2 = c02 * g0 + c12 * g1 + c22 * g2;
+    for (int j = 0; j < 3; ++j) {
+      double *p = R + 3 * j;
+      double t[3] = {p[0], p[1], p[2]};
+      if (it == 0) {  // second order: orthonormal to |w|^3
+        t[0] = p[0] + 0.5 * (w1 * p[2] - w2 * p[1]);
+        t[1] = p[1] + 0.5 * (w2 * p[0] - w0 * p[2]);
+        t[2] = p[2] + 0.5 * (w0 * p[1] - w1 * p[0]);
+      }
+      p[0] += w1 * t[2] - w2 * t[1];
+      p[1] += w2 * t[0] - w0 * t[2];
+      p[2] += w0 * t[1] - w1 * t[0];
+    }
+  }
+  return true;
+}
+
+// corotational energy and stress from the signed singular values
+template <class T>
+BT_HD_NOINLINE T psi_corot_svd(const T *F, const T *pv) {
+  T U[9], S[3], V[9];
+  svd3(F, U, S, V);
+  T tr = S[0] + S[1] + S[2] - T(3);
+  return pv[1] * ((S[0] - T(1)) * (S[0] - T(1)) + (S[1] - T(1)) * (S[1] - T(1)) + (S[2] - T(1)) * (S[2] - T(1))) +
+         T(0.5) * pv[0] * tr * tr;
+}
+// with the reference's inversion fix (src/dpsi_stretch_dF.cpp:20-45)
+template <class T>
+BT_HD_NOINLINE void pk1_corot_svd(const T *F, const T *pv, T *P) {
+  T U[9], S[3], V[9];
+  svd3(F, U, S, V);
+  T det = S[0] * S[1] * S[2];
+  if (det <= T(-1e-10))
+    for (int i = 0; i < 3; ++i)
+      if (S[i] < T(0)) S[i] = -S[i];
+  if (det3(U) <= T(0))
+    for (int k = 0; k < 3; ++k) U[k + 6] = -U[k + 6];
+  if (det3(V) <= T(0))
+    for (int k = 0; k < 3; ++k) V[k + 6] = -V[k + 6];
+  T tr = S[0] + S[1] + S[2] - T(3), d[3];
+  for (int i = 0; i < 3; ++i) d[i] = T(2) * pv[1] * (S[i] - T(1)) + pv[0] * tr;
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j)
+      P[i + 3 * j] = U[i] * d[0] * V[j] + U[i + 3] * d[1] * V[j + 3] + U[i + 6] * d[2] * V[j + 6];
+}
+
 // ----------------------------------------------------------------------------
 // FP64 energy and first Piola-Kirchhoff stress (scaled by vol via pv)
 // ----------------------------------------------------------------------------
@@ -557,11 +693,20 @@ BT_HD T psi_model(int model, const T *F, const T *pv_in) {
     for (int i = 0; i < 9; ++i) trEE += E[i] * E[i];  // E symmetric: tr(E E) = sum E_ij^2
     return pv[1] * trEE + T(0.5) * pv[0] * trE * trE;
   }
-  T U[9], S[3], V[9];
-  svd3(F, U, S, V);
-  T tr = S[0] + S[1] + S[2] - T(3);
-  return pv[1] * ((S[0] - T(1)) * (S[0] - T(1)) + (S[1] - T(1)) * (S[1] - T(1)) + (S[2] - T(1)) * (S[2] - T(1))) +
-         T(0.5) * pv[0] * tr * tr;
+  if constexpr (sizeof(T) == 8) {
+    T R[9];
+    if (polar_rot<1>(F, R)) {
+      // sum (S_i - 1)^2 = |F - R|^2 and sum S_i - 3 = R : (F - R)
+      T e2 = T(0), tr = T(0);
+      for (int i = 0; i < 9; ++i) {
+        const T e = F[i] - R[i];
+        e2 += e * e;
+        tr += R[i] * e;
+      }
+      return pv[1] * e2 + T(0.5) * pv[0] * tr * tr;
+    }
+  }
+  return psi_corot_svd(F, pv);
 }
 
 template <class T>
@@ -585,8 +730,8 @@ BT_HD void pk1_model(int model, const T *F, const T *pv_in, T *P) {
     cof3(G, F);
     T J = F[0] * G[0] + F[1] * G[1] + F[2] * G[2];
     if (model == MODEL_NH) {
-      T a = T(2) * pv[0], b = T(2) * pv[0] / J, c = T(2) * pv[1] * (J - T(1));
-      for (int i = 0; i < 9; ++i) P[i] = a * F[i] - b * G[i] + c * G[i];
+      const T a = T(2) * pv[0], c = T(2) * pv[1] * (J - T(1)) - a / J;
+      for (int i = 0; i < 9; ++i) P[i] = a * F[i] + c * G[i];
     } else {
       T I1 = T(0);
       for (int i = 0; i < 9; ++i) I1 += F[i] * F[i];
@@ -611,22 +756,21 @@ BT_HD void pk1_model(int model, const T *F, const T *pv_in, T *P) {
       for (int j = 0; j < 3; ++j) P[i + 3 * j] = F[i] * S[3 * j] + F[i + 3] * S[3 * j + 1] + F[i + 6] * S[3 * j + 2];
     return;
   }
-  // corotational with the reference's inversion fix (src/dpsi_stretch_dF.cpp:20-45)
-  T U[9], S[3], V[9];
-  svd3(F, U, S, V);
-  T det = S[0] * S[1] * S[2];
-  if (det <= T(-1e-10))
-    for (int i = 0; i < 3; ++i)
-      if (S[i] < T(0)) S[i] = -S[i];
-  if (det3(U) <= T(0))
-    for (int k = 0; k < 3; ++k) U[k + 6] = -U[k + 6];
-  if (det3(V) <= T(0))
-    for (int k = 0; k < 3; ++k) V[k + 6] = -V[k + 6];
-  T tr = S[0] + S[1] + S[2] - T(3), d[3];
-  for (int i = 0; i < 3; ++i) d[i] = T(2) * pv[1] * (S[i] - T(1)) + pv[0] * tr;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j)
-      P[i + 3 * j] = U[i] * d[0] * V[j] + U[i + 3] * d[1] * V[j + 3] + U[i + 6] * d[2] * V[j + 6];
+  if constexpr (sizeof(T) == 8) {
+    T R[9];
+    if (polar_rot<2>(F, R)) {
+      // U (2 mu (S - 1) + lambda tr) V^T = 2 mu (F - R) + lambda (R : (F - R)) R
+      T tr = T(0);
+      for (int i = 0; i < 9; ++i) {
+        P[i] = F[i] - R[i];
+        tr += R[i] * P[i];
+      }
+      const T m = T(2) * pv[1], l = pv[0] * tr;
+      for (int i = 0; i < 9; ++i) P[i] = m * P[i] + l * R[i];
+      return;
+    }
+  }
+  pk1_corot_svd(F, pv, P);
 }
 
 // ----------------------------------------------------------------------------
@@ -647,15 +791,83 @@ BT_HD float bt_log1p(float x) { return std::log1p(x); }
 BT_HD float bt_expm1(float x) { return std::expm1(x); }
 #endif
 
-// j - log1p(j) (>= 0), series sum_{k>=2} (-1)^k j^k / k for |j| < 0.02
-template <class T>
-BT_HD T j_minus_log1p(T j) {
-  if (bt_abs(j) < T(0.02)) {
-    T s = T(0);
+// j - log1p(j) (>= 0), without cancellation. Table-driven (P. Tang, "Table-driven
+// implementation of the logarithm function", 1990): with c near 1 / (1 + j) from a
+// row of the table and d = c - 1 (exact), r = c (1 + j) - 1 = d + j c is at most
+// 0.025 and
+//   j - log1p(j) = [r - log1p(r)] - d j + (log c - d),
+// whose three parts are all O(j^2); r - log1p(r) is its series. Row k serves
+// j in [(k - 1/2) / 64, (k + 1/2) / 64]; row 0 has c = 1. 16 FP64 operations for
+// |j| < 11/16; a series below 0.02 and log1p above it took 14 and ~35, both in
+// a warp that has both.
+constexpr int kLogRows = 44;
+#ifdef __CUDACC__
+static __device__
+#endif
+    const double kLogTab[2 * kLogRows + 1][2] = {  // 1 / (1 + k / 64) rounded to FP32, less 1; its log less that
+    {2.200000047683716, -1.036849222976874}, {2.047619104385376, -0.9332584401226758},
+    {1.9090909957885742, -0.8412503359848963}, {1.7826087474822998, -0.7592198614253263},
+    {1.6666667461395264, -0.6858374633254782}, {1.559999942779541, -0.619992706639812},
+    {1.461538553237915, -0.5607519706468229}, {1.3703703880310059, -0.5073241632250826},
+    {1.2857143878936768, -0.45903577000572626}, {1.2068965435028076, -0.4153092938549001},
+    {1.133333444595337, -0.3756476907437576}, {1.0645160675048828, -0.33962021843268003}, {1.0, -0.3068528194400547},
+    {0.9393939971923828, -0.27701844549686927}, {0.8823529481887817, -0.24983038571998098},
+    {0.8285714387893677, -0.22503641133117408}, {0.7777777910232544, -0.20241363866911197},
+    {0.7297297716140747, -0.18176457668424065}, {0.6842105388641357, -0.1629136077802691},
+    {0.6410256624221802, -0.1457042121536388}, {0.6000000238418579, -0.12999637969496128},
+    {0.5609755516052246, -0.11566457220276423}, {0.523809552192688, -0.10259606848993312},
+    {0.4883720874786377, -0.09068912353781856}, {0.4545454978942871, -0.07985201865055447},
+    {0.4222222566604614, -0.07000163885672268}, {0.3913043737411499, -0.06106266824412173},
+    {0.3617020845413208, -0.05296663455667557}, {0.3333333730697632, -0.04565127081566031},
+    {0.30612242221832275, -0.03905965745837436}, {0.2799999713897705, -0.03313991580998675},
+    {0.2549020051956177, -0.027844519170014383}, {0.23076927661895752, -0.02312987458781073},
+    {0.20754718780517578, -0.018956003096464676}, {0.18518519401550293, -0.015286149769524887},
+    {0.16363632678985596, -0.012086460327623057}, {0.14285719394683838, -0.009325756618833173},
+    {0.12280702590942383, -0.006975202933721554}, {0.10344827175140381, -0.005008202663441594},
+    {0.08474576473236084, -0.0034001234157632863}, {0.06666672229766846, -0.002128149006034467},
+    {0.04918026924133301, -0.0011711059343284382}, {0.032258033752441406, -0.0005093652401839369},
+    {0.015873074531555176, -0.00012465982141804808}, {0.0, 0.0}, {-0.01538461446762085, -0.00011957113702183036},
+    {-0.030303001403808594, -0.000468627460623151}, {-0.04477614164352417, -0.0010334176708346697},
+    {-0.05882352590560913, -0.0018010921855354202}, {-0.0724637508392334, -0.0027596517719028083},
+    {-0.08571428060531616, -0.0038978724964355382}, {-0.09859156608581543, -0.005205246222279801},
+    {-0.1111111044883728, -0.006671923717430083}, {-0.12328767776489258, -0.008288687474407318},
+    {-0.13513511419296265, -0.010046871437148604}, {-0.14666664600372314, -0.011938359958528792},
+    {-0.15789473056793213, -0.013955518908146525}, {-0.16883116960525513, -0.01609116982007944},
+    {-0.1794871687889099, -0.018338561502494008}, {-0.18987339735031128, -0.02069134661132916},
+    {-0.19999998807907104, -0.023143548333977627}, {-0.20987653732299805, -0.025689526539188292},
+    {-0.2195122241973877, -0.02832397696009724}, {-0.22891569137573242, -0.031041870314097324},
+    {-0.238095223903656, -0.03383847295353443}, {-0.24705880880355835, -0.036709344769312376},
+    {-0.25581395626068115, -0.03965026035844503}, {-0.26436781883239746, -0.042657220187804705},
+    {-0.27272725105285645, -0.04572645026335623}, {-0.2808988690376282, -0.04885440709029154},
+    {-0.2888888716697693, -0.05203769108643728}, {-0.2967032790184021, -0.05527311899306689},
+    {-0.30434781312942505, -0.058557661933492086}, {-0.31182795763015747, -0.061888453094749184},
+    {-0.3191489577293396, -0.06526277284596048}, {-0.3263157606124878, -0.06867800478754367},
+    {-0.3333333134651184, -0.07213176484072403}, {-0.34020620584487915, -0.07562172003247725},
+    {-0.3469387888908386, -0.07914562690915829}, {-0.35353535413742065, -0.08270141356881999},
+    {-0.36000001430511475, -0.08628711067504681}, {-0.3663366436958313, -0.0899008056182402},
+    {-0.37254899740219116, -0.09354069713215085}, {-0.3786407709121704, -0.0972051246445678},
+    {-0.38461536169052124, -0.10089241683827728}, {-0.39047616720199585, -0.10460106141163084},
+    {-0.3962264060974121, -0.10832958975382209}, {-0.40186917781829834, -0.11207660494890402},
+    {-0.40740740299224854, -0.11584073332171874},
+};
+BT_HD double j_minus_log1p(double j) {
+#if defined(__CUDA_ARCH__) || !defined(__CUDACC__)
+  if (bt_abs(j) < 0.6875) {
+    const double v = j + 0x1.8p46;  // the low word of the sum holds rint(64 j)
+#ifdef __CUDA_ARCH__
+    const double2 e = __ldg(reinterpret_cast<const double2 *>(kLogTab[__double2loint(v) + kLogRows]));
+    const double d = e.x, t = e.y;
+#else
+    const int k = (int)(64.0 * (v - 0x1.8p46));
+    const double d = kLogTab[k + kLogRows][0], t = kLogTab[k + kLogRows][1];
+#endif
+    const double r = j * (1.0 + d) + d;  // 1 + d = c, exact
+    double s = -1.0 / 9.0;
 #pragma unroll
-    for (int k = 13; k >= 2; --k) s = s * j + ((k % 2 == 0) ? T(1) : T(-1)) / T(k);
-    return s * j * j;
+    for (int k = 8; k >= 2; --k) s = s * r + ((k % 2 == 0) ? 1.0 : -1.0) / k;
+    return s * r * r - d * j + t;
   }
+#endif
   return j - bt_log1p(j);
 }
 // expm1(y) - y, series sum_{k>=2} y^k / k! for |y| < 0.02
@@ -677,7 +889,8 @@ BT_HD T expm1_minus_y(T y) {
   return bt_expm1(y) - y;
 }
 
-// invariants of H: tr H, |H|^2, q2 = ((tr H)^2 - tr(H H))/2, det H, j = det(I + H) - 1
+// invariants of H: tr H, |H|^2, q2 = ((tr H)^2 - tr(H H))/2 as the sum of the
+// principal 2x2 minors, det H, j = det(I + H) - 1
 template <class T>
 struct DispInv {
   T tr, nrm2, q2, det, j;
@@ -685,11 +898,9 @@ struct DispInv {
     tr = H[0] + H[4] + H[8];
     nrm2 = T(0);
     for (int i = 0; i < 9; ++i) nrm2 += H[i] * H[i];
-    T trHH = T(0);
-    for (int i = 0; i < 3; ++i)
-      for (int k = 0; k < 3; ++k) trHH += H[i + 3 * k] * H[k + 3 * i];
-    q2 = T(0.5) * (tr * tr - trHH);
-    det = det3(H);
+    const T m0 = H[4] * H[8] - H[7] * H[5];
+    q2 = m0 + (H[0] * H[8] - H[6] * H[2]) + (H[0] * H[4] - H[3] * H[1]);
+    det = H[0] * m0 + H[3] * (H[7] * H[2] - H[1] * H[8]) + H[6] * (H[1] * H[5] - H[4] * H[2]);
     j = tr + q2 + det;
   }
 };
@@ -705,8 +916,7 @@ BT_HD T psi_model_disp(int model, const T *H, const T *pv) {
       return pv[0] * (d.nrm2 - T(2) * (d.q2 + d.det) + T(2) * g2) + pv[1] * d.j * d.j;
     // J^-2/3 I1 - 3 = 3 g1 + 2 g2 - 2 (q2 + det) + |H|^2 + e (2 tr H + |H|^2),
     // e = J^-2/3 - 1 = expm1(y), y = -2/3 ln J, g1 = expm1(y) - y
-    const T L = bt_log1p(d.j);
-    const T y = T(-2) / T(3) * L;
+    const T y = T(-2) / T(3) * (d.j - g2);
     const T g1 = expm1_minus_y(y);
     const T e = g1 + y;
     return pv[0] * (T(3) * g1 + T(2) * g2 - T(2) * (d.q2 + d.det) + d.nrm2 + e * (T(2) * d.tr + d.nrm2)) +

@@ -173,7 +173,9 @@ __global__ void k_prep_u(int nV, const double *__restrict__ x, const double *__r
 // ---------------------------------------------------------- FP64 energy -----
 // Displacement gradient H = F - I of tet r at positions q = q_base + scale x,
 // from FP64 displacements u = q - X when the element data belongs to the rest
-// shape X (exact rest: H = 0), else F - I from positions.
+// shape X (exact rest: H = 0), else F - I from positions. RAW: q = x (no base,
+// scale 1, no step), which spares twelve FP64 operations; the values are the same bits.
+template <bool RAW>
 __device__ __forceinline__ void disp_grad64(const TetRec64 &r, const double *__restrict__ x,
                                             const double *__restrict__ q_base, double scale,
                                             const double *__restrict__ X, const double *__restrict__ dx,
@@ -186,10 +188,14 @@ __device__ __forceinline__ void disp_grad64(const TetRec64 &r, const double *__r
     for (int d = 0; d < 3; ++d) {
       const int i = 3 * id[a] + d;
       double xv = x[i];
-      if (dx) xv += alpha * dx[i];
-      double base = q_base ? q_base[i] : 0.0;
-      if (X) base -= X[i];
-      u[a][d] = base + scale * xv;
+      if constexpr (RAW) {
+        u[a][d] = X ? xv - X[i] : xv;
+      } else {
+        if (dx) xv += alpha * dx[i];
+        double base = q_base ? q_base[i] : 0.0;
+        if (X) base -= X[i];
+        u[a][d] = base + scale * xv;
+      }
     }
   def_grad(H, u[0], u[1], u[2], u[3], r.dphi, false);
   if (!X) {
@@ -199,7 +205,10 @@ __device__ __forceinline__ void disp_grad64(const TetRec64 &r, const double *__r
   }
 }
 
-template <int MODEL>
+// Bound by the FP64 pipe (2 operations per clock and SM) for every law: n = 96
+// Neohookean 1,525 -> 1,101 us, ~100 operations per tet at 84% of the pipe's rate;
+// corotational energy and stress together, 413k tets, 1,630 -> 470 us (polar_rot).
+template <int MODEL, bool RAW>
 __global__ void k_energy(int nT, const TetRec64 *__restrict__ rec, const double *__restrict__ x,
                          const double *__restrict__ q_base, double scale, const double *__restrict__ X,
                          double mass_coeff, const double *__restrict__ x_hat, int ndof,
@@ -208,7 +217,7 @@ __global__ void k_energy(int nT, const TetRec64 *__restrict__ rec, const double 
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nT; t += gridDim.x * blockDim.x) {
     const TetRec64 &r = rec[t];
     double H[9];
-    disp_grad64(r, x, q_base, scale, X, nullptr, 0.0, H);
+    disp_grad64<RAW>(r, x, q_base, scale, X, nullptr, 0.0, H);
     acc += psi_model_disp<double>(MODEL, H, r.pv);
     if (mass_coeff != 0.0) {
       const int id[4] = {r.idx.x, r.idx.y, r.idx.z, r.idx.w};
@@ -240,7 +249,7 @@ __global__ void k_energy_elem(int nT, const TetRec64 *__restrict__ rec, const do
                               const double *__restrict__ X, double *__restrict__ e) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nT; t += gridDim.x * blockDim.x) {
     double H[9];
-    disp_grad64(rec[t], q, nullptr, 1.0, X, nullptr, 0.0, H);
+    disp_grad64<true>(rec[t], q, nullptr, 1.0, X, nullptr, 0.0, H);
     e[t] = psi_model_disp<double>(MODEL, H, rec[t].pv);
   }
 }
@@ -259,8 +268,8 @@ __global__ void k_energy_diff(int nT, const TetRec64 *__restrict__ rec, const do
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nT; t += gridDim.x * blockDim.x) {
     const TetRec64 &r = rec[t];
     double H0[9], H1[9];
-    disp_grad64(r, x, q_base, scale, X, nullptr, 0.0, H0);
-    disp_grad64(r, x, q_base, scale, X, dx, alpha, H1);
+    disp_grad64<false>(r, x, q_base, scale, X, nullptr, 0.0, H0);
+    disp_grad64<false>(r, x, q_base, scale, X, dx, alpha, H1);
     acc += psi_model_disp<double>(MODEL, H1, r.pv) - psi_model_disp<double>(MODEL, H0, r.pv);
     if (mass_coeff != 0.0) {
       const int id[4] = {r.idx.x, r.idx.y, r.idx.z, r.idx.w};
@@ -305,8 +314,8 @@ __global__ void k_energy_diff_seg(int nT, int nV, const TetRec64 *__restrict__ r
     }
     const TetRec64 &r = rec[t];
     double H0[9], H1[9];
-    disp_grad64(r, x, q_base, scale, X, nullptr, 0.0, H0);
-    disp_grad64(r, x, q_base, scale, X, dx, alpha, H1);
+    disp_grad64<false>(r, x, q_base, scale, X, nullptr, 0.0, H0);
+    disp_grad64<false>(r, x, q_base, scale, X, dx, alpha, H1);
     double acc = psi_model_disp<double>(MODEL, H1, r.pv) - psi_model_disp<double>(MODEL, H0, r.pv);
     if (mass_coeff != 0.0) {
       const int id[4] = {r.idx.x, r.idx.y, r.idx.z, r.idx.w};
@@ -351,8 +360,10 @@ __global__ void k_dot_partials(int n, const double *__restrict__ a, const double
 }
 
 // -------------------------------------------------------- FP64 gradient -----
-// element gradient (12 doubles per tet, AoS) of the objective
-template <int MODEL>
+// Element gradient (12 doubles per tet, AoS) of the objective. Bound by the FP64
+// pipe (n = 96 Neohookean 1,658 -> 1,284 us, ~125 operations). Node 0 takes
+// minus the sum of the others (phi_0 = -(phi_1 + phi_2 + phi_3)); RAW as in disp_grad64.
+template <int MODEL, bool RAW>
 __global__ void k_grad_elem(int nT, const TetRec64 *__restrict__ rec, const double *__restrict__ x,
                             const double *__restrict__ q_base, double scale, double mass_coeff,
                             const double *__restrict__ x_hat, double *__restrict__ ge) {
@@ -364,18 +375,16 @@ __global__ void k_grad_elem(int nT, const TetRec64 *__restrict__ rec, const doub
       for (int d = 0; d < 3; ++d) {
         double xv = x[3 * id[a] + d];
         xs[a][d] = xv;
-        q[a][d] = scale * xv + (q_base ? q_base[3 * id[a] + d] : 0.0);
+        q[a][d] = RAW ? xv : scale * xv + (q_base ? q_base[3 * id[a] + d] : 0.0);
       }
-    double F[9], P[9], phi[4][3];
+    double F[9], P[9];
     def_grad(F, q[0], q[1], q[2], q[3], r.dphi, false);
     pk1_model<double>(MODEL, F, r.pv, P);
-    phi4(r.dphi, phi);
+    if constexpr (!RAW)
+      for (int i = 0; i < 9; ++i) P[i] *= scale;
     double out[12];
-    for (int a = 0; a < 4; ++a) {
-      double g[3];
-      mv3(g, P, phi[a]);
-      for (int d = 0; d < 3; ++d) out[3 * a + d] = scale * g[d];
-    }
+    for (int a = 1; a < 4; ++a) mv3(out + 3 * a, P, r.dphi + 3 * (a - 1));
+    for (int d = 0; d < 3; ++d) out[d] = -(out[3 + d] + out[6 + d] + out[9 + d]);
     if (mass_coeff != 0.0) {
       double dd[4][3], s[3] = {0, 0, 0};
       for (int a = 0; a < 4; ++a)
@@ -399,6 +408,7 @@ __global__ void k_grad_gather(int nV, const int *__restrict__ inc_ptr, const int
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nV; v += gridDim.x * blockDim.x) {
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
     const int k1 = inc_ptr[v + 1];
+#pragma unroll 4
     for (int k = inc_ptr[v]; k < k1; ++k) {
       const int ta = __ldg(inc_tet + k);
       const double *p = ge + 12ll * (ta >> 2) + 3 * (ta & 3);
@@ -969,13 +979,18 @@ int energy(bartels_ctx ctx, bartels_mesh_plan plan, int model, const ObjectiveDe
            double *d_out) {
   BT_CHECK(ctx->partials.ensure(kRedBlocks * sizeof(double)));
   int g = grid_for(ctx, plan->nT, 256);
-  if (g > kRedBlocks) g = kRedBlocks;
+  // whole rounds of blocks over the SMs
+  if (g > kRedBlocks) g = ctx->num_sms < kRedBlocks ? kRedBlocks / ctx->num_sms * ctx->num_sms : kRedBlocks;
   double *part = ctx->partials.as<double>();
   const int ndof = 3 * plan->nV;
   const double *X = plan->dphi_matches_rest ? plan->X : nullptr;
-#define BT_EN(M)                                                                                                \
-  BT_LAUNCH(ctx, k_energy<M>, g, 256, 0, plan->nT, plan->rec64, x, obj.q_base, obj.scale, X, obj.mass_coeff,   \
+  const bool raw = !obj.q_base && obj.scale == 1.0;
+#define BT_EN2(M, RAW)                                                                                             \
+  BT_LAUNCH(ctx, (k_energy<M, RAW>), g, 256, 0, plan->nT, plan->rec64, x, obj.q_base, obj.scale, X, obj.mass_coeff, \
             obj.x_hat, ndof, obj.f_ext, obj.force_scale, part)
+#define BT_EN(M)               \
+  if (raw) BT_EN2(M, true);    \
+  else BT_EN2(M, false)
   switch (model) {
     case MODEL_NH: BT_EN(MODEL_NH); break;
     case MODEL_STVK: BT_EN(MODEL_STVK); break;
@@ -986,6 +1001,7 @@ int energy(bartels_ctx ctx, bartels_mesh_plan plan, int model, const ObjectiveDe
     default: return fail(BARTELS_E_INVALID_ARG, "unknown model");
   }
 #undef BT_EN
+#undef BT_EN2
   return reduce_sum(ctx, part, g, d_out);
 }
 
@@ -1039,8 +1055,13 @@ int gradient(bartels_ctx ctx, bartels_mesh_plan plan, int model, const Objective
   BT_CHECK(plan->w_grad_e.ensure(sizeof(double) * 12 * (size_t)plan->nT));
   double *ge = plan->w_grad_e.as<double>();
   const int gt = grid_for(ctx, plan->nT, 256);
-#define BT_GE(M) \
-  BT_LAUNCH(ctx, k_grad_elem<M>, gt, 256, 0, plan->nT, plan->rec64, x, obj.q_base, obj.scale, obj.mass_coeff, obj.x_hat, ge)
+  const bool raw = !obj.q_base && obj.scale == 1.0;
+#define BT_GE2(M, RAW)                                                                                        \
+  BT_LAUNCH(ctx, (k_grad_elem<M, RAW>), gt, 256, 0, plan->nT, plan->rec64, x, obj.q_base, obj.scale,          \
+            obj.mass_coeff, obj.x_hat, ge)
+#define BT_GE(M)               \
+  if (raw) BT_GE2(M, true);    \
+  else BT_GE2(M, false)
   switch (model) {
     case MODEL_NH: BT_GE(MODEL_NH); break;
     case MODEL_STVK: BT_GE(MODEL_STVK); break;
@@ -1051,6 +1072,7 @@ int gradient(bartels_ctx ctx, bartels_mesh_plan plan, int model, const Objective
     default: return fail(BARTELS_E_INVALID_ARG, "unknown model");
   }
 #undef BT_GE
+#undef BT_GE2
   BT_LAUNCH(ctx, k_grad_gather, grid_for(ctx, plan->nV, 256), 256, 0, plan->nV, plan->inc_ptr, plan->inc_tet, ge,
             obj.f_ext, obj.force_scale, obj.pinned, g);
   return BARTELS_OK;
@@ -1204,7 +1226,8 @@ int noalloc_gradient(bartels_ctx ctx, bartels_mesh_plan plan, int model, const d
   }
   if (plan->nT == 0) return BARTELS_OK;
   const int gt = grid_for(ctx, plan->nT, 256);
-#define BT_GN(M) BT_LAUNCH(ctx, k_grad_elem<M>, gt, 256, 0, plan->nT, plan->rec64, q_d, nullptr, 1.0, 0.0, nullptr, ge)
+#define BT_GN(M) \
+  BT_LAUNCH(ctx, (k_grad_elem<M, true>), gt, 256, 0, plan->nT, plan->rec64, q_d, nullptr, 1.0, 0.0, nullptr, ge)
   switch (model) {
     case MODEL_NH: BT_GN(MODEL_NH); break;
     case MODEL_STVK: BT_GN(MODEL_STVK); break;
