@@ -106,7 +106,8 @@ struct bartels_lpcg_s {
   float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
   __nv_bfloat16 *wbf = nullptr;
   int *err = nullptr;
-  double *scal = nullptr;  // device scalars: [0] trace, [1] logdiag sum, [2] n_free, [3] grad norm^2
+  double *scal = nullptr;  // device scalars: [0] trace, [1] logdiag sum, [2] n_free; [8..] the parts of the
+                           // gradient's and of the residual probe's norm^2
   int64_t step = 0;
   bool bf_dirty = true;
   bartels::DevBuf part;    // reduction partials
@@ -550,16 +551,18 @@ __device__ __forceinline__ void ghat_of(const float *rw, bool diag, float (&G)[3
   }
 }
 
-// u_p = Ghat^T w_p: row j gathers the transposed blocks Ghat_ij, i >= j.
+// u_p = Ghat^T w_p: row j gathers the transposed blocks Ghat_ij, i >= j. A grid row
+// per probe, as in the next kernel (15.6k vertices are 62 blocks: 41 and 75 us with
+// the probes in turn, now 21 and 35).
 __global__ void k_lp_gt_apply(int nV, int np, const int *__restrict__ brp, const int *__restrict__ bcol,
                               const int *__restrict__ diag_pos, const int *__restrict__ urp,
                               const int *__restrict__ up2low, const unsigned char *__restrict__ pinned,
                               const float *__restrict__ raw, const float *__restrict__ w, float *__restrict__ u) {
   const int n = 3 * nV;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nV; j += gridDim.x * blockDim.x) {
-    const int rb = brp[j], d = diag_pos[j], nb = brp[j + 1] - rb;
-    const bool pj = pinned && pinned[j];
-    for (int p = 0; p < np; ++p) {
+  for (int p = blockIdx.y; p < np; p += gridDim.y)
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nV; j += gridDim.x * blockDim.x) {
+      const int rb = brp[j], d = diag_pos[j], nb = brp[j + 1] - rb;
+      const bool pj = pinned && pinned[j];
       float s[3] = {0.f, 0.f, 0.f};
       if (!pj)
         for (int m = 0; m < nb - d; ++m) {
@@ -573,7 +576,6 @@ __global__ void k_lp_gt_apply(int nV, int np, const int *__restrict__ brp, const
         }
       for (int c = 0; c < 3; ++c) u[(int64_t)p * n + 3 * j + c] = s[c];
     }
-  }
 }
 
 // v_p = Ahat u_p (rows of pinned vertices 0); partials of sum_p u_p.v_p and of
@@ -586,10 +588,10 @@ k_lp_ahat_apply(int nV, int np, const int *__restrict__ brp, const int *__restri
                 double *__restrict__ part) {
   const int n = 3 * nV;
   double acc = 0.0, ld = 0.0, nf = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nV; i += gridDim.x * blockDim.x) {
-    const bool pv = pinned && pinned[i];
-    const int rb = brp[i], re = brp[i + 1];
-    for (int p = 0; p < np; ++p) {
+  for (int p = blockIdx.y; p < np; p += gridDim.y)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nV; i += gridDim.x * blockDim.x) {
+      const bool pv = pinned && pinned[i];
+      const int rb = brp[i], re = brp[i + 1];
       float s[3] = {0.f, 0.f, 0.f};
       if (!pv)
         for (int q = rb; q < re; ++q) {
@@ -604,13 +606,12 @@ k_lp_ahat_apply(int nV, int np, const int *__restrict__ brp, const int *__restri
         vv[(int64_t)p * n + 3 * i + k] = s[k];
         acc += (double)ui[k] * s[k];
       }
+      if (!pv && p == 0) {
+        const float *rw = raw + 9ll * (lrp[i] + diag_pos[i]);
+        ld += (double)rw[0] + rw[1] + rw[2];
+        nf += 3.0;
+      }
     }
-    if (!pv) {
-      const float *rw = raw + 9ll * (lrp[i] + diag_pos[i]);
-      ld += (double)rw[0] + rw[1] + rw[2];
-      nf += 3.0;
-    }
-  }
   __shared__ double red[3][8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double vals[3] = {acc, ld, nf};
@@ -624,20 +625,25 @@ k_lp_ahat_apply(int nV, int np, const int *__restrict__ brp, const int *__restri
     for (int k = 0; k < 3; ++k) {
       double x = 0.0;
       for (int i = 0; i < (int)(blockDim.x >> 5); ++i) x += red[k][i];
-      part[3ll * blockIdx.x + k] = x;
+      part[3ll * (blockIdx.y * gridDim.x + blockIdx.x) + k] = x;
     }
   }
 }
 
 // fixed-order sum of the partials into scal[0..2] (trace, logdiag, n_free)
 __global__ void k_lp_loss_sum(int nparts, int np, const double *__restrict__ part, double *__restrict__ scal) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = 0; i < nparts; ++i) {
-      a += part[3 * i];
-      b += part[3 * i + 1];
-      c += part[3 * i + 2];
-    }
+  double a = 0.0, b = 0.0, c = 0.0;
+  for (int i = threadIdx.x; i < nparts; i += 32) {
+    a += part[3 * i];
+    b += part[3 * i + 1];
+    c += part[3 * i + 2];
+  }
+  for (int o = 16; o; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  }
+  if (threadIdx.x == 0) {
     scal[0] = a / np;
     scal[1] = b;
     scal[2] = c;
@@ -860,50 +866,193 @@ __global__ void k_lp_add_left(int nV, const float *__restrict__ dha, float *__re
     dh[i] += dha[(i / kH) * 2 * kH + (i % kH)];
 }
 
-// Weight gradient partials: out[k][n] = sum_r A[r][k] * B[r][n] over the
-// block's row range (A == nullptr means a column of ones: bias gradient).
-template <class TB>
-__global__ void __launch_bounds__(256)
+// Weight gradient partials: out[k][n] = sum_r A[r][k] * B[r][n] over the block's
+// row range, followed by the column sums of B (sums = 1) or of A (sums = 2): the
+// bias gradient that shares the rows. TK x TN outputs per thread over rows staged in
+// shared memory; every output adds its rows in order in one thread, so the values
+// do not depend on the tile. One output per thread with both operands read from
+// L2 for every product took 120 us for 15.6k rows of 64 x 128 and 63 us on average
+// for an edge-level one; now 19 and 28 us. The tile is 64 wide where the matrix
+// is wider than 16 and 16 otherwise (the widths are 4, 6, 9, 10, 64 and 128).
+__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 16 : 0)
+               : "memory");
+}
+// RT rows of W columns from c0 on (C in all) into dst; what lies outside is 0. 16-byte
+// copies where the tile is full and the rows are aligned.
+template <int W, int RT, int NTH>
+__device__ __forceinline__ void lp_stage(float *dst, const float *src, int ld, int64_t rb, int64_t r1, int c0, int C) {
+  if (c0 + W <= C && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(src + c0) & 15) == 0) {
+#pragma unroll
+    for (int i = threadIdx.x; i < RT * W / 4; i += NTH) {
+      const int64_t r = rb + i / (W / 4);
+      const bool in = r < r1;
+      cp_async16(dst + 4 * i, src + (in ? r : r1 - 1) * ld + c0 + 4 * (i % (W / 4)), in);
+    }
+  } else {
+#pragma unroll
+    for (int i = threadIdx.x; i < RT * W; i += NTH) {
+      const int64_t r = rb + i / W;
+      const int c = c0 + i % W;
+      const bool in = r < r1 && c < C;
+      cp_async4(dst + i, in ? src + r * ld + c : src, in);
+    }
+  }
+}
+template <int W, int RT, int NTH>
+__device__ __forceinline__ void lp_stage(float *dst, const __nv_bfloat16 *src, int ld, int64_t rb, int64_t r1, int c0,
+                                         int C) {
+#pragma unroll 8
+  for (int i = threadIdx.x; i < RT * W; i += NTH) {
+    const int64_t r = rb + i / W;
+    const int c = c0 + i % W;
+    dst[i] = r < r1 && c < C ? (float)src[r * ld + c] : 0.f;
+  }
+}
+template <class TB, int KT, int NT, int TK, int TN>
+__global__ void __launch_bounds__(KT *NT / (TK * TN))
 k_lp_outer(int64_t R, int K, int N, const float *__restrict__ A, int lda, const TB *__restrict__ B, int ldb,
-           int64_t rows_per_block, float *__restrict__ part) {
+           int64_t rows_per_block, int sums, float *__restrict__ part) {
+  constexpr int NTH = KT * NT / (TK * TN), RT = KT + NT > 80 ? 16 : 32, S = 3, SZ = RT * (KT + NT);
+  __shared__ __align__(16) float buf[S * SZ];
+  const int k0 = blockIdx.y * KT, n0 = blockIdx.z * NT;
+  const int tid = threadIdx.x, tk = TK * (tid / (NT / TN)), tn = TN * (tid % (NT / TN));
   const int64_t r0 = blockIdx.x * rows_per_block;
   const int64_t r1 = r0 + rows_per_block < R ? r0 + rows_per_block : R;
-  const int KN = K * N;
-  for (int o = threadIdx.x; o < KN; o += blockDim.x) {
-    const int k = o / N, nn = o - k * N;
-    float acc = 0.f;
-    for (int64_t r = r0; r < r1; ++r) {
-      const float a = A ? A[r * lda + k] : 1.f;
-      acc += a * (float)B[r * ldb + nn];
+  const int tiles = r1 > r0 ? (int)((r1 - r0 + RT - 1) / RT) : 0;
+  auto stage = [&](int t) {
+    if (t < tiles) {
+      float *b = buf + t % S * SZ;
+      lp_stage<KT, RT, NTH>(b, A, lda, r0 + (int64_t)t * RT, r1, k0, K);
+      lp_stage<NT, RT, NTH>(b + RT * KT, B, ldb, r0 + (int64_t)t * RT, r1, n0, N);
     }
-    part[(int64_t)blockIdx.x * KN + o] = acc;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int t = 0; t < S - 1; ++t) stage(t);
+  float c[TK][TN] = {}, cs[TK > TN ? TK : TN] = {};
+  for (int t = 0; t < tiles; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+    __syncthreads();  // tile t has landed and tile t - 1's buffer is free
+    stage(t + S - 1);
+    const float *sA = buf + t % S * SZ, *sB = sA + RT * KT;
+#pragma unroll 4
+    for (int rr = 0; rr < RT; ++rr) {
+      float a[TK], b[TN];
+#pragma unroll
+      for (int x = 0; x < TK; ++x) a[x] = sA[rr * KT + tk + x];
+#pragma unroll
+      for (int y = 0; y < TN; ++y) b[y] = sB[rr * NT + tn + y];
+#pragma unroll
+      for (int x = 0; x < TK; ++x)
+#pragma unroll
+        for (int y = 0; y < TN; ++y) c[x][y] += a[x] * b[y];
+      if (sums == 1) {
+#pragma unroll
+        for (int y = 0; y < TN; ++y) cs[y] += b[y];
+      } else if (sums == 2) {
+#pragma unroll
+        for (int x = 0; x < TK; ++x) cs[x] += a[x];
+      }
+    }
+  }
+  const int KN = K * N;
+  float *out = part + blockIdx.x * (int64_t)(KN + (sums == 1 ? N : sums == 2 ? K : 0));
+#pragma unroll
+  for (int x = 0; x < TK; ++x)
+#pragma unroll
+    for (int y = 0; y < TN; ++y) {
+      const int k = k0 + tk + x, n = n0 + tn + y;
+      if (k < K && n < N) out[k * N + n] = c[x][y];
+    }
+  if (sums == 1 && k0 + tk == 0) {
+#pragma unroll
+    for (int y = 0; y < TN; ++y)
+      if (n0 + tn + y < N) out[KN + n0 + tn + y] = cs[y];
+  }
+  if (sums == 2 && n0 + tn == 0) {
+#pragma unroll
+    for (int x = 0; x < TK; ++x)
+      if (k0 + tk + x < K) out[KN + k0 + tk + x] = cs[x];
   }
 }
-__global__ void k_lp_outer_sum(int nparts, int KN, const float *__restrict__ part, float *__restrict__ out) {
-  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < KN; o += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int g = 0; g < nparts; ++g) s += part[(int64_t)g * KN + o];
-    out[o] = s;
+// The partials of every matrix by one launch: a block brings 32 outputs of 64
+// parts at a time to shared memory and its first warp adds them in the parts'
+// order while the others fetch the next. (A launch of one to 32 blocks per matrix
+// took 14 - 25 us each, 25 of them; now 22 us for all.)
+constexpr int kLpJobs = 8 + 3 * kLayers;
+struct LpSumJob {
+  int64_t off;  // of the partials, in floats
+  int nparts, KN, nb, out, bias;  // outputs of the matrix and of its bias, and where they go
+};
+struct LpSumJobs {
+  int n, block0[kLpJobs + 1];
+  LpSumJob j[kLpJobs];
+};
+__global__ void __launch_bounds__(256) k_lp_outer_sum(LpSumJobs jobs, const float *__restrict__ part,
+                                                      float *__restrict__ grad) {
+  __shared__ float tile[64][32];
+  int q = 0;
+  while (q + 1 < jobs.n && (int)blockIdx.x >= jobs.block0[q + 1]) ++q;
+  const LpSumJob &job = jobs.j[q];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, len = job.KN + job.nb;
+  const int o = 32 * (blockIdx.x - jobs.block0[q]) + lane;
+  const float *p = part + job.off + (o < len ? o : 0);
+  float s = 0.f;
+  for (int g0 = 0; g0 < job.nparts; g0 += 64) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int g = g0 + 8 * i + w;
+      v[i] = g < job.nparts ? p[(int64_t)g * len] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tile[8 * i + w][lane] = v[i];
+    __syncthreads();
+    const int n = min(64, job.nparts - g0);
+    if (w == 0) {
+#pragma unroll 16
+      for (int g = 0; g < n; ++g) s += tile[g][lane];
+    }
   }
+  if (w == 0 && o < len) grad[o < job.KN ? job.out + o : job.bias + o - job.KN] = s;
 }
 
-// gradient norm^2 (fixed order) and Adam with global-norm clipping
-__global__ void k_lp_gnorm(int n, const float *__restrict__ g, double *__restrict__ out) {
+// norm^2 in fixed order: kNormParts partial sums, added up where they are used
+constexpr int kNormParts = 32;
+__global__ void __launch_bounds__(256) k_lp_gnorm(int n, const float *__restrict__ g, double *__restrict__ out) {
   __shared__ double red[256];
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += (double)g[i] * g[i];
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) s += (double)g[i] * g[i];
   red[threadIdx.x] = s;
   __syncthreads();
-  for (int k = blockDim.x / 2; k > 0; k >>= 1) {
+  for (int k = 128; k > 0; k >>= 1) {
     if ((int)threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = red[0];
+  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
 }
+__device__ __forceinline__ double lp_norm2(const double *__restrict__ parts) {
+  __shared__ double total;
+  if (threadIdx.x < 32) {
+    double v = parts[threadIdx.x];
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) total = v;
+  }
+  __syncthreads();
+  return total;
+}
+// Adam with global-norm clipping
 __global__ void k_lp_adam(int n, float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
                           float *__restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
                           const double *__restrict__ gn2, float clip) {
-  const double gn = sqrt(*gn2);
+  const double gn = sqrt(lp_norm2(gn2));
   const float sc = (clip > 0.f && gn > clip) ? (float)(clip / gn) : 1.f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i] * sc;
@@ -916,7 +1065,8 @@ __global__ void k_lp_adam(int n, float *__restrict__ w, const float *__restrict_
 }
 
 __global__ void k_lp_scale_probe(int64_t n, const double *__restrict__ nrm2, float *__restrict__ w) {
-  const float sc = *nrm2 > 0.0 ? (float)sqrt((double)n / *nrm2) : 0.f;
+  const double n2 = lp_norm2(nrm2);
+  const float sc = n2 > 0.0 ? (float)sqrt((double)n / n2) : 0.f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     w[i] *= sc;
 }
@@ -1115,7 +1265,7 @@ static int lp_forward(bartels_lpcg net, bartels_mesh_plan plan, LpcgPlanState *s
             plan->diag_pos, fp->lrp, fp->meta, plan->pinned, s->fe,
             s->linv, s->h[kLayers], s->st, P + kL.Wf, P + kL.bf, P + kL.Wo, P + kL.bo, P + kL.Wd, P + kL.bd,
             P + kL.Wskip, s->raw, s->gl);
-  BT_LAUNCH(ctx, k_factor_transpose, gv, 256, 0, nV, plan->bcol, fp->meta, fp->lrp, fp->urp, fp->low2up, s->gl,
+  BT_LAUNCH(ctx, k_factor_transpose, grid_for_n(ctx, nV, 64), 64, 0, nV, plan->bcol, fp->meta, fp->lrp, fp->urp, fp->low2up, s->gl,
             s->gu);
   return BARTELS_OK;
 }
@@ -1134,18 +1284,45 @@ int lpcg_factor(bartels_lpcg net, bartels_mesh_plan plan, const float *values, c
   return BARTELS_OK;
 }
 
-template <class TB>
-static int lp_outer(bartels_lpcg net, int64_t R, int K, int N, const float *A, int lda, const TB *B, int ldb,
-                    float *out) {
-  bartels_ctx ctx = net->ctx;
-  const int64_t target = std::max<int64_t>(1, (R + 63) / 64);
-  const int nparts = (int)std::min<int64_t>(target, 512);
+// The weight gradients of one pass: every matrix's partials side by side in
+// net->part, summed by one launch at the end.
+struct LpOuterPass {
+  LpSumJobs jobs{};
+  int64_t used = 0;
+  static int parts(int64_t R) { return (int)std::min<int64_t>(std::max<int64_t>(1, (R + 63) / 64), 512); }
+  // floats of all matrices' partials on nV vertices, nnzb blocks and nl lower blocks
+  static int64_t need(int64_t nV, int64_t nnzb, int64_t nl) {
+    const int64_t v = (2 * kH * kH + kH) * (1 + 2 * kLayers) + (kH + 1) * 6 + (kDx + 1) * kH;
+    return v * parts(nV) + (int64_t)kLayers * (kDe + 1) * kH * parts(nnzb) +
+           ((kDe + 1) * kH + (kH + 1) * 9 + kDe * 9) * (int64_t)parts(nl);
+  }
+};
+
+template <class TB, int KT, int NT, int TK, int TN>
+static int lp_outer_t(bartels_ctx ctx, int nparts, int64_t R, int K, int N, const float *A, int lda, const TB *B,
+                      int ldb, int sums, float *part) {
   const int64_t rpb = (R + nparts - 1) / nparts;
-  BT_CHECK(net->part.ensure(sizeof(float) * (size_t)nparts * K * N));
-  float *part = net->part.as<float>();
-  BT_LAUNCH(ctx, k_lp_outer<TB>, nparts, 256, 0, R, K, N, A, lda, B, ldb, rpb, part);
-  BT_LAUNCH(ctx, k_lp_outer_sum, (K * N + 255) / 256, 256, 0, nparts, K * N, part, out);
+  const dim3 grid(nparts, (K + KT - 1) / KT, (N + NT - 1) / NT);
+  BT_LAUNCH(ctx, (k_lp_outer<TB, KT, NT, TK, TN>), grid, KT * NT / (TK * TN), 0, R, K, N, A, lda, B, ldb, rpb, sums, part);
   return BARTELS_OK;
+}
+// out = A^T B; bias: the column sums of B (sums = 1) or A (sums = 2)
+template <class TB>
+static int lp_outer(bartels_lpcg net, LpOuterPass &pass, int64_t R, int K, int N, const float *A, int lda,
+                    const TB *B, int ldb, int out, int sums = 0, int bias = 0) {
+  LpSumJobs &jb = pass.jobs;
+  const int nb = sums == 1 ? N : sums == 2 ? K : 0, len = K * N + nb, nparts = LpOuterPass::parts(R);
+  if (jb.n >= kLpJobs || (size_t)(pass.used + (int64_t)nparts * len) * sizeof(float) > net->part.bytes)
+    return fail(BARTELS_E_INVALID_ARG, "weight-gradient scratch");
+  float *part = net->part.as<float>() + pass.used;
+  jb.j[jb.n] = {pass.used, nparts, K * N, nb, out, bias};
+  jb.block0[jb.n + 1] = jb.block0[jb.n] + (len + 31) / 32;
+  jb.n++;
+  pass.used += (int64_t)nparts * len;
+  if (K > 16 && N > 16) return lp_outer_t<TB, 64, 64, 4, 4>(net->ctx, nparts, R, K, N, A, lda, B, ldb, sums, part);
+  if (K > 16) return lp_outer_t<TB, 64, 16, 4, 4>(net->ctx, nparts, R, K, N, A, lda, B, ldb, sums, part);
+  if (N > 16) return lp_outer_t<TB, 16, 64, 4, 4>(net->ctx, nparts, R, K, N, A, lda, B, ldb, sums, part);
+  return lp_outer_t<TB, 16, 16, 2, 2>(net->ctx, nparts, R, K, N, A, lda, B, ldb, sums, part);
 }
 
 static int lp_to_bf16(bartels_ctx ctx, int64_t n, const float *a, __nv_bfloat16 *b) {
@@ -1166,7 +1343,6 @@ static int lp_loss_grad(bartels_lpcg net, bartels_mesh_plan plan, const float *v
   const int nV = plan->nV;
   const int64_t n3 = 3ll * nV;
   const float *P = net->params;
-  float *G = net->grad;
   BT_CHECK(lp_forward(net, plan, s, vals));
   const int gv = grid_for_n(ctx, nV, 256), gw = grid_warps(ctx, nV);
   // probes
@@ -1174,18 +1350,19 @@ static int lp_loss_grad(bartels_lpcg net, bartels_mesh_plan plan, const float *v
   if (r64) {
     float *w = s->wprobe + (int64_t)nrand * n3;
     BT_LAUNCH(ctx, k_lp_resid_probe, gv, 256, 0, nV, r64, s->linv, plan->pinned, w);
-    BT_LAUNCH(ctx, k_lp_gnorm, 1, 256, 0, (int)n3, w, net->scal + 4);
-    BT_LAUNCH(ctx, k_lp_scale_probe, grid_for_n(ctx, n3, 256), 256, 0, n3, net->scal + 4, w);
+    BT_LAUNCH(ctx, k_lp_gnorm, kNormParts, 256, 0, (int)n3, w, net->scal + 8 + kNormParts);
+    BT_LAUNCH(ctx, k_lp_scale_probe, grid_for_n(ctx, n3, 256), 256, 0, n3, net->scal + 8 + kNormParts, w);
   }
   // trace estimate and loss
-  BT_LAUNCH(ctx, k_lp_gt_apply, gv, 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->urp, fp->up2low,
+  const int ny = std::min(np, 64);
+  BT_LAUNCH(ctx, k_lp_gt_apply, dim3(gv, ny), 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->urp, fp->up2low,
             plan->pinned, s->raw, s->wprobe, s->uprobe);
-  BT_CHECK(net->ctx->partials.ensure(sizeof(double) * 3 * (size_t)gv));
+  BT_CHECK(net->ctx->partials.ensure(sizeof(double) * 3 * (size_t)gv * ny));
   double *lpart = net->ctx->partials.as<double>();
-  BT_LAUNCH(ctx, k_lp_ahat_apply, gv, 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned,
+  BT_LAUNCH(ctx, k_lp_ahat_apply, dim3(gv, ny), 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned,
             s->fe, s->raw, s->uprobe, s->vprobe, lpart);
-  BT_LAUNCH(ctx, k_lp_loss_sum, 1, 32, 0, gv, np, lpart, net->scal);
-  BT_LAUNCH(ctx, k_lp_dghat, gv, 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned, s->raw,
+  BT_LAUNCH(ctx, k_lp_loss_sum, 1, 32, 0, gv * ny, np, lpart, net->scal);
+  BT_LAUNCH(ctx, k_lp_dghat, grid_for_n(ctx, nV, 64), 64, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned, s->raw,
             s->wprobe, s->vprobe, net->scal, s->dg, s->dd);
   // head backward
   BT_LAUNCH(ctx, k_lp_head_bwd, gw, 256, 0, nV, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned, s->fe,
@@ -1193,22 +1370,20 @@ static int lp_loss_grad(bartels_lpcg net, bartels_mesh_plan plan, const float *v
             s->dpre_h);
   BT_LAUNCH(ctx, k_lp_head_bwd_t, gw, 256, 0, nV, plan->brp, plan->diag_pos, fp->urp, fp->up2low, s->dpre_h, s->dst);
   const int64_t nl = s->nnzl;
-  BT_CHECK(lp_outer<float>(net, nl, kDe, kH, s->e_h, kDe, s->dpre_h, kH, G + kL.Wf));
-  BT_CHECK(lp_outer<float>(net, nl, 1, kH, nullptr, 0, s->dpre_h, kH, G + kL.bf));
-  BT_CHECK(lp_outer<float>(net, nl, kH, 9, s->z_h, kH, s->dg, 9, G + kL.Wo));
-  BT_CHECK(lp_outer<float>(net, nl, 1, 9, nullptr, 0, s->dg, 9, G + kL.bo));
-  BT_CHECK(lp_outer<float>(net, nl, kDe, 9, s->e_h, kDe, s->dg, 9, G + kL.Wskip));
-  BT_CHECK(lp_outer<float>(net, nV, kH, 6, s->h[kLayers], kH, s->dd, 6, G + kL.Wd));
-  BT_CHECK(lp_outer<float>(net, nV, 1, 6, nullptr, 0, s->dd, 6, G + kL.bd));
-  BT_CHECK(lp_outer<__nv_bfloat16>(net, nV, 2 * kH, kH, s->dst, 2 * kH, s->ha[kLayers], 2 * kH, G + kL.Wst));
+  LpOuterPass wg;
+  BT_CHECK(net->part.ensure(sizeof(float) * (size_t)LpOuterPass::need(nV, s->nnzb, nl)));
+  BT_CHECK(lp_outer(net, wg, nl, kDe, kH, s->e_h, kDe, s->dpre_h, kH, kL.Wf, 1, kL.bf));
+  BT_CHECK(lp_outer(net, wg, nl, kH, 9, s->z_h, kH, s->dg, 9, kL.Wo, 1, kL.bo));
+  BT_CHECK(lp_outer(net, wg, nl, kDe, 9, s->e_h, kDe, s->dg, 9, kL.Wskip));
+  BT_CHECK(lp_outer(net, wg, nV, kH, 6, s->h[kLayers], kH, s->dd, 6, kL.Wd, 1, kL.bd));
+  BT_CHECK(lp_outer(net, wg, nV, 2 * kH, kH, s->dst, 2 * kH, s->ha[kLayers], 2 * kH, kL.Wst));
   BT_CHECK(lp_to_bf16(ctx, 2ll * kH * nV, s->dst, s->dbf));
   BT_CHECK(lp_gemm(net, nV, 64, 128, s->dbf, 128, kB.stT, nullptr, s->dh, 64, 0, nullptr, 0, s->dh, 64, nullptr, 0));
   // message-passing layers, last to first
   for (int l = kLayers - 1; l >= 0; --l) {
     BT_LAUNCH(ctx, k_lp_relu_mask, grid_for_n(ctx, (int64_t)kH * nV, 256), 256, 0, (int64_t)kH * nV, s->upre[l], s->dh,
               s->du);
-    BT_CHECK(lp_outer<__nv_bfloat16>(net, nV, kH, 2 * kH, s->du, kH, s->ha[l], 2 * kH, G + kL.Wu[l]));
-    BT_CHECK(lp_outer<float>(net, nV, 1, kH, nullptr, 0, s->du, kH, G + kL.bu[l]));
+    BT_CHECK(lp_outer(net, wg, nV, kH, 2 * kH, s->du, kH, s->ha[l], 2 * kH, kL.Wu[l], 2, kL.bu[l]));
     BT_CHECK(lp_to_bf16(ctx, (int64_t)kH * nV, s->du, s->dbf));
     BT_CHECK(lp_gemm(net, nV, 128, 64, s->dbf, 64, kB.uT[l], nullptr, nullptr, 0, 0, nullptr, 0, s->dha, 128, nullptr,
                      0));
@@ -1216,9 +1391,8 @@ static int lp_loss_grad(bartels_lpcg net, bartels_mesh_plan plan, const float *v
     BT_LAUNCH(ctx, k_lp_msg_bwd, gw, 256, 0, nV, plan->brp, plan->bcol, plan->pinned, s->fe, s->invdeg, s->pq[l],
               P + kL.We[l], P + kL.be[l], s->dha, s->dpre_e, s->dpq);
     BT_LAUNCH(ctx, k_lp_msg_bwd_t, gw, 256, 0, nV, plan->brp, fp->rev, s->dpre_e, s->dpq);
-    BT_CHECK(lp_outer<float>(net, s->nnzb, kDe, kH, s->fe, kFe, s->dpre_e, kH, G + kL.We[l]));
-    BT_CHECK(lp_outer<float>(net, s->nnzb, 1, kH, nullptr, 0, s->dpre_e, kH, G + kL.be[l]));
-    BT_CHECK(lp_outer<__nv_bfloat16>(net, nV, 2 * kH, kH, s->dpq, 2 * kH, s->ha[l], 2 * kH, G + kL.Wpq[l]));
+    BT_CHECK(lp_outer(net, wg, s->nnzb, kDe, kH, s->fe, kFe, s->dpre_e, kH, kL.We[l], 1, kL.be[l]));
+    BT_CHECK(lp_outer(net, wg, nV, 2 * kH, kH, s->dpq, 2 * kH, s->ha[l], 2 * kH, kL.Wpq[l]));
     BT_CHECK(lp_to_bf16(ctx, 2ll * kH * nV, s->dpq, s->dbf));
     BT_CHECK(lp_gemm(net, nV, 64, 128, s->dbf, 128, kB.pqT[l], nullptr, s->dh, 64, 0, nullptr, 0, s->dh, 64, nullptr,
                      0));
@@ -1226,8 +1400,8 @@ static int lp_loss_grad(bartels_lpcg net, bartels_mesh_plan plan, const float *v
   // embedding
   BT_LAUNCH(ctx, k_lp_relu_mask, grid_for_n(ctx, (int64_t)kH * nV, 256), 256, 0, (int64_t)kH * nV, s->pre0, s->dh,
             s->du);
-  BT_CHECK(lp_outer<float>(net, nV, kDx, kH, s->xn, kDx, s->du, kH, G + kL.W0));
-  BT_CHECK(lp_outer<float>(net, nV, 1, kH, nullptr, 0, s->du, kH, G + kL.b0));
+  BT_CHECK(lp_outer(net, wg, nV, kDx, kH, s->xn, kDx, s->du, kH, kL.W0, 1, kL.b0));
+  BT_LAUNCH(ctx, k_lp_outer_sum, wg.jobs.block0[wg.jobs.n], 256, 0, wg.jobs, net->part.as<float>(), net->grad);
   // loss on the host
   double sc[3];
   BT_CUDA(cudaMemcpyAsync(sc, net->scal, sizeof(sc), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1246,9 +1420,9 @@ static int lp_adam(bartels_lpcg net, float lr, float clip) {
   net->step++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)net->step), c2 = 1.f - std::pow(b2, (float)net->step);
-  BT_LAUNCH(ctx, k_lp_gnorm, 1, 256, 0, kL.total, net->grad, net->scal + 3);
+  BT_LAUNCH(ctx, k_lp_gnorm, kNormParts, 256, 0, kL.total, net->grad, net->scal + 8);
   BT_LAUNCH(ctx, k_lp_adam, grid_for_n(ctx, kL.total, 256), 256, 0, kL.total, net->params, net->grad, net->m, net->v,
-            lr, b1, b2, 1e-8f, c1, c2, net->scal + 3, clip);
+            lr, b1, b2, 1e-8f, c1, c2, net->scal + 8, clip);
   net->bf_dirty = true;
   return BARTELS_OK;
 }
@@ -1268,7 +1442,7 @@ int lpcg_create(bartels_ctx ctx, bartels_lpcg *out) {
   e = e == cudaSuccess ? cudaMalloc(&n->v, 4 * P) : e;
   e = e == cudaSuccess ? cudaMalloc(&n->wbf, 2 * (size_t)kB.total) : e;
   e = e == cudaSuccess ? cudaMalloc(&n->err, sizeof(int)) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->scal, 8 * sizeof(double)) : e;
+  e = e == cudaSuccess ? cudaMalloc(&n->scal, (8 + 2 * kNormParts) * sizeof(double)) : e;
   if (e == cudaSuccess) e = cudaMemsetAsync(n->params, 0, 4 * P, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(n->grad, 0, 4 * P, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(n->m, 0, 4 * P, ctx->stream);
