@@ -74,6 +74,7 @@ SIGNATURES = [
     ("bartels_plan_create", C.c_int, [_P, C.c_int, _D, C.c_int, _I, C.POINTER(_P)]),
     ("bartels_plan_destroy", C.c_int, [_P]),
     ("bartels_plan_set_element_data", C.c_int, [_P, _D, _D, _D, _D]),
+    ("bartels_plan_set_element_rows", C.c_int, [_P, C.c_int, _D, _D, _D]),
     ("bartels_plan_csr_size", C.c_int, [_P, _I, C.POINTER(C.c_int64)]),
     ("bartels_plan_csr_pattern", C.c_int, [_P, _I, _I]),
     ("bartels_tetmesh_q", C.c_int, [_P, _P, C.c_int, _D, _D, _D, _D, _D]),

@@ -13,6 +13,7 @@ from __future__ import annotations
 import atexit
 import ctypes as C
 import hashlib
+import itertools
 import sys
 import weakref
 from collections import OrderedDict
@@ -38,6 +39,20 @@ def _iptr(a):
 
 def _f64(a):
     return np.ascontiguousarray(a, dtype=np.float64)
+
+
+def _is_rows(a, n, k):
+    """None, or an (n, k) FP64 array stored row by row."""
+    return a is None or (isinstance(a, np.ndarray) and a.shape == (n, k) and a.dtype == np.float64
+                         and a.flags.c_contiguous)
+
+
+_memcmp = C.CDLL(None).memcmp
+_memcmp.argtypes, _memcmp.restype = [C.c_void_p, C.c_void_p, C.c_size_t], C.c_int
+
+
+def _same_bytes(a, b):
+    return a.shape == b.shape and _memcmp(a.ctypes.data, b.ctypes.data, a.nbytes) == 0
 
 
 def _colmajor(a, dtype):
@@ -159,7 +174,16 @@ class MeshPlan:
                                                   opt(density)), "bartels_plan_set_element_data")
 
     # --- energy / gradient / Hessian ------------------------------------
-    def _elem(self, dphidX, volume, params):
+    def _elem(self, model, dphidX, volume, params, where):
+        """The element data of an energy, gradient or Hessian call as the C entry's three pointers.
+        Row-major arrays go to the plan as they are; other forms are transposed here for the entry to upload."""
+        if ((dphidX is not None or params is not None) and _is_rows(dphidX, self.nT, 12)
+                and _is_rows(params, self.nT, 2)):
+            v = None if volume is None else _f64(np.ravel(volume))
+            check(lib().bartels_plan_set_element_rows(self.handle, MODELS[model],
+                                                      *[None if a is None else _dptr(a) for a in (dphidX, v, params)]),
+                  where)
+            return v, (None, None, None)
         keep = []
         out = []
         for a, cm in ((dphidX, True), (volume, False), (params, True)):
@@ -172,7 +196,7 @@ class MeshPlan:
         return keep, out
 
     def q(self, model, q, dphidX=None, volume=None, params=None) -> float:
-        keep, (d, v, p) = self._elem(dphidX, volume, params)
+        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_q")
         qa = _f64(q)
         e = C.c_double()
         check(lib().bartels_tetmesh_q(self.ctx.handle, self.handle, MODELS[model], _dptr(qa), d, v, p, C.byref(e)),
@@ -180,7 +204,7 @@ class MeshPlan:
         return e.value
 
     def dq(self, model, q, dphidX=None, volume=None, params=None):
-        keep, (d, v, p) = self._elem(dphidX, volume, params)
+        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_dq")
         qa = _f64(q)
         g = np.zeros(3 * self.nV)
         check(lib().bartels_tetmesh_dq(self.ctx.handle, self.handle, MODELS[model], _dptr(qa), d, v, p, _dptr(g)),
@@ -188,7 +212,7 @@ class MeshPlan:
         return g
 
     def dq2_values(self, model, q, dphidX=None, volume=None, params=None, psd_tol=None, corot_exact=False):
-        keep, (d, v, p) = self._elem(dphidX, volume, params)
+        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_dq2")
         qa = _f64(q)
         vals = np.zeros(self.nnz)
         psd = _lib.PSD_NONE if psd_tol is None else _lib.PSD_SIMPLE_FIX
@@ -278,21 +302,25 @@ def newton_params(**kw) -> "_lib.NewtonParams":
 
 
 # ---------------------------------------------------------------- drop-ins --
-_plans: "OrderedDict[str, MeshPlan]" = OrderedDict()
+# by a running number; each with its own copy of the mesh it was made for
+_plans: "OrderedDict[int, MeshPlan]" = OrderedDict()
+_plan_number = itertools.count()
 
 
 def _plan_for(V, E) -> MeshPlan:
     V = _f64(V)
     E = np.ascontiguousarray(E, dtype=np.int32)
-    key = hashlib.sha1(f"{V.shape}{E.shape}".encode() + V.tobytes() + E.tobytes()).hexdigest()
-    p = _plans.get(key)
-    if p is None:
-        p = MeshPlan(V, E)
-        _plans[key] = p
-        while len(_plans) > 4:
-            _plans.popitem(last=False)[1].close()
-    else:
-        _plans.move_to_end(key)
+    # by content, the newest first: a comparison reads the mesh once (48,000 tets:
+    # 40 us), where a digest of it copied and hashed it (570 us)
+    for key, p in reversed(list(_plans.items())):
+        if _same_bytes(V, p.made_for[0]) and _same_bytes(E, p.made_for[1]):
+            _plans.move_to_end(key)
+            return p
+    p = MeshPlan(V, E)
+    p.made_for = (V.copy(), E.copy())
+    _plans[next(_plan_number)] = p
+    while len(_plans) > 4:
+        _plans.popitem(last=False)[1].close()
     return p
 
 

@@ -12,7 +12,7 @@
 
 namespace bartels {
 int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const double *vol, const double *params,
-                          const double *density);
+                          const double *density, bool rows = false, bool sync = true);
 void plan_free(bartels_mesh_plan plan);
 int launch_prep_u(bartels_ctx ctx, bartels_mesh_plan plan, const double *x, const double *q_base, double scale,
                   bool displacement, float4 *u);
@@ -59,13 +59,14 @@ bool valid_model(int m) { return m >= 0 && m <= 5; }
 // Linear elasticity takes the reference's (Young's modulus, Poisson ratio) per
 // tet (src/d2psi_linear_elasticity_de2.cpp:10-11); the kernels use the Lame
 // pair (lambda, mu). Returns params itself for every other model.
-const double *model_params(int model, const double *params, int nT, std::vector<double> &buf) {
+const double *model_params(int model, const double *params, int nT, bool rows, std::vector<double> &buf) {
   if (model != BARTELS_LINEAR_ELASTICITY || !params) return params;
   buf.resize(2 * (size_t)nT);
+  const size_t ts = rows ? 2 : 1, cs = rows ? 1 : (size_t)nT;
   for (int t = 0; t < nT; ++t) {
-    const double E = params[t], nu = params[t + (size_t)nT];
-    buf[t] = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
-    buf[t + (size_t)nT] = E / (2.0 * (1.0 + nu));
+    const double E = params[t * ts], nu = params[t * ts + cs];
+    buf[t * ts] = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+    buf[t * ts + cs] = E / (2.0 * (1.0 + nu));
   }
   return buf.data();
 }
@@ -252,6 +253,16 @@ int bartels_plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, 
   return plan_set_element_data(plan, dphidX, vol, params, density);
 }
 
+int bartels_plan_set_element_rows(bartels_mesh_plan plan, int model, const double *dphidX, const double *vol,
+                                  const double *params) {
+  if (!plan) return fail(BARTELS_E_INVALID_ARG, "null plan");
+  if (!valid_model(model)) return fail(BARTELS_E_INVALID_ARG, "bad arguments");
+  BT_CHECK(check_ctx(plan->ctx));
+  std::vector<double> pbuf;
+  return plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, true, pbuf), nullptr, true,
+                               false);
+}
+
 int bartels_plan_csr_size(bartels_mesh_plan plan, int *n, int64_t *nnz) {
   if (!plan) return fail(BARTELS_E_INVALID_ARG, "null plan");
   if (n) *n = 3 * plan->nV;
@@ -279,7 +290,8 @@ int bartels_tetmesh_q(bartels_ctx ctx, bartels_mesh_plan plan, int model, const 
   BT_CHECK(check_plan(ctx, plan));
   if (!valid_model(model) || !q || !energy_out) return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   std::vector<double> pbuf;
-  BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, pbuf), nullptr));
+  BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, false, pbuf), nullptr, false,
+                                 false));
   double *dq;
   BT_CHECK(stage_vec(ctx, ctx->stage_e, q, 3 * (size_t)plan->nV, &dq));
   BT_CHECK(ctx->scalars.ensure(64 * sizeof(double)));
@@ -297,7 +309,8 @@ int bartels_tetmesh_dq(bartels_ctx ctx, bartels_mesh_plan plan, int model, const
   BT_CHECK(check_plan(ctx, plan));
   if (!valid_model(model) || !q || !g) return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   std::vector<double> pbuf;
-  BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, pbuf), nullptr));
+  BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, false, pbuf), nullptr, false,
+                                 false));
   const size_t n = 3 * (size_t)plan->nV;
   double *dq;
   BT_CHECK(stage_vec(ctx, ctx->stage_e, q, n, &dq));
@@ -318,7 +331,8 @@ int bartels_tetmesh_dq2(bartels_ctx ctx, bartels_mesh_plan plan, int model, cons
   if (!valid_model(model) || !q || !csr_values || (psd_mode != BARTELS_PSD_NONE && psd_mode != BARTELS_PSD_SIMPLE_FIX))
     return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   std::vector<double> pbuf;
-  BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, pbuf), nullptr));
+  BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, false, pbuf), nullptr, false,
+                                 false));
   const size_t n = 3 * (size_t)plan->nV;
   const int64_t nnz = 9 * plan->nnzb;
   double *dq;

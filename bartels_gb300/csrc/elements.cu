@@ -83,14 +83,16 @@ __global__ void k_dphi_vol(int nT, const double *__restrict__ X, const int4 *__r
 // |phi_0 + phi_1 + phi_2 + phi_3| relative to |phi| (must be ~0: the plan
 // stores rows 1..3 only), err[1] the largest |sum_a (X_a - X_0) phi_a^T - I|
 // (0 when dphidX belongs to the plan's rest shape).
-__global__ void k_import_dphi(int nT, const double *__restrict__ src, const double *__restrict__ X,
+// entry (t, c) of src is src[t ts + c cs]
+__global__ void k_import_dphi(int nT, const double *__restrict__ src, size_t ts, size_t cs,
+                              const double *__restrict__ X,
                               const int4 *__restrict__ E, double *__restrict__ dphi9, double *__restrict__ err) {
   double e0 = 0.0, e1 = 0.0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nT; t += gridDim.x * blockDim.x) {
     double phi[4][3], mag = 0.0;
     for (int a = 0; a < 4; ++a)
       for (int d = 0; d < 3; ++d) {
-        phi[a][d] = src[t + (size_t)nT * (a + 4 * d)];
+        phi[a][d] = src[t * ts + (a + 4 * d) * cs];
         mag = fmax(mag, fabs(phi[a][d]));
       }
     for (int d = 0; d < 3; ++d) {
@@ -922,10 +924,11 @@ int launch_dphi_vol(bartels_ctx ctx, int nV, const double *X3, int nT, const int
   return BARTELS_OK;
 }
 
-int launch_import_dphi(bartels_ctx ctx, bartels_mesh_plan plan, const double *src_d, double *err_d) {
+int launch_import_dphi(bartels_ctx ctx, bartels_mesh_plan plan, const double *src_d, bool rows, double *err_d) {
+  const size_t ts = rows ? 12 : 1, cs = rows ? 1 : (size_t)plan->nT;
   BT_CUDA(cudaMemsetAsync(err_d, 0, 2 * sizeof(double), ctx->stream));
-  BT_LAUNCH(ctx, k_import_dphi, grid_for(ctx, plan->nT, 256), 256, 0, plan->nT, src_d, plan->X, plan->E,
-            plan->dphi64, err_d);
+  BT_LAUNCH(ctx, k_import_dphi, grid_for(ctx, plan->nT, 256), 256, 0, plan->nT, src_d, ts, cs, plan->X,
+            plan->E, plan->dphi64, err_d);
   return BARTELS_OK;
 }
 

@@ -53,7 +53,7 @@ void DevBuf::release() {
   bytes = 0;
 }
 
-int launch_import_dphi(bartels_ctx ctx, bartels_mesh_plan plan, const double *src_d, double *err_d);
+int launch_import_dphi(bartels_ctx ctx, bartels_mesh_plan plan, const double *src_d, bool rows, double *err_d);
 
 template <class T>
 static int upload(bartels_ctx ctx, T **dst, const T *src, size_t n) {
@@ -201,8 +201,11 @@ int plan_build(bartels_mesh_plan plan, const double *V, const int *E) {
 }
 
 // Upload caller element data (reference layouts) into the plan.
+// rows: dphidX (nT x 12) and params (nT x 2) are row-major, else column-major. Without
+// `sync` the records may still be under way on the context's stream on return
+// (pageable sources have been staged by then).
 int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const double *vol, const double *params,
-                          const double *density) {
+                          const double *density, bool rows, bool sync) {
   bartels_ctx ctx = plan->ctx;
   const size_t nT = (size_t)plan->nT;
   if (nT == 0) return BARTELS_OK;
@@ -211,7 +214,7 @@ int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const do
     BT_CHECK(ctx->stage_a.ensure(sizeof(double) * 12 * nT));
     BT_CHECK(ctx->stage_b.ensure(sizeof(double) * 2));
     BT_CUDA(cudaMemcpyAsync(ctx->stage_a.p, dphidX, sizeof(double) * 12 * nT, cudaMemcpyHostToDevice, ctx->stream));
-    BT_CHECK(launch_import_dphi(ctx, plan, ctx->stage_a.as<double>(), ctx->stage_b.as<double>()));
+    BT_CHECK(launch_import_dphi(ctx, plan, ctx->stage_a.as<double>(), rows, ctx->stage_b.as<double>()));
     double err[2];
     BT_CUDA(cudaMemcpyAsync(err, ctx->stage_b.p, sizeof(err), cudaMemcpyDeviceToHost, ctx->stream));
     BT_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -225,7 +228,10 @@ int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const do
     BT_CUDA(cudaMemcpyAsync(plan->vol, vol, sizeof(double) * nT, cudaMemcpyHostToDevice, ctx->stream));
     changed = true;
   }
-  if (params) {
+  if (params && rows) {
+    BT_CUDA(cudaMemcpyAsync(plan->params, params, sizeof(double) * 2 * nT, cudaMemcpyHostToDevice, ctx->stream));
+    changed = true;
+  } else if (params) {
     // column-major nT x 2 -> per-tet pairs
     std::vector<double> p(2 * nT);
     for (size_t t = 0; t < nT; ++t) {
@@ -233,7 +239,6 @@ int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const do
       p[2 * t + 1] = params[t + nT];
     }
     BT_CUDA(cudaMemcpyAsync(plan->params, p.data(), sizeof(double) * 2 * nT, cudaMemcpyHostToDevice, ctx->stream));
-    BT_CUDA(cudaStreamSynchronize(ctx->stream));
     changed = true;
   }
   if (density) {
@@ -241,7 +246,7 @@ int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const do
     changed = true;
   }
   if (changed) BT_CHECK(plan_refresh_records(plan));
-  BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (sync) BT_CUDA(cudaStreamSynchronize(ctx->stream));
   return BARTELS_OK;
 }
 
