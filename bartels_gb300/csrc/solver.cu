@@ -875,7 +875,7 @@ static int pcg_enqueue_iters(bartels_ctx ctx, const PcgOperator &op, const PcgWo
 }
 
 // Loop condition of the device-driven inner solve: a CUDA graph while-node
-// whose body is one PCG iteration runs until the solve is done. The body count
+// whose body is PCG iterations runs until the solve is done. The body count
 // is bounded independently of the iteration count (the iteration cap of the
 // state bounds both).
 __global__ void k_pcg_cond(cudaGraphConditionalHandle h, PcgState *st) {
@@ -892,8 +892,11 @@ static int launch_cond(bartels_ctx ctx, cudaGraphConditionalHandle h, PcgState *
 }
 
 // Executable graph of the inner PCG loop. Preferred: one while-node whose body
-// is one iteration (*device_loop = true: a launch runs the inner solve to its
-// end with no host round trip and no iteration after convergence). Fallback:
+// is body_iters iterations (*device_loop = true: a launch runs the inner solve to
+// its end with no host round trip; kernels after convergence turn into no-ops).
+// One with multigrid; four without, where an iteration is three kernels of a few
+// microseconds and the loop's condition shows (block-Jacobi on 68.9k vertices
+// 28.7 -> 26.9 ms; with multigrid four bodies gained 0 - 1% and cost packed solves 3%). Fallback:
 // a fixed run of `chunk` iterations whose kernels turn into no-ops once the
 // state is done. *launches: kernel launches per body / chunk.
 // BARTELS_PCG_DEVICE_LOOP=0 selects the fixed-length form (kernel profilers
@@ -906,8 +909,8 @@ static bool device_loop_allowed() {
   return allowed;
 }
 
-static int build_loop_graph(bartels_ctx ctx, PcgState *st, const std::function<int(int)> &enqueue, int chunk,
-                            cudaGraphExec_t *exec, int64_t *launches, bool *device_loop) {
+static int build_loop_graph(bartels_ctx ctx, PcgState *st, const std::function<int(int)> &enqueue, int body_iters,
+                            int chunk, cudaGraphExec_t *exec, int64_t *launches, bool *device_loop) {
   *exec = nullptr;
   *device_loop = false;
   cudaGraph_t graph = nullptr;
@@ -929,7 +932,7 @@ static int build_loop_graph(bartels_ctx ctx, PcgState *st, const std::function<i
     const int64_t before = ctx->launches;
     e = cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      int s = enqueue(1);
+      int s = enqueue(body_iters);
       if (s == BARTELS_OK) s = launch_cond(ctx, h, st);
       cudaGraph_t captured = nullptr;
       e = cudaStreamEndCapture(ctx->stream, &captured);
@@ -1054,7 +1057,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     BT_CHECK(pcg_small_fill(ctx, small, base + o_small, small_off, rp, ci, op.values, op.pinned));
   } else {
     BT_CHECK(build_loop_graph(
-        ctx, w.st, [&](int k) { return pcg_enqueue_iters(ctx, op, w, n, nb, k); }, chunk, &exec, &graph_launches,
+        ctx, w.st, [&](int k) { return pcg_enqueue_iters(ctx, op, w, n, nb, k); }, op.mg ? 1 : 4, chunk, &exec, &graph_launches,
         &device_loop));
   }
   int status = BARTELS_OK;
@@ -1465,7 +1468,7 @@ static int seg_pcg_solve(bartels_ctx ctx, const PcgOperator &op, const double *b
   int64_t graph_launches = 0;
   bool device_loop = false;
   BT_CHECK(build_loop_graph(
-      ctx, w.st, [&](int k) { return seg_enqueue_iters(ctx, op, w, sp, k); }, 8, &exec, &graph_launches,
+      ctx, w.st, [&](int k) { return seg_enqueue_iters(ctx, op, w, sp, k); }, 1, 8, &exec, &graph_launches,
       &device_loop));
   rep->iterations = 0;
   rep->refinements = 0;
