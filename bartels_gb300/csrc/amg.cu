@@ -1931,6 +1931,7 @@ int resid0(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const f
     const SellView sv = plan->sell->view();
     const int S = sell_split(ctx, sv.nslices), g = sell_grid(ctx, sv.nslices, S);
     if (S == 1) BT_LAUNCH_PDL(ctx, k_mg0_resid_sell<1>, g, 256, 0, sv, a16, b, x, out, plan->pinned, st);
+    else if (S == 2) BT_LAUNCH_PDL(ctx, k_mg0_resid_sell<2>, g, 256, 0, sv, a16, b, x, out, plan->pinned, st);
     else BT_LAUNCH_PDL(ctx, k_mg0_resid_sell<4>, g, 256, 0, sv, a16, b, x, out, plan->pinned, st);
   } else {
     const int G = plan_lanes_spmv(ctx, plan);
@@ -2073,6 +2074,8 @@ int mg_enqueue_apply(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
       const uint2 *a16 = mg->a16;
       if (S == 1)
         BT_LAUNCH_PDL(ctx, k_mg0_post_bj_sell<1>, g, 256, 0, sv, a16, sm.minv, r, l0.x, z, plan->pinned, c0, part, st);
+      else if (S == 2)
+        BT_LAUNCH_PDL(ctx, k_mg0_post_bj_sell<2>, g, 256, 0, sv, a16, sm.minv, r, l0.x, z, plan->pinned, c0, part, st);
       else
         BT_LAUNCH_PDL(ctx, k_mg0_post_bj_sell<4>, g, 256, 0, sv, a16, sm.minv, r, l0.x, z, plan->pinned, c0, part, st);
     } else {

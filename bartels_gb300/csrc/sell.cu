@@ -154,11 +154,20 @@ int sell_fill_bf16(bartels_ctx ctx, bartels_mesh_plan plan, const float *values,
   return BARTELS_OK;
 }
 
-int sell_split(bartels_ctx ctx, int nslices) { return nslices >= ctx->num_sms * 16 ? 1 : 4; }
+// Warps per slice: one while there are two rounds of warps or so, else two or four,
+// so that every SM has enough loads in flight. Whole solves with 1 / 2 / 4: 489
+// slices (Newton, 15.6k vertices) 12.7 / 11.7 / 11.0 ms, 1,583 slices 7.6 / 7.1 / 7.3,
+// 2,154 slices (block-Jacobi) 23.6 / 21.5 / 26.9, 3,677 slices 10.2 / 11.2 / 10.9.
+int sell_split(bartels_ctx ctx, int nslices) {
+  return nslices >= ctx->num_sms * 16 ? 1 : nslices >= ctx->num_sms * 8 ? 2 : 4;
+}
 
+// Five CTAs per SM are what the SpMV's 48 registers let reside: more came in a
+// second, thinner round (n = 96 multigrid solve 48.1 ms with eight, 46.2 with five,
+// 51.0 with six; n = 80 30.3 / 28.8 / 30.8).
 int sell_grid(bartels_ctx ctx, int nslices, int split) {
   const int per = 8 / split;
-  return std::max(1, std::min((nslices + per - 1) / per, ctx->num_sms * 8));
+  return std::max(1, std::min((nslices + per - 1) / per, ctx->num_sms * 5));
 }
 
 }  // namespace bartels

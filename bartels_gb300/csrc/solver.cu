@@ -822,6 +822,8 @@ static int pcg_spmv_blk(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w
     const int S = sell_split(ctx, sv.nslices), g = sell_grid(ctx, sv.nslices, S);
     if (S == 1)
       BT_LAUNCH_PDL(ctx, k_pcg_spmv_sell<1>, g, 256, 0, sv, op.vsell, w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st);
+    else if (S == 2)
+      BT_LAUNCH_PDL(ctx, k_pcg_spmv_sell<2>, g, 256, 0, sv, op.vsell, w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st);
     else
       BT_LAUNCH_PDL(ctx, k_pcg_spmv_sell<4>, g, 256, 0, sv, op.vsell, w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st);
     return BARTELS_OK;

@@ -2,8 +2,8 @@
 
 Row lengths and counts at the layout's edges: one tet, vertex counts around a
 slice (32 rows) and a window (256 rows), a shuffled numbering with uneven rows,
-pinned rows, and a mesh with enough slices for one warp per slice (four warps
-share a slice below that)."""
+pinned rows, and meshes with enough slices for two and for one warp per slice (four
+below that)."""
 import ctypes as C
 
 import numpy as np
@@ -41,7 +41,7 @@ def _mesh(kind):
 
 
 @pytest.mark.parametrize("kind", ["tet", "strip31", "strip33", "strip255", "strip256", "strip257", "strip1000",
-                                  "shuf9", "shuf20", "cube44"])
+                                  "shuf9", "shuf20", "cube35", "cube44"])
 @pytest.mark.parametrize("pin", [False, True])
 def test_spmv_matches_fp64(kind, pin):
     torch = pytest.importorskip("torch")
