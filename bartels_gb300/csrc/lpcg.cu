@@ -1265,8 +1265,8 @@ static int lp_forward(bartels_lpcg net, bartels_mesh_plan plan, LpcgPlanState *s
             plan->diag_pos, fp->lrp, fp->meta, plan->pinned, s->fe,
             s->linv, s->h[kLayers], s->st, P + kL.Wf, P + kL.bf, P + kL.Wo, P + kL.bo, P + kL.Wd, P + kL.bd,
             P + kL.Wskip, s->raw, s->gl);
-  BT_LAUNCH(ctx, k_factor_transpose, grid_for_n(ctx, nV, 64), 64, 0, nV, plan->bcol, fp->meta, fp->lrp, fp->urp, fp->low2up, s->gl,
-            s->gu);
+  BT_LAUNCH(ctx, k_factor_transpose, grid_for_n(ctx, nV, 64), 64, 0, nV, plan->bcol, fp->meta, fp->lrp, fp->urp,
+            fp->low2up, s->gl, s->gu);
   return BARTELS_OK;
 }
 
@@ -1303,7 +1303,8 @@ static int lp_outer_t(bartels_ctx ctx, int nparts, int64_t R, int K, int N, cons
                       int ldb, int sums, float *part) {
   const int64_t rpb = (R + nparts - 1) / nparts;
   const dim3 grid(nparts, (K + KT - 1) / KT, (N + NT - 1) / NT);
-  BT_LAUNCH(ctx, (k_lp_outer<TB, KT, NT, TK, TN>), grid, KT * NT / (TK * TN), 0, R, K, N, A, lda, B, ldb, rpb, sums, part);
+  BT_LAUNCH(ctx, (k_lp_outer<TB, KT, NT, TK, TN>), grid, KT * NT / (TK * TN), 0, R, K, N, A, lda, B, ldb, rpb, sums,
+            part);
   return BARTELS_OK;
 }
 // out = A^T B; bias: the column sums of B (sums = 1) or A (sums = 2)
@@ -1355,15 +1356,15 @@ static int lp_loss_grad(bartels_lpcg net, bartels_mesh_plan plan, const float *v
   }
   // trace estimate and loss
   const int ny = std::min(np, 64);
-  BT_LAUNCH(ctx, k_lp_gt_apply, dim3(gv, ny), 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->urp, fp->up2low,
-            plan->pinned, s->raw, s->wprobe, s->uprobe);
+  BT_LAUNCH(ctx, k_lp_gt_apply, dim3(gv, ny), 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos,
+            fp->urp, fp->up2low, plan->pinned, s->raw, s->wprobe, s->uprobe);
   BT_CHECK(net->ctx->partials.ensure(sizeof(double) * 3 * (size_t)gv * ny));
   double *lpart = net->ctx->partials.as<double>();
-  BT_LAUNCH(ctx, k_lp_ahat_apply, dim3(gv, ny), 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned,
-            s->fe, s->raw, s->uprobe, s->vprobe, lpart);
+  BT_LAUNCH(ctx, k_lp_ahat_apply, dim3(gv, ny), 256, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos,
+            fp->lrp, plan->pinned, s->fe, s->raw, s->uprobe, s->vprobe, lpart);
   BT_LAUNCH(ctx, k_lp_loss_sum, 1, 32, 0, gv * ny, np, lpart, net->scal);
-  BT_LAUNCH(ctx, k_lp_dghat, grid_for_n(ctx, nV, 64), 64, 0, nV, np, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned, s->raw,
-            s->wprobe, s->vprobe, net->scal, s->dg, s->dd);
+  BT_LAUNCH(ctx, k_lp_dghat, grid_for_n(ctx, nV, 64), 64, 0, nV, np, plan->brp, plan->bcol,
+            plan->diag_pos, fp->lrp, plan->pinned, s->raw, s->wprobe, s->vprobe, net->scal, s->dg, s->dd);
   // head backward
   BT_LAUNCH(ctx, k_lp_head_bwd, gw, 256, 0, nV, plan->brp, plan->bcol, plan->diag_pos, fp->lrp, plan->pinned, s->fe,
             s->st, P + kL.Wf, P + kL.bf, P + kL.Wo, P + kL.Wd, s->dg, s->dd, s->dst, s->dh, s->e_h, s->z_h,

@@ -374,8 +374,8 @@ def run_gpu(args, rank, world):
         ctx.synchronize()
         return a.elapsed_time(b) / reps * 1e-3
 
-    # the PCG loop's own SpMV kernel (over the padded copy of the values the loop
-    # reads), timed by the library with CUDA events on its stream
+    # the PCG loop's own SpMV kernel (over the sliced-ELL copy of the values the
+    # loop reads), timed by the library with CUDA events on its stream
     spmv_us = C.c_double()
     _lib.check(L.bartels_plan_pcg_spmv_time_d(ctx.handle, plan.handle, None, C.c_void_p(xs.data_ptr()),
                                               C.c_void_p(ys.data_ptr()), 30, C.byref(spmv_us)), "pcg_spmv_time")
@@ -498,7 +498,7 @@ def run_gpu(args, rank, world):
         "time_steps_ended_at_noise_floor": main_arm["steps_at_noise_floor"],
         "pcg_iters_per_newton": pcg_its / max(newton_its, 1),
         "roofline": {"bound": "hbm", "achieved": spmv_gbs, "peak": peak, "unit": "GB/s",
-                     "frac": spmv_gbs / peak, "traffic": traffic, "kernel": "k_pcg_spmv_blk (the PCG loop's SpMV, FP32, rows padded to 4 entries)",
+                     "frac": spmv_gbs / peak, "traffic": traffic, "kernel": "k_pcg_spmv_sell (the PCG loop's SpMV, FP32, sliced-ELL copy of the values)",
                      "bytes_per_launch": spmv_bytes, "us_per_launch": spmv_s * 1e6, "peak_source": peak_kind},
         "kernels": {"dq2_psd_off": {"us_per_launch": hess_off_s * 1e6, "state": "rest (q = X)",
                                     "compulsory_bytes": hess_bytes, "achieved_gbs": hess_bytes / hess_off_s / 1e9,

@@ -467,8 +467,8 @@ int bartels_plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *
 /* The PCG loop's SpMV kernel, y_d = A x_d with A the FP32 values_d (NULL:
  * the plan's last assembled Hessian), timed: 3 warm-up launches, then reps
  * launches between CUDA events on the context's stream; *us_per_launch gets
- * the mean. The loop reads a copy of the values whose scalar rows are padded
- * to multiples of 4 entries (4 values per 16-byte load); the copy is made
+ * the mean. The loop reads a copy of the values in sliced-ELL form (a
+ * warp's loads are contiguous, 4 values per 16-byte load); the copy is made
  * here once, as the solver makes it once per linear solve (environment
  * BARTELS_PCG_PADDED=0 keeps the values' own layout). For measurement; no
  * counterpart in the reference. */
