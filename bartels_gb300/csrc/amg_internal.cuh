@@ -103,6 +103,7 @@ struct MgSmoother {
   const float *minv = nullptr;
   const __nv_bfloat16 *gl = nullptr, *gu = nullptr;
   const FactorPattern *fp = nullptr;
+  const uint2 *lsell = nullptr, *usell = nullptr;  // the factor in the plan's sliced-ELL layouts, on large meshes
 };
 
 // Build (or keep) the hierarchy for the plan's pattern and pinned set.

@@ -189,6 +189,7 @@ struct bartels_mesh_plan_s {
   // sliced-ELL layout of the block rows (built on the first solve); w_sell holds
   // the FP32 values in it for the PCG loop's SpMV
   bartels::SellPattern *sell = nullptr;
+  bartels::SellPattern *sell_factor[2] = {nullptr, nullptr};  // the learned factor's lower and upper parts
   int nchunks64 = 0;
   // Hessian tuning: vertices per assembly CTA (128, or 64 with chunk_v64) and
   // threads per CTA of the PSD pre-pass kernels (64, 128 or 256)
@@ -215,7 +216,7 @@ struct bartels_mesh_plan_s {
   // packed-mesh segments (nullptr: one system)
   bartels::SegInfo *seg = nullptr;
   // solver workspace
-  bartels::DevBuf w_values, w_minv, w_vec, w_grad_e, w_energy, w_u, w_pcg, w_psd, w_spmv, w_sell;
+  bartels::DevBuf w_values, w_minv, w_vec, w_grad_e, w_energy, w_u, w_pcg, w_psd, w_spmv, w_sell, w_sell_factor;
 };
 
 namespace bartels {

@@ -364,6 +364,10 @@ void plan_free(bartels_mesh_plan plan) {
   if (plan->chunk_v64) cudaFree(plan->chunk_v64);
   delete plan->sell;
   plan->sell = nullptr;
+  for (SellPattern *&p : plan->sell_factor) {
+    delete p;
+    p = nullptr;
+  }
   plan->chunk_v64 = nullptr;
   void *ptrs[] = {plan->X,        plan->E,      plan->dphi64,  plan->vol,     plan->params,  plan->density,
                   plan->rec32,    plan->rec64,  plan->inc_ptr, plan->inc_tet, plan->inc_pos, plan->brp,
@@ -381,6 +385,7 @@ void plan_free(bartels_mesh_plan plan) {
   plan->w_psd.release();
   plan->w_spmv.release();
   plan->w_sell.release();
+  plan->w_sell_factor.release();
 }
 
 }  // namespace bartels

@@ -2,19 +2,29 @@
 #include <algorithm>
 #include <vector>
 
+#include "lpcg_internal.cuh"
 #include "sell.cuh"
 
 namespace bartels {
 
 constexpr int kSellWindow = 256;  // rows ordered by length within windows of this many
 
+// start and number of row v's blocks in a layout
+__device__ __forceinline__ int2 sell_range(int part, const int *brp, const int *diag_pos, int v) {
+  const int rb = brp[v], nb = brp[v + 1] - rb;
+  if (part == kSellFull) return make_int2(rb, nb);
+  const int d = diag_pos[v];
+  return part == kSellLower ? make_int2(rb, d + 1) : make_int2(rb + d, nb - d);
+}
+
 // One CTA per window: rank of each row by descending block count (ties keep
 // the vertex order), and the groups of the window's slices.
 __global__ void __launch_bounds__(kSellWindow)
-k_sell_order(int nV, const int *__restrict__ brp, int *__restrict__ row, int *__restrict__ groups) {
+k_sell_order(int nV, int part, const int *__restrict__ brp, const int *__restrict__ diag_pos, int *__restrict__ row,
+             int *__restrict__ groups) {
   __shared__ int cnt[kSellWindow];
   const int v = blockIdx.x * kSellWindow + threadIdx.x;
-  const int c = v < nV ? brp[v + 1] - brp[v] : -1;
+  const int c = v < nV ? sell_range(part, brp, diag_pos, v).y : -1;
   cnt[threadIdx.x] = c;
   __syncthreads();
   int rank = 0;
@@ -24,11 +34,13 @@ k_sell_order(int nV, const int *__restrict__ brp, int *__restrict__ row, int *__
 }
 
 __global__ void __launch_bounds__(256)
-k_sell_cols(SellView sv, const int *__restrict__ brp, const int *__restrict__ bcol, int4 *__restrict__ col) {
+k_sell_cols(SellView sv, int part, const int *__restrict__ brp, const int *__restrict__ diag_pos,
+            const int *__restrict__ bcol, int4 *__restrict__ col) {
   const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
   for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < sv.nslices; s += nw) {
     const int v = sv.row[32 * s + lane];
-    const int rb = v >= 0 ? brp[v] : 0, nb = v >= 0 ? brp[v + 1] - rb : 0, own = v >= 0 ? 3 * v : 0;
+    const int2 rg = v >= 0 ? sell_range(part, brp, diag_pos, v) : make_int2(0, 0);
+    const int rb = rg.x, nb = rg.y, own = v >= 0 ? 3 * v : 0;
     for (int g = sv.off[s]; g < sv.off[s + 1]; ++g) {
       const int j = 4 * (g - sv.off[s]);
       int c[4];
@@ -109,22 +121,62 @@ k_sell_fill(SellView sv, const int *__restrict__ brp, const int *__restrict__ bc
   }
 }
 
+// A warp per slice: lane l copies its row's groups, three 8-byte loads per scalar row.
+__global__ void __launch_bounds__(256)
+k_sell_fill_factor(SellView sv, int part, const int *__restrict__ brp, const int *__restrict__ diag_pos,
+                   const int4 *__restrict__ meta, const __nv_bfloat16 *__restrict__ g, uint2 *__restrict__ out) {
+  const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < sv.nslices; s += nw) {
+    const int v = sv.row[32 * s + lane];
+    const int nb = v >= 0 ? sell_range(part, brp, diag_pos, v).y : 0, rsp = padded_row(nb);
+    const int4 m = v >= 0 ? __ldg(meta + v) : make_int4(0, 0, 0, 0);
+    const __nv_bfloat16 *row = g + (part == kSellLower ? m.y : m.z);
+    const int g0 = sv.off[s], ng = sv.off[s + 1] - g0;
+    for (int c = 0; c < ng; ++c) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        unsigned w[6];  // 12 entries: blocks 4c .. 4c + 3, three columns each
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const int e = 12 * c + 4 * q;
+          const uint2 t = e < rsp ? __ldg(reinterpret_cast<const uint2 *>(row + (int64_t)r * rsp + e)) : make_uint2(0, 0);
+          w[2 * q] = t.x;
+          w[2 * q + 1] = t.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          unsigned h[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int e = 3 * j + k;
+            h[j] = 4 * c + j < nb ? (w[e / 2] >> (16 * (e & 1))) & 0xFFFFu : 0u;
+          }
+          out[288ll * (g0 + c) + 32 * (3 * r + k) + lane] = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+        }
+      }
+    }
+  }
+}
+
 SellPattern::~SellPattern() {
   if (off) cudaFree(off);
   if (row) cudaFree(row);
   if (col) cudaFree(col);
 }
 
-int plan_sell(bartels_mesh_plan plan, SellPattern **out) {
-  if (!plan->sell) {
+int plan_sell(bartels_mesh_plan plan, SellPattern **out, int part) {
+  SellPattern *&slot = part == kSellFull ? plan->sell : plan->sell_factor[part - 1];
+  if (!slot) {
     bartels_ctx ctx = plan->ctx;
     auto *p = new SellPattern();
-    plan->sell = p;
+    slot = p;
+    p->part = part;
     const int nwin = (plan->nV + kSellWindow - 1) / kSellWindow;
     p->nslices = nwin * (kSellWindow / 32);
     BT_CUDA(cudaMalloc(&p->row, sizeof(int) * 32 * (size_t)p->nslices));
     BT_CUDA(cudaMalloc(&p->off, sizeof(int) * ((size_t)p->nslices + 1)));
-    BT_LAUNCH(ctx, k_sell_order, nwin, kSellWindow, 0, plan->nV, plan->brp, p->row, p->off);
+    BT_LAUNCH(ctx, k_sell_order, nwin, kSellWindow, 0, plan->nV, part, plan->brp, plan->diag_pos, p->row,
+              p->off);
     std::vector<int> g(p->nslices + 1, 0);
     BT_CUDA(cudaMemcpyAsync(g.data() + 1, p->off, sizeof(int) * p->nslices, cudaMemcpyDeviceToHost, ctx->stream));
     BT_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -133,10 +185,11 @@ int plan_sell(bartels_mesh_plan plan, SellPattern **out) {
     p->groups = g[p->nslices];
     BT_CUDA(cudaMemcpyAsync(p->off, g.data(), sizeof(int) * (p->nslices + 1), cudaMemcpyHostToDevice, ctx->stream));
     BT_CUDA(cudaMalloc(&p->col, sizeof(int4) * 32 * (size_t)std::max<int64_t>(p->groups, 1)));
-    BT_LAUNCH(ctx, k_sell_cols, sell_grid(ctx, p->nslices, 1), 256, 0, p->view(), plan->brp, plan->bcol, p->col);
+    BT_LAUNCH(ctx, k_sell_cols, sell_grid(ctx, p->nslices, 1), 256, 0, p->view(), part, plan->brp,
+              plan->diag_pos, plan->bcol, p->col);
     BT_CUDA(cudaStreamSynchronize(ctx->stream));  // g is a local
   }
-  *out = plan->sell;
+  *out = slot;
   return BARTELS_OK;
 }
 
@@ -151,6 +204,14 @@ int sell_fill_bf16(bartels_ctx ctx, bartels_mesh_plan plan, const float *values,
   const SellView sv = plan->sell->view();
   const int g = std::max(1, std::min(sv.nslices, ctx->num_sms * 16));
   BT_LAUNCH(ctx, k_sell_fill<true>, g, 128, 0, sv, plan->brp, plan->bcol, values, rev, (void *)out);
+  return BARTELS_OK;
+}
+
+int sell_fill_factor(bartels_ctx ctx, bartels_mesh_plan plan, int part, const int4 *meta, const __nv_bfloat16 *g,
+                     uint2 *out) {
+  const SellView sv = plan->sell_factor[part - 1]->view();
+  BT_LAUNCH(ctx, k_sell_fill_factor, sell_grid(ctx, sv.nslices, 1), 256, 0, sv, part, plan->brp, plan->diag_pos, meta,
+            g, out);
   return BARTELS_OK;
 }
 

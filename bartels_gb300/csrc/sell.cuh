@@ -32,8 +32,13 @@ struct SellView {
   const int4 *col = nullptr;  // 32 per group: 3 x the column vertices of the lane's 4 blocks
 };
 
-// Storage of one layout (full rows), built on first use.
+// The blocks of a row that a layout holds: all of them, or the learned factor's lower
+// part (columns up to the diagonal) or upper part (from the diagonal on).
+enum SellPart { kSellFull = 0, kSellLower = 1, kSellUpper = 2 };
+
+// Storage of one layout, built on first use.
 struct SellPattern {
+  int part = kSellFull;
   int nslices = 0;
   int64_t groups = 0;
   int *off = nullptr, *row = nullptr;
@@ -41,12 +46,16 @@ struct SellPattern {
   ~SellPattern();
   SellView view() const { return {nslices, off, row, col}; }
 };
-int plan_sell(bartels_mesh_plan plan, SellPattern **out);
+int plan_sell(bartels_mesh_plan plan, SellPattern **out, int part = kSellFull);
 // values (scalar-CSR) into the layout: FP32 (9 groups x 32 float4) as they are
 int sell_fill_f32(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, float4 *out);
 // BF16, exactly symmetric: block (v, w), w < v, takes the transpose of (w, v), the
 // diagonal block its symmetric part; rev[p] is the position of block p's transpose
 int sell_fill_bf16(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, const int *rev, uint2 *out);
+// the factor's BF16 storage of that part (rows of three scalar rows padded to 4
+// entries; off[v].y / .z is a row's offset in the lower / upper storage)
+int sell_fill_factor(bartels_ctx ctx, bartels_mesh_plan plan, int part, const int4 *meta, const __nv_bfloat16 *g,
+                     uint2 *out);
 
 // Warps per slice: one where the slices fill the GPU; four (each takes every
 // fourth group) on small meshes, where a pass is bound by its chain of loads.

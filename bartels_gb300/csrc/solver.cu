@@ -1552,6 +1552,19 @@ static int mg_values(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
   if (learned) {
     BT_CHECK(lpcg_factor(plan->lpcg_net, plan, values, &sm.gl, &sm.gu));
     sm.fp = plan->factor;
+    if (sell_split(ctx, (plan->nV + 31) / 32) == 1) {
+      // the V-cycle applies it twice per iteration: lay it out once
+      SellPattern *lo, *up;
+      BT_CHECK(plan_sell(plan, &lo, kSellLower));
+      BT_CHECK(plan_sell(plan, &up, kSellUpper));
+      const size_t nl = 288 * (size_t)lo->groups, nu = 288 * (size_t)up->groups;
+      BT_CHECK(plan->w_sell_factor.ensure(sizeof(uint2) * std::max<size_t>(nl + nu, 1)));
+      uint2 *out = plan->w_sell_factor.as<uint2>();
+      BT_CHECK(sell_fill_factor(ctx, plan, kSellLower, plan->factor->meta, sm.gl, out));
+      BT_CHECK(sell_fill_factor(ctx, plan, kSellUpper, plan->factor->meta, sm.gu, out + nl));
+      sm.lsell = out;
+      sm.usell = out + nl;
+    }
   } else {
     BT_CHECK(plan->w_minv.ensure(24 * (size_t)plan->nV));
     BT_CHECK(launch_minv_blk(ctx, plan, values, plan->w_minv.as<float>()));
