@@ -1871,7 +1871,7 @@ int restrict_into(bartels_ctx ctx, MgHierarchy *mg, const MgLevel &f, const floa
   float *cx = fuse ? c.x : nullptr, *cr = fuse && !exact ? c.r : nullptr, *cd = fuse && !exact ? c.d : nullptr;
   const float *cf = fuse ? coef : nullptr;
   // A warp per aggregate while one per SM sub-partition's eight warps is enough for
-  // all: its ~25 members then are one round of loads (solve on 109k vertices, 4.6k
+  // all: its ~25 members then are one round of loads (solve on 117k vertices, 4.6k
   // aggregates: 13.4 -> 13.0 ms). With 34.8k aggregates eight lanes are faster
   // (48.4 ms, 16 or 32 lanes 49.1).
 #define BT_RL(L)                                                                                              \
