@@ -801,10 +801,13 @@ BT_HD float bt_expm1(float x) { return std::expm1(x); }
 // |j| < 11/16; a series below 0.02 and log1p above it took 14 and ~35, both in
 // a warp that has both.
 constexpr int kLogRows = 44;
+// (rows are read as one 16-byte load)
 #ifdef __CUDACC__
-static __device__
+alignas(16) static __device__ const double kLogTab[2 * kLogRows + 1][2] = {
+#else
+alignas(16) static const double kLogTab[2 * kLogRows + 1][2] = {
 #endif
-    const double kLogTab[2 * kLogRows + 1][2] = {  // 1 / (1 + k / 64) rounded to FP32, less 1; its log less that
+    // 1 / (1 + k / 64) rounded to FP32, less 1; its log less that
     {2.200000047683716, -1.036849222976874}, {2.047619104385376, -0.9332584401226758},
     {1.9090909957885742, -0.8412503359848963}, {1.7826087474822998, -0.7592198614253263},
     {1.6666667461395264, -0.6858374633254782}, {1.559999942779541, -0.619992706639812},
