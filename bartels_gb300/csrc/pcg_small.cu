@@ -83,8 +83,13 @@ __device__ __forceinline__ unsigned small_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ void small_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void small_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void small_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  small_arrive();
+  small_wait();
 }
 
 // Sums across warps and CTAs are unevaluated float pairs h + l (two-sum): exact to
@@ -157,6 +162,9 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
   extern __shared__ __align__(16) char sm[];
   __shared__ float s_warps[2][32];
   __shared__ __align__(8) float2 s_pap[kCtas], s_rz[2 * kCtas];
+  // A CTA's shared memory may be written by the others only once it is known to
+  // run: all arrive here and wait before the first reduction. Staging lies between.
+  small_arrive();
   const unsigned rank = small_rank();
   const int n = m.n, r0 = rank * m.rows, nr = max(0, min(m.rows, n - r0)), nv = (nr + 2) / 3;
   float *sp = reinterpret_cast<float *>(sm);           // the whole direction
@@ -229,6 +237,7 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
   const float st_beta = st->beta;
   int it = cont ? st->it : 0;
   const int last = it + max_it;
+  small_wait();
   small_reduce<2>(arz, arr, s_warps, s_rz, rank, d2);
   if (warp == 0) {
     // as k_pcg_init: beta against the replaced residual when the direction continues
