@@ -176,7 +176,8 @@ class MeshPlan:
     # --- energy / gradient / Hessian ------------------------------------
     def _elem(self, model, dphidX, volume, params, where):
         """The element data of an energy, gradient or Hessian call as the C entry's three pointers.
-        Row-major arrays go to the plan as they are; other forms are transposed here for the entry to upload."""
+        Row-major arrays go to the plan as they are; other forms are transposed here for the entry to upload.
+        Called last before the entry, which waits for the copies: nothing may fail between the two."""
         if ((dphidX is not None or params is not None) and _is_rows(dphidX, self.nT, 12)
                 and _is_rows(params, self.nT, 2)):
             v = None if volume is None else _f64(np.ravel(volume))
@@ -196,29 +197,30 @@ class MeshPlan:
         return keep, out
 
     def q(self, model, q, dphidX=None, volume=None, params=None) -> float:
-        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_q")
         qa = _f64(q)
         e = C.c_double()
+        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_q")
         check(lib().bartels_tetmesh_q(self.ctx.handle, self.handle, MODELS[model], _dptr(qa), d, v, p, C.byref(e)),
               "bartels_tetmesh_q")
         return e.value
 
     def dq(self, model, q, dphidX=None, volume=None, params=None):
-        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_dq")
         qa = _f64(q)
         g = np.zeros(3 * self.nV)
+        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_dq")
         check(lib().bartels_tetmesh_dq(self.ctx.handle, self.handle, MODELS[model], _dptr(qa), d, v, p, _dptr(g)),
               "bartels_tetmesh_dq")
         return g
 
     def dq2_values(self, model, q, dphidX=None, volume=None, params=None, psd_tol=None, corot_exact=False):
-        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_dq2")
         qa = _f64(q)
         vals = np.zeros(self.nnz)
         psd = _lib.PSD_NONE if psd_tol is None else _lib.PSD_SIMPLE_FIX
+        tol = float(psd_tol or 0.0)
         flags = _lib.DQ2_COROT_EXACT if corot_exact else 0
-        check(lib().bartels_tetmesh_dq2(self.ctx.handle, self.handle, MODELS[model], _dptr(qa), d, v, p, psd,
-                                        float(psd_tol or 0.0), flags, _dptr(vals)), "bartels_tetmesh_dq2")
+        keep, (d, v, p) = self._elem(model, dphidX, volume, params, "bartels_tetmesh_dq2")
+        check(lib().bartels_tetmesh_dq2(self.ctx.handle, self.handle, MODELS[model], _dptr(qa), d, v, p, psd, tol,
+                                        flags, _dptr(vals)), "bartels_tetmesh_dq2")
         return vals
 
     def dq2(self, model, q, dphidX=None, volume=None, params=None, psd_tol=None, corot_exact=False):

@@ -259,8 +259,8 @@ int bartels_plan_set_element_rows(bartels_mesh_plan plan, int model, const doubl
   if (!valid_model(model)) return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   BT_CHECK(check_ctx(plan->ctx));
   std::vector<double> pbuf;
-  return plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, true, pbuf), nullptr, true,
-                               false);
+  const double *pd = model_params(model, params, plan->nT, true, pbuf);
+  return plan_set_element_data(plan, dphidX, vol, pd, nullptr, true, !pbuf.empty());
 }
 
 int bartels_plan_csr_size(bartels_mesh_plan plan, int *n, int64_t *nnz) {
@@ -290,6 +290,7 @@ int bartels_tetmesh_q(bartels_ctx ctx, bartels_mesh_plan plan, int model, const 
   BT_CHECK(check_plan(ctx, plan));
   if (!valid_model(model) || !q || !energy_out) return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   std::vector<double> pbuf;
+  StreamWait wait{ctx->stream};  // the copies read pbuf and the caller's arrays
   BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, false, pbuf), nullptr, false,
                                  false));
   double *dq;
@@ -299,6 +300,7 @@ int bartels_tetmesh_q(bartels_ctx ctx, bartels_mesh_plan plan, int model, const 
   BT_CHECK(energy(ctx, plan, model, obj, dq, ctx->scalars.as<double>()));
   BT_CUDA(cudaMemcpyAsync(ctx->host_scalars, ctx->scalars.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  wait.armed = false;
   *energy_out = ctx->host_scalars[0];
   if (!std::isfinite(*energy_out)) return fail(BARTELS_E_NONFINITE, "energy is not finite (J <= 0 for Neo-Hookean?)");
   return BARTELS_OK;
@@ -309,6 +311,7 @@ int bartels_tetmesh_dq(bartels_ctx ctx, bartels_mesh_plan plan, int model, const
   BT_CHECK(check_plan(ctx, plan));
   if (!valid_model(model) || !q || !g) return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   std::vector<double> pbuf;
+  StreamWait wait{ctx->stream};  // the copies read pbuf and the caller's arrays
   BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, false, pbuf), nullptr, false,
                                  false));
   const size_t n = 3 * (size_t)plan->nV;
@@ -319,6 +322,7 @@ int bartels_tetmesh_dq(bartels_ctx ctx, bartels_mesh_plan plan, int model, const
   BT_CHECK(gradient(ctx, plan, model, obj, dq, plan->w_vec.as<double>()));
   BT_CUDA(cudaMemcpyAsync(g, plan->w_vec.p, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  wait.armed = false;
   for (size_t i = 0; i < n; ++i)
     if (!std::isfinite(g[i])) return fail(BARTELS_E_NONFINITE, "gradient is not finite");
   return BARTELS_OK;
@@ -331,6 +335,7 @@ int bartels_tetmesh_dq2(bartels_ctx ctx, bartels_mesh_plan plan, int model, cons
   if (!valid_model(model) || !q || !csr_values || (psd_mode != BARTELS_PSD_NONE && psd_mode != BARTELS_PSD_SIMPLE_FIX))
     return fail(BARTELS_E_INVALID_ARG, "bad arguments");
   std::vector<double> pbuf;
+  StreamWait wait{ctx->stream};  // the copies read pbuf and the caller's arrays
   BT_CHECK(plan_set_element_data(plan, dphidX, vol, model_params(model, params, plan->nT, false, pbuf), nullptr, false,
                                  false));
   const size_t n = 3 * (size_t)plan->nV;
@@ -347,6 +352,7 @@ int bartels_tetmesh_dq2(bartels_ctx ctx, bartels_mesh_plan plan, int model, cons
   BT_CHECK(values_to_double(ctx, plan->w_values.as<float>(), ctx->stage_d.as<double>(), nnz));
   BT_CUDA(cudaMemcpyAsync(csr_values, ctx->stage_d.p, sizeof(double) * nnz, cudaMemcpyDeviceToHost, ctx->stream));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  wait.armed = false;
   return BARTELS_OK;
 }
 

@@ -124,6 +124,16 @@ struct SegInfo {
   ~SegInfo();
 };
 
+// Waits for the stream where it goes out of scope, unless disarmed: host memory
+// declared before it outlives the copies that read it, on every return.
+struct StreamWait {
+  cudaStream_t stream;
+  bool armed = true;
+  ~StreamWait() {
+    if (armed) cudaStreamSynchronize(stream);
+  }
+};
+
 // Device buffer with geometric growth.
 struct DevBuf {
   void *p = nullptr;

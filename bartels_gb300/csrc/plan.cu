@@ -202,13 +202,16 @@ int plan_build(bartels_mesh_plan plan, const double *V, const int *E) {
 
 // Upload caller element data (reference layouts) into the plan.
 // rows: dphidX (nT x 12) and params (nT x 2) are row-major, else column-major. Without
-// `sync` the records may still be under way on the context's stream on return
-// (pageable sources have been staged by then).
+// `sync` the copies may still read the caller's arrays on return (CUDA does not
+// promise that a pageable source has been staged by then), so they have to outlive
+// the context's next wait. Any failure waits first.
 int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const double *vol, const double *params,
                           const double *density, bool rows, bool sync) {
   bartels_ctx ctx = plan->ctx;
   const size_t nT = (size_t)plan->nT;
   if (nT == 0) return BARTELS_OK;
+  std::vector<double> p;  // column-major parameters per tet; outlives the wait
+  StreamWait wait{ctx->stream};
   bool changed = false;
   if (dphidX) {
     BT_CHECK(ctx->stage_a.ensure(sizeof(double) * 12 * nT));
@@ -233,7 +236,7 @@ int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const do
     changed = true;
   } else if (params) {
     // column-major nT x 2 -> per-tet pairs
-    std::vector<double> p(2 * nT);
+    p.resize(2 * nT);
     for (size_t t = 0; t < nT; ++t) {
       p[2 * t] = params[t];
       p[2 * t + 1] = params[t + nT];
@@ -246,7 +249,8 @@ int plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, const do
     changed = true;
   }
   if (changed) BT_CHECK(plan_refresh_records(plan));
-  if (sync) BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (sync || !p.empty()) BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  wait.armed = false;
   return BARTELS_OK;
 }
 

@@ -131,8 +131,9 @@ int bartels_plan_set_element_data(bartels_mesh_plan plan, const double *dphidX, 
 /* The element data of the energy, gradient and Hessian entries below for `model`,
  * with dphidX (nT x 12) and params (nT x 2) row-major: no transposition on the
  * host (48,000 tets: 0.9 ms per call in NumPy). Any pointer may be NULL as above.
- * It does not wait for the device: buffers in pinned memory stay unchanged until
- * the plan's next call has returned. */
+ * It does not wait for the device: the buffers, pinned or not, stay alive and
+ * unchanged until an entry below that returns an energy, a gradient or a Hessian
+ * of the plan, or bartels_ctx_synchronize, has returned. */
 int bartels_plan_set_element_rows(bartels_mesh_plan plan, int model, const double *dphidX, const double *vol,
                                   const double *params);
 /* Scalar CSR size of the 3nV x 3nV pattern. */
