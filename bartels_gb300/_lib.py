@@ -64,6 +64,7 @@ _P = C.c_void_p
 SIGNATURES = [
     ("bartels_status_string", C.c_char_p, [C.c_int]),
     ("bartels_last_error", C.c_char_p, []),
+    ("bartels_fail_alloc", C.c_int64, [C.c_int64]),
     ("bartels_ctx_create", C.c_int, [C.c_int, C.POINTER(_P)]),
     ("bartels_ctx_destroy", C.c_int, [_P]),
     ("bartels_ctx_synchronize", C.c_int, [_P]),

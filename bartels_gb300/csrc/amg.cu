@@ -256,7 +256,7 @@ int upload(MgHierarchy *mg, T **dst, const std::vector<T> &src) {
   *dst = nullptr;
   if (src.empty()) return BARTELS_OK;
   void *p = nullptr;
-  BT_CUDA(cudaMalloc(&p, sizeof(T) * src.size()));
+  BT_CUDA(dev_malloc(&p, sizeof(T) * src.size()));
   mg->allocs.push_back(p);
   BT_CUDA(cudaMemcpy(p, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
   *dst = static_cast<T *>(p);
@@ -266,7 +266,7 @@ int upload(MgHierarchy *mg, T **dst, const std::vector<T> &src) {
 int dalloc(MgHierarchy *mg, void **dst, size_t bytes) {
   *dst = nullptr;
   if (bytes == 0) return BARTELS_OK;
-  BT_CUDA(cudaMalloc(dst, (bytes + 255) & ~size_t(255)));
+  BT_CUDA(dev_malloc(dst, (bytes + 255) & ~size_t(255)));
   mg->allocs.push_back(*dst);
   return BARTELS_OK;
 }

@@ -116,6 +116,8 @@ const char *bartels_status_string(int s) {
 
 const char *bartels_last_error(void) { return last_error_cstr(); }
 
+int64_t bartels_fail_alloc(int64_t n) { return set_fail_alloc(n); }
+
 int bartels_ctx_create(int device, bartels_ctx *out) {
   if (!out) return fail(BARTELS_E_INVALID_ARG, "null output");
   int count = 0;
@@ -554,7 +556,7 @@ int bartels_newton_set_problem(bartels_mesh_plan plan, const double *q_base, con
       *dst = nullptr;
       return BARTELS_OK;
     }
-    if (!*dst) BT_CUDA(cudaMalloc(dst, sizeof(double) * n));
+    if (!*dst) BT_CUDA(dev_malloc(dst, sizeof(double) * n));
     BT_CUDA(cudaMemcpyAsync(*dst, src, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
     return BARTELS_OK;
   };
@@ -574,7 +576,7 @@ int bartels_newton_set_problem(bartels_mesh_plan plan, const double *q_base, con
     plan->pinned_gen++;
   }
   if (pinned) {
-    if (!plan->pinned) BT_CUDA(cudaMalloc(&plan->pinned, (size_t)plan->nV));
+    if (!plan->pinned) BT_CUDA(dev_malloc(&plan->pinned, (size_t)plan->nV));
     BT_CUDA(cudaMemcpyAsync(plan->pinned, pinned, (size_t)plan->nV, cudaMemcpyHostToDevice, ctx->stream));
   } else if (plan->pinned) {
     cudaFree(plan->pinned);

@@ -1249,8 +1249,13 @@ int noalloc_gradient(bartels_ctx ctx, bartels_mesh_plan plan, int model, const d
 int plan_build_csr_pattern(bartels_mesh_plan plan) {
   if (plan->csr_rp) return BARTELS_OK;
   bartels_ctx ctx = plan->ctx;
-  BT_CUDA(cudaMalloc(&plan->csr_rp, sizeof(int) * (3 * (size_t)plan->nV + 1)));
-  BT_CUDA(cudaMalloc(&plan->csr_col, sizeof(int) * 9 * (size_t)plan->nnzb));
+  BT_CUDA(dev_malloc(&plan->csr_rp, sizeof(int) * (3 * (size_t)plan->nV + 1)));
+  const cudaError_t e = dev_malloc(&plan->csr_col, sizeof(int) * 9 * (size_t)plan->nnzb);
+  if (e != cudaSuccess) {  // the row pointers alone would read as a complete pattern
+    cudaFree(plan->csr_rp);
+    plan->csr_rp = nullptr;
+    BT_CUDA(e);
+  }
   BT_LAUNCH(ctx, k_csr_pattern, grid_for(ctx, plan->nV, 128), 128, 0, plan->nV, plan->brp, plan->bcol, plan->csr_rp,
             plan->csr_col);
   return BARTELS_OK;

@@ -124,6 +124,16 @@ struct SegInfo {
   ~SegInfo();
 };
 
+// cudaMalloc, with *p = nullptr and no pending error where it fails. set_fail_alloc(n) has the
+// calling thread's n-th allocation from now on fail (0: none) and returns how many were still
+// to come before the one set earlier (0: it has failed, or none was set).
+cudaError_t dev_malloc(void **p, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(T **p, size_t bytes) {
+  return dev_malloc(reinterpret_cast<void **>(p), bytes);
+}
+int64_t set_fail_alloc(int64_t n);
+
 // Waits for the stream where it goes out of scope, unless disarmed: host memory
 // declared before it outlives the copies that read it, on every return.
 struct StreamWait {

@@ -1097,7 +1097,7 @@ static int grid_warps(bartels_ctx ctx, int64_t nwarps) { return grid_for_n(ctx, 
 template <class T>
 static int lp_alloc(LpcgPlanState &s, T **p, size_t n) {
   void *q = nullptr;
-  BT_CUDA(cudaMalloc(&q, sizeof(T) * std::max<size_t>(n, 1)));
+  BT_CUDA(dev_malloc(&q, sizeof(T) * std::max<size_t>(n, 1)));
   s.allocs.push_back(q);
   *p = static_cast<T *>(q);
   return BARTELS_OK;
@@ -1437,13 +1437,13 @@ int lpcg_create(bartels_ctx ctx, bartels_lpcg *out) {
   n->ctx = ctx;
   const size_t P = kL.total;
   cudaError_t e = cudaSuccess;
-  e = e == cudaSuccess ? cudaMalloc(&n->params, 4 * P) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->grad, 4 * P) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->m, 4 * P) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->v, 4 * P) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->wbf, 2 * (size_t)kB.total) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->err, sizeof(int)) : e;
-  e = e == cudaSuccess ? cudaMalloc(&n->scal, (8 + 2 * kNormParts) * sizeof(double)) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->params, 4 * P) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->grad, 4 * P) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->m, 4 * P) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->v, 4 * P) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->wbf, 2 * (size_t)kB.total) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->err, sizeof(int)) : e;
+  e = e == cudaSuccess ? dev_malloc(&n->scal, (8 + 2 * kNormParts) * sizeof(double)) : e;
   if (e == cudaSuccess) e = cudaMemsetAsync(n->params, 0, 4 * P, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(n->grad, 0, 4 * P, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(n->m, 0, 4 * P, ctx->stream);

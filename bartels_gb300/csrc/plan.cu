@@ -32,13 +32,31 @@ int fail(int status, const std::string &msg) {
 }
 const char *last_error_cstr() { return g_last_error.c_str(); }
 
+static thread_local int64_t g_fail_alloc = 0;  // allocations up to the one reported as failed (0: none)
+int64_t set_fail_alloc(int64_t n) {
+  const int64_t left = g_fail_alloc;
+  g_fail_alloc = n > 0 ? n : 0;
+  return left;
+}
+
+cudaError_t dev_malloc(void **p, size_t bytes) {
+  *p = nullptr;
+  if (g_fail_alloc > 0 && --g_fail_alloc == 0) return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();  // reported here: the next launch's check must not find it again
+  }
+  return e;
+}
+
 int DevBuf::ensure(size_t n) {
   if (n <= bytes) return BARTELS_OK;
   const size_t want = std::max(n, bytes + bytes / 2);
   if (p) cudaFree(p);
   p = nullptr;
   bytes = 0;
-  cudaError_t e = cudaMalloc(&p, want);
+  cudaError_t e = dev_malloc(&p, want);
   if (e != cudaSuccess) {
     p = nullptr;
     return fail(BARTELS_E_DEVICE, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -57,7 +75,7 @@ int launch_import_dphi(bartels_ctx ctx, bartels_mesh_plan plan, const double *sr
 
 template <class T>
 static int upload(bartels_ctx ctx, T **dst, const T *src, size_t n) {
-  BT_CUDA(cudaMalloc(dst, sizeof(T) * std::max<size_t>(n, 1)));
+  BT_CUDA(dev_malloc(dst, sizeof(T) * std::max<size_t>(n, 1)));
   if (n) BT_CUDA(cudaMemcpyAsync(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream));
   return BARTELS_OK;
 }
@@ -182,14 +200,14 @@ int plan_build(bartels_mesh_plan plan, const double *V, const int *E) {
   BT_CHECK(upload(ctx, &plan->diag_pos, diag.data(), diag.size()));
   BT_CHECK(upload(ctx, &plan->chunk_v, chunks.data(), chunks.size()));
   // --- element data defaults: geometry from V, params and density zero
-  BT_CUDA(cudaMalloc(&plan->dphi64, sizeof(double) * 9 * std::max<size_t>(nT, 1)));
-  BT_CUDA(cudaMalloc(&plan->vol, sizeof(double) * std::max<size_t>(nT, 1)));
-  BT_CUDA(cudaMalloc(&plan->params, sizeof(double) * 2 * std::max<size_t>(nT, 1)));
-  BT_CUDA(cudaMalloc(&plan->density, sizeof(double) * std::max<size_t>(nT, 1)));
+  BT_CUDA(dev_malloc(&plan->dphi64, sizeof(double) * 9 * std::max<size_t>(nT, 1)));
+  BT_CUDA(dev_malloc(&plan->vol, sizeof(double) * std::max<size_t>(nT, 1)));
+  BT_CUDA(dev_malloc(&plan->params, sizeof(double) * 2 * std::max<size_t>(nT, 1)));
+  BT_CUDA(dev_malloc(&plan->density, sizeof(double) * std::max<size_t>(nT, 1)));
   BT_CUDA(cudaMemsetAsync(plan->params, 0, sizeof(double) * 2 * (size_t)nT, ctx->stream));
   BT_CUDA(cudaMemsetAsync(plan->density, 0, sizeof(double) * (size_t)nT, ctx->stream));
-  BT_CUDA(cudaMalloc(&plan->rec32, sizeof(TetRec32) * std::max<size_t>(nT, 1)));
-  BT_CUDA(cudaMalloc(&plan->rec64, sizeof(TetRec64) * std::max<size_t>(nT, 1)));
+  BT_CUDA(dev_malloc(&plan->rec32, sizeof(TetRec32) * std::max<size_t>(nT, 1)));
+  BT_CUDA(dev_malloc(&plan->rec64, sizeof(TetRec64) * std::max<size_t>(nT, 1)));
   if (nT > 0) {
     BT_CHECK(launch_dphi_vol(ctx, nV, plan->X, nT, plan->E, nullptr, plan->dphi64, plan->vol));
     BT_CHECK(plan_refresh_records(plan));
@@ -285,7 +303,7 @@ int plan_chunks64(bartels_mesh_plan plan) {
     floats += need;
   }
   if (chunks.back() != plan->nV) chunks.push_back(plan->nV);
-  BT_CUDA(cudaMalloc(&plan->chunk_v64, sizeof(int) * chunks.size()));
+  BT_CUDA(dev_malloc(&plan->chunk_v64, sizeof(int) * chunks.size()));
   BT_CUDA(cudaMemcpy(plan->chunk_v64, chunks.data(), sizeof(int) * chunks.size(), cudaMemcpyHostToDevice));
   plan->nchunks64 = (int)chunks.size() - 1;
   return BARTELS_OK;

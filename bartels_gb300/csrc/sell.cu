@@ -1,5 +1,6 @@
 // Building and filling the sliced-ELL layout (sell.cuh).
 #include <algorithm>
+#include <memory>
 #include <vector>
 
 #include "lpcg_internal.cuh"
@@ -168,26 +169,28 @@ int plan_sell(bartels_mesh_plan plan, SellPattern **out, int part) {
   SellPattern *&slot = part == kSellFull ? plan->sell : plan->sell_factor[part - 1];
   if (!slot) {
     bartels_ctx ctx = plan->ctx;
-    auto *p = new SellPattern();
-    slot = p;
+    std::unique_ptr<SellPattern> p(new SellPattern());  // the plan's once it is complete
     p->part = part;
     const int nwin = (plan->nV + kSellWindow - 1) / kSellWindow;
     p->nslices = nwin * (kSellWindow / 32);
-    BT_CUDA(cudaMalloc(&p->row, sizeof(int) * 32 * (size_t)p->nslices));
-    BT_CUDA(cudaMalloc(&p->off, sizeof(int) * ((size_t)p->nslices + 1)));
+    BT_CUDA(dev_malloc(&p->row, sizeof(int) * 32 * (size_t)p->nslices));
+    BT_CUDA(dev_malloc(&p->off, sizeof(int) * ((size_t)p->nslices + 1)));
     BT_LAUNCH(ctx, k_sell_order, nwin, kSellWindow, 0, plan->nV, part, plan->brp, plan->diag_pos, p->row,
               p->off);
     std::vector<int> g(p->nslices + 1, 0);
+    StreamWait wait{ctx->stream};  // the copies below read and write g
     BT_CUDA(cudaMemcpyAsync(g.data() + 1, p->off, sizeof(int) * p->nslices, cudaMemcpyDeviceToHost, ctx->stream));
     BT_CUDA(cudaStreamSynchronize(ctx->stream));
     for (int s = 0; s < p->nslices; ++s) g[s + 1] += g[s];
     while (p->nslices > 0 && g[p->nslices] == g[p->nslices - 1]) p->nslices--;  // slices past the last vertex
     p->groups = g[p->nslices];
     BT_CUDA(cudaMemcpyAsync(p->off, g.data(), sizeof(int) * (p->nslices + 1), cudaMemcpyHostToDevice, ctx->stream));
-    BT_CUDA(cudaMalloc(&p->col, sizeof(int4) * 32 * (size_t)std::max<int64_t>(p->groups, 1)));
+    BT_CUDA(dev_malloc(&p->col, sizeof(int4) * 32 * (size_t)std::max<int64_t>(p->groups, 1)));
     BT_LAUNCH(ctx, k_sell_cols, sell_grid(ctx, p->nslices, 1), 256, 0, p->view(), part, plan->brp,
               plan->diag_pos, plan->bcol, p->col);
-    BT_CUDA(cudaStreamSynchronize(ctx->stream));  // g is a local
+    BT_CUDA(cudaStreamSynchronize(ctx->stream));
+    wait.armed = false;
+    slot = p.release();
   }
   *out = slot;
   return BARTELS_OK;

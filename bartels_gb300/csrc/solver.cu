@@ -1623,7 +1623,7 @@ int plan_set_segments(bartels_mesh_plan plan, int nseg, const int *voff, const i
   sg->h_toff.assign(toff, toff + nseg + 1);
   sg->active.assign(nseg, 1);
   auto alloc = [&](void **dst, size_t bytes) -> int {
-    BT_CUDA(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
+    BT_CUDA(dev_malloc(dst, std::max<size_t>(bytes, 16)));
     sg->allocs.push_back(*dst);
     return BARTELS_OK;
   };
@@ -2051,10 +2051,10 @@ __global__ void k_advance_ie(int n, double dt, const double *__restrict__ v, dou
 int advance_implicit_euler(bartels_ctx ctx, bartels_mesh_plan plan, double dt, const double *v) {
   const int n = 3 * plan->nV;
   if (!plan->q_base) {
-    BT_CUDA(cudaMalloc(&plan->q_base, sizeof(double) * n));
+    BT_CUDA(dev_malloc(&plan->q_base, sizeof(double) * n));
     BT_CUDA(cudaMemsetAsync(plan->q_base, 0, sizeof(double) * n, ctx->stream));
   }
-  if (!plan->x_hat) BT_CUDA(cudaMalloc(&plan->x_hat, sizeof(double) * n));
+  if (!plan->x_hat) BT_CUDA(dev_malloc(&plan->x_hat, sizeof(double) * n));
   BT_LAUNCH(ctx, k_advance_ie, grid_vec(ctx, n), 256, 0, n, dt, v, plan->q_base, plan->x_hat);
   return BARTELS_OK;
 }
@@ -2250,9 +2250,9 @@ int plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, 
       cudaEventElapsedTime(&ms, e0, e1);
       return ms;
     };
-    if (cudaMalloc(&x, 4 * n) != cudaSuccess || cudaMalloc(&y, 4 * n) != cudaSuccess ||
-        cudaMalloc(&gl, 2 * (size_t)fp->lsize + 16) != cudaSuccess || cudaMalloc(&st, sizeof(PcgState)) != cudaSuccess ||
-        cudaMalloc(&part, 8 * 4096) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
+    if (dev_malloc(&x, 4 * n) != cudaSuccess || dev_malloc(&y, 4 * n) != cudaSuccess ||
+        dev_malloc(&gl, 2 * (size_t)fp->lsize + 16) != cudaSuccess || dev_malloc(&st, sizeof(PcgState)) != cudaSuccess ||
+        dev_malloc(&part, 8 * 4096) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
         cudaEventCreate(&e1) != cudaSuccess) {
       cleanup();
       return fail(BARTELS_E_DEVICE, "autotuner scratch allocation failed");

@@ -336,7 +336,7 @@ __global__ void k_tri3d_stvk_hess(int nT, const int4 *__restrict__ E, const doub
 
 template <class T>
 int tri_upload(bartels_ctx ctx, T **dst, const T *src, size_t n) {
-  BT_CUDA(cudaMalloc(dst, sizeof(T) * std::max<size_t>(n, 1)));
+  BT_CUDA(dev_malloc(dst, sizeof(T) * std::max<size_t>(n, 1)));
   if (n) BT_CUDA(cudaMemcpyAsync(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream));
   return BARTELS_OK;
 }

@@ -103,6 +103,11 @@ int bartels_ctx_destroy(bartels_ctx ctx);
 int bartels_ctx_synchronize(bartels_ctx ctx);
 /* The context's cudaStream_t, as void*. */
 void *bartels_ctx_stream(bartels_ctx ctx);
+/* For tests of out-of-memory handling: the calling thread's n-th device
+ * allocation by this library from now on reports out-of-memory instead of being
+ * made (0: none). Returns how many allocations were still to come before the one
+ * set earlier (0: it has been reported, or none was set). */
+int64_t bartels_fail_alloc(int64_t n);
 /* Number of kernels this library enqueued on ctx since creation. */
 int64_t bartels_ctx_kernel_launches(bartels_ctx ctx);
 
