@@ -29,6 +29,7 @@
 // FP32 master weights and refreshes the BF16 copies the GEMMs read.
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "internal.cuh"
@@ -1119,8 +1120,8 @@ static int lp_state(bartels_mesh_plan plan, bool train, int nprobe, LpcgPlanStat
   }
   lp_state_free(s);
   plan->lpcg = nullptr;
-  s = new LpcgPlanState();
-  plan->lpcg = s;
+  std::unique_ptr<LpcgPlanState, void (*)(LpcgPlanState *)> own(new LpcgPlanState(), lp_state_free);
+  s = own.get();
   const size_t nV = plan->nV, nnzb = plan->nnzb, nnzl = fp->nnzl;
   s->nV = plan->nV;
   s->nnzb = plan->nnzb;

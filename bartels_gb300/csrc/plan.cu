@@ -190,6 +190,7 @@ int plan_build(bartels_mesh_plan plan, const double *V, const int *E) {
   plan->h_bcol = bcol;
   plan->h_chunk_v = chunks;
   // --- upload
+  StreamWait wait{ctx->stream};  // the copies read the arrays above
   BT_CHECK(upload(ctx, &plan->X, X.data(), X.size()));
   BT_CHECK(upload(ctx, &plan->E, E4.data(), E4.size()));
   BT_CHECK(upload(ctx, &plan->inc_ptr, inc_ptr.data(), inc_ptr.size()));
@@ -215,6 +216,7 @@ int plan_build(bartels_mesh_plan plan, const double *V, const int *E) {
   plan->dphi_matches_rest = true;
   BT_CHECK(plan_chunks64(plan));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  wait.armed = false;
   return BARTELS_OK;
 }
 
@@ -314,6 +316,7 @@ int plan_factor_pattern(bartels_mesh_plan plan, FactorPattern **out) {
   FactorPattern &f = *plan->factor;
   *out = plan->factor;
   if (f.built) return BARTELS_OK;
+  f.release();  // of an attempt that ran out of memory
   const int nV = plan->nV;
   const std::vector<int> &brp = plan->h_brp, &bcol = plan->h_bcol;
   std::vector<int> diag(nV), lrp(nV + 1, 0), urp(nV + 1, 0);
@@ -357,6 +360,7 @@ int plan_factor_pattern(bartels_mesh_plan plan, FactorPattern **out) {
   f.lsize = lseg;
   f.usize = useg;
   bartels_ctx ctx = plan->ctx;
+  StreamWait wait{ctx->stream};  // the copies read the arrays above
   BT_CHECK(upload(ctx, &f.meta, meta.data(), meta.size()));
   BT_CHECK(upload(ctx, &f.lrp, lrp.data(), lrp.size()));
   BT_CHECK(upload(ctx, &f.urp, urp.data(), urp.size()));
@@ -364,6 +368,7 @@ int plan_factor_pattern(bartels_mesh_plan plan, FactorPattern **out) {
   BT_CHECK(upload(ctx, &f.up2low, up2low.data(), up2low.size()));
   BT_CHECK(upload(ctx, &f.rev, rev.data(), rev.size()));
   BT_CUDA(cudaStreamSynchronize(ctx->stream));
+  wait.armed = false;
   f.nnzl = nnzl;
   f.nnzu = nnzu;
   f.built = true;

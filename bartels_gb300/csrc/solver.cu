@@ -18,6 +18,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <vector>
 
 #include "devmath.cuh"
@@ -1616,8 +1617,7 @@ int plan_set_segments(bartels_mesh_plan plan, int nseg, const int *voff, const i
           return fail(BARTELS_E_INVALID_ARG, "tet " + std::to_string(t) + " has a vertex outside its segment");
     }
   }
-  auto *sg = new SegInfo();
-  plan->seg = sg;
+  std::unique_ptr<SegInfo> sg(new SegInfo());  // the plan's once it is complete
   sg->nseg = nseg;
   sg->h_voff.assign(voff, voff + nseg + 1);
   sg->h_toff.assign(toff, toff + nseg + 1);
@@ -1663,6 +1663,7 @@ int plan_set_segments(bartels_mesh_plan plan, int nseg, const int *voff, const i
   BT_CUDA(cudaMemcpy(sg->toff, toff, sizeof(int64_t) * (nseg + 1), cudaMemcpyHostToDevice));
   BT_CUDA(cudaMemcpy(sg->vseg, vseg.data(), sizeof(int) * plan->nV, cudaMemcpyHostToDevice));
   BT_CUDA(cudaMemcpy(sg->tseg, tseg.data(), sizeof(int) * plan->nT, cudaMemcpyHostToDevice));
+  plan->seg = sg.release();
   return BARTELS_OK;
 }
 

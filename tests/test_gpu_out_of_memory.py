@@ -67,3 +67,72 @@ def _with_values(n):
 @pytest.mark.parametrize("n", [6, 21])  # the cluster's small solve, and the loop over the sliced-ELL copy
 def test_block_jacobi_solve(n):
     _sweep(_with_values(n), _solver("jacobi"), 30)
+
+
+def test_packed_segments():
+    import ctypes as C
+    import bartels_gb300 as bg
+    from bartels_gb300 import _lib
+    from bartels_gb300.meshes import kuhn_cube, material_params
+    from test_gpu_multigrid import _hessian, _plan as make_plan, _rhs, _solve
+    Vs, Es, voff, toff = [], [], [0], [0]
+    for n in (2, 9, 5):
+        V, E = kuhn_cube(n)
+        Vs.append(V)
+        Es.append(E + voff[-1])
+        voff.append(voff[-1] + len(V))
+        toff.append(toff[-1] + len(E))
+    V, E = np.concatenate(Vs), np.concatenate(Es).astype(np.int32)
+    pinned = np.abs(V[:, 2]) < 1e-12
+    vo, to = np.array(voff, np.int32), np.array(toff, np.int64)
+
+    def make():
+        plan = make_plan(V, E, material_params("neohookean", len(E), 2e6, 0.45), pinned)
+        return plan, _hessian(plan, V + 0.002 * np.random.default_rng(0).uniform(-1, 1, V.shape))
+
+    def call(state):
+        plan, vals = state
+        _lib.check(bg.lib().bartels_plan_set_segments(plan.handle, 3, vo.ctypes.data_as(C.POINTER(C.c_int)),
+                                                      to.ctypes.data_as(C.POINTER(C.c_int64))), "set_segments")
+        x, rep = _solve(plan, vals, _rhs(len(V), pinned), "jacobi")
+        assert rep.converged
+        return x
+
+    _sweep(make, call, 60)
+
+
+@pytest.mark.parametrize("what", ["factor", "train"])
+def test_learned_preconditioner(what):
+    from bartels_gb300 import lpcg
+    from bartels_gb300.lpcg import LearnedPreconditioner
+    from test_gpu_multigrid import _rhs, _torch
+    torch = _torch()
+
+    class Both:  # a plan and its network, closed together
+        def __init__(self, plan, net):
+            self.plan, self.net = plan, net
+
+        def close(self):
+            self.plan.close()
+            self.net.close()
+
+    values = _with_values(5)
+
+    def make():
+        plan, V, vals, pinned = values()
+        net = LearnedPreconditioner.load(ctx=plan.ctx)
+        if what == "factor":
+            net.attach(plan)
+        return Both(plan, net), V, vals, pinned
+
+    def call(state):
+        both, V, vals, pinned = state
+        if what == "train":
+            loss = both.net.train_step(both.plan, vals, None, nprobes=2, seed=3, lr=0.0)
+            return np.append(both.net.grad(), loss)
+        b = _rhs(len(V), pinned)
+        x = torch.zeros_like(b)
+        assert lpcg.plan_pcg(both.plan, vals, b, x, rel_tol=1e-8, max_iters=20000).converged
+        return x.cpu().numpy()
+
+    _sweep(make, call, 120)
