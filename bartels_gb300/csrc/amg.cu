@@ -47,6 +47,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 
 #include "amg_internal.cuh"
 #include "lpcg_internal.cuh"
@@ -507,8 +508,8 @@ int mg_prepare(bartels_ctx ctx, bartels_mesh_plan plan) {
   }
   if (H.size() < 2) return fail(BARTELS_E_UNSUPPORTED, "multigrid: the system is too small for a coarse level");
 
-  auto *mg = new MgHierarchy();
-  plan->mg = mg;
+  std::unique_ptr<MgHierarchy> own(new MgHierarchy());  // the plan's once it is complete
+  MgHierarchy *mg = own.get();
   mg->pinned_gen = plan->pinned_gen;
   mg->dense = dense;
   mg->coarse_blockdiag = dense ? 0 : coarse_blockdiag;
@@ -595,6 +596,7 @@ int mg_prepare(bartels_ctx ctx, bartels_mesh_plan plan) {
   BT_CUDA(cudaMemset(mg->coef, 0, sizeof(float) * kMgMaxLevels * kMgCoef));
   BT_CHECK(build_cluster(ctx, mg, H));
   if (mg->cl.ctas && mg->cl.first == 1 && H.size() > 2) mg->lv[1].deg = mg->cl.lv[0].deg = degcl;
+  plan->mg = own.release();
   return BARTELS_OK;
 }
 
@@ -2049,6 +2051,7 @@ int mg_setup_numeric(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
   // segment on the finest level of a packed plan)
   const int nseg = (plan->seg && plan->seg->nseg > 0) ? plan->seg->nseg : 0;
   if (nseg > mg->segn_n) {
+    mg->segn_n = 0;
     BT_CHECK(dalloc_n(mg, &mg->segn, 2 * (size_t)nseg));
     mg->segn_n = nseg;
   }

@@ -136,3 +136,12 @@ def test_learned_preconditioner(what):
         return x.cpu().numpy()
 
     _sweep(make, call, 120)
+
+
+@pytest.mark.parametrize("kind", ["multigrid", "learned_multigrid"])
+def test_multigrid_solve(kind):
+    import bartels_gb300 as bg
+    from bartels_gb300.lpcg import LearnedPreconditioner
+    net = LearnedPreconditioner.load(ctx=bg.Context.default())
+    _sweep(_with_values(8), _solver(kind, net), 160)
+    net.close()
