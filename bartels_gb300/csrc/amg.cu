@@ -366,65 +366,73 @@ int64_t cluster_layout(MgClArgs &a) {
 
 // The coarse part of the hierarchy as one cluster launch (k_mgc_cluster):
 // levels from the finest one that fits the cluster's shared memory down to the
-// coarsest. Leaves cl.ctas = 0 (the per-level launches) when not even the
-// coarsest level fits or the device cannot host the cluster.
+// coarsest, on 16 CTAs or, where the device cannot host so many as one cluster,
+// 8 or 4. Leaves cl.ctas = 0 (the per-level launches) when not even the coarsest
+// level fits or no cluster can be hosted.
 int build_cluster(bartels_ctx ctx, MgHierarchy *mg, const std::vector<HostLevel> &H) {
   constexpr int kSmem = 220 * 1024;
   const int L = (int)H.size();
-  const int want = env_int("BARTELS_MG_CLUSTER", kMgClusterMax, 4, kMgClusterMax);
+  int want = env_int("BARTELS_MG_CLUSTER", kMgClusterMax, 0, kMgClusterMax);
   mg->cl = MgClArgs();
+  if (want == 0) return BARTELS_OK;
+  want = std::max(want, 4);
   BT_CUDA(cudaFuncSetAttribute(k_mgc_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   BT_CUDA(cudaFuncSetAttribute(k_mgc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  for (int first = std::max(1, L - kMgClusterLevels); first < L; ++first) {
-    MgClArgs a;
-    a.first = first;
-    a.nlev = L - first;
-    a.last_mode = mg->dense ? kMgLastDense : (mg->coarse_blockdiag ? kMgLastExact : kMgLastCheb);
-    a.nd = mg->nd;
-    a.ainv = mg->ainv;
-    a.coef = mg->coef;
-    a.ctas = want;
-    for (int l = 0; l < a.nlev; ++l) {
-      const HostLevel &h = H[first + l];
-      MgClLevel &c = a.lv[l];
-      cluster_split(h, mg->dense && l + 1 == a.nlev, a.ctas, c.split);
-      for (int q = 0; q <= a.ctas; ++q) {
-        c.bsplit[q] = h.rp[c.split[q]];
-        c.msplit[q] = l > 0 ? H[first + l - 1].mptr[c.split[q]] : 0;
+  for (int ctas : {want, 8, 4}) {
+    if (ctas > want) continue;
+    for (int first = std::max(1, L - kMgClusterLevels); first < L; ++first) {
+      MgClArgs a;
+      a.first = first;
+      a.nlev = L - first;
+      a.last_mode = mg->dense ? kMgLastDense : (mg->coarse_blockdiag ? kMgLastExact : kMgLastCheb);
+      a.nd = mg->nd;
+      a.ainv = mg->ainv;
+      a.coef = mg->coef;
+      a.ctas = ctas;
+      for (int l = 0; l < a.nlev; ++l) {
+        const HostLevel &h = H[first + l];
+        MgClLevel &c = a.lv[l];
+        cluster_split(h, mg->dense && l + 1 == a.nlev, a.ctas, c.split);
+        for (int q = 0; q <= a.ctas; ++q) {
+          c.bsplit[q] = h.rp[c.split[q]];
+          c.msplit[q] = l > 0 ? H[first + l - 1].mptr[c.split[q]] : 0;
+        }
       }
-    }
-    const int64_t smem = cluster_layout(a);
-    if (smem > kSmem) continue;
-    a.smem = (int)smem;
-    cudaLaunchAttribute at[1];
-    const cudaLaunchConfig_t cfg = cluster_config(ctx, a.ctas, kClThreads, a.smem, at);
-    int fit = 0;
-    BT_CUDA(cudaOccupancyMaxActiveClusters(&fit, k_mgc_cluster, &cfg));
-    if (fit < 1) return fail(BARTELS_E_UNSUPPORTED, "multigrid: the device cannot host the coarse-cycle cluster");
-    for (int l = 0; l < a.nlev; ++l) {
-      const MgLevel &d = mg->lv[first + l];
-      MgClLevel &c = a.lv[l];
-      c.deg = d.deg;
-      c.rp = d.rp;
-      c.ci = d.ci;
-      c.agg = d.agg;
-      c.val16 = d.val16;
-      c.dinv = d.dinv;
-      c.Q = d.Q;
-      c.gb = d.b;
-      c.gx = d.x;
-      c.gd = d.d;
-      c.gd2 = d.d2;
-      c.gres = l + 1 < a.nlev ? d.x2 : d.x;  // as level_result
-      if (l > 0) {
-        c.mptr = mg->lv[first + l - 1].mptr;
-        c.midx = mg->lv[first + l - 1].midx;
+      const int64_t smem = cluster_layout(a);
+      if (smem > kSmem) continue;
+      a.smem = (int)smem;
+      cudaLaunchAttribute at[1];
+      const cudaLaunchConfig_t cfg = cluster_config(ctx, a.ctas, kClThreads, a.smem, at);
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, k_mgc_cluster, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        fit = 0;
       }
+      if (fit < 1) continue;
+      for (int l = 0; l < a.nlev; ++l) {
+        const MgLevel &d = mg->lv[first + l];
+        MgClLevel &c = a.lv[l];
+        c.deg = d.deg;
+        c.rp = d.rp;
+        c.ci = d.ci;
+        c.agg = d.agg;
+        c.val16 = d.val16;
+        c.dinv = d.dinv;
+        c.Q = d.Q;
+        c.gb = d.b;
+        c.gx = d.x;
+        c.gd = d.d;
+        c.gd2 = d.d2;
+        c.gres = l + 1 < a.nlev ? d.x2 : d.x;  // as level_result
+        if (l > 0) {
+          c.mptr = mg->lv[first + l - 1].mptr;
+          c.midx = mg->lv[first + l - 1].midx;
+        }
+      }
+      mg->cl = a;
+      return BARTELS_OK;
     }
-    mg->cl = a;
-    return BARTELS_OK;
   }
-  if (mg->dense) return fail(BARTELS_E_DEVICE, "multigrid: the dense level does not fit the cluster");
   return BARTELS_OK;
 }
 
@@ -1444,6 +1452,21 @@ k_mgc_MA(int n, const int *__restrict__ rp, const int *__restrict__ ci, const __
   BT_CROW_LOOP_END
 }
 
+// coarsest level, dense, outside the cluster launch: x = Ainv b, a warp per row
+__global__ void __launch_bounds__(256)
+k_mg_dense_apply(int nd, const float *__restrict__ ainv, const float *__restrict__ b, float *__restrict__ x,
+                 const PcgState *__restrict__ st) {
+  pdl_wait();
+  pdl_trigger();
+  if (st && st->done) return;
+  const int lane = threadIdx.x & 31, i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= nd) return;
+  float s = 0.f;
+  for (int j = lane; j < nd; j += 32) s += __ldg(ainv + (int64_t)i * nd + j) * __ldcg(b + j);
+  s = warp_sumf(s);
+  if (lane == 0) x[i] = s;
+}
+
 // ==================================== coarse levels in one cluster launch ===
 // The coarse part of the V-cycle (every level from cl.first down to the
 // coarsest and back) as one kernel of one thread-block cluster. Each CTA owns
@@ -1866,7 +1889,8 @@ int restrict_into(bartels_ctx ctx, MgHierarchy *mg, const MgLevel &f, const floa
                   bool *first_done) {
   MgLevel &c = mg->lv[l];
   const bool last = l + 1 == (int)mg->lv.size();
-  const bool fuse = !(mg->cl.ctas && l == mg->cl.first);  // the cluster kernel takes the first step itself
+  // the cluster kernel takes the first step itself
+  const bool fuse = !(mg->cl.ctas && l == mg->cl.first) && !(last && mg->dense);
   const bool exact = last && mg->coarse_blockdiag;  // x = Dinv b
   const float *coef = exact ? nullptr : mg->coef + kMgCoef * l;
   const float *dinv = fuse ? (const float *)c.dinv : nullptr;
@@ -1905,8 +1929,9 @@ int enqueue_coarse(bartels_ctx ctx, MgHierarchy *mg, int l, bool first_done, con
   const float *coef = mg->coef + kMgCoef * l;
   const int last = (int)mg->lv.size() - 1;
   if (l == last) {
-    // (a dense coarsest level is always part of the cluster launch)
-    if (mg->coarse_blockdiag) {
+    if (mg->dense) {
+      BT_LAUNCH_PDL(ctx, k_mg_dense_apply, (mg->nd + 7) / 8, 256, 0, mg->nd, mg->ainv, c.b, c.x, st);
+    } else if (mg->coarse_blockdiag) {
       if (!first_done)
         BT_LAUNCH_PDL(ctx, k_mgc_first, grid_n(ctx, c.n), 256, 0, c.n, c.dinv, c.b, c.x, (float *)nullptr,
                   (float *)nullptr, (const float *)nullptr, st);
