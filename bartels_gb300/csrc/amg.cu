@@ -807,7 +807,9 @@ struct MgInvArgs {
   const float *val = nullptr;
   float *panel = nullptr, *ainv = nullptr;
 };
-constexpr int kInvThreads = 512;
+constexpr int kInvThreads = 512, kInvCtas = 8;
+// own rows and the panel of the largest dense level
+constexpr int kInvSmem = (int)sizeof(float) * (6 * ((kDenseNodes + kInvCtas - 1) / kInvCtas) + 6) * 6 * kDenseNodes;
 __global__ void __launch_bounds__(kInvThreads, 1)
 k_mg_dense_inv(const __grid_constant__ MgInvArgs a) {
   extern __shared__ __align__(16) float sA[];  // own rows (6 x own nodes) x nd, then the panel 6 x nd
@@ -2062,10 +2064,11 @@ int mg_setup_numeric(bartels_ctx ctx, bartels_mesh_plan plan, const float *value
     ia.val = c.val;
     ia.panel = mg->panel;
     ia.ainv = mg->ainv;
-    const int ctas = std::min(c.n, 8), per = (c.n + ctas - 1) / ctas;
+    const int ctas = std::min(c.n, kInvCtas), per = (c.n + ctas - 1) / ctas;
     for (int q = 0; q <= kMgClusterMax; ++q) ia.split[q] = std::min(c.n, q * per);
     const int smem = (int)sizeof(float) * (6 * per + 6) * mg->nd;
-    BT_CUDA(cudaFuncSetAttribute(k_mg_dense_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the same value from every thread: a smaller one would take another context's launch its memory
+    BT_CUDA(cudaFuncSetAttribute(k_mg_dense_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem));
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = cluster_config(ctx, ctas, kInvThreads, smem, at);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mg_dense_inv, ia);

@@ -1086,8 +1086,8 @@ static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *
                          float cM, float tol, int corot_exact, float *values) {
   const bool small = plan->hess_chunk == 64;
   const int smem = (small ? kSmallFloats : kChunkFloats) * (int)sizeof(float);
-  static bool attr_set = false;  // per template instance
-  if (!attr_set) {
+  static DeviceOnce attrs;  // per template instance
+  if (attrs.pending(ctx->device)) {
     BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kChunkFloats * (int)sizeof(float)));
     BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1095,7 +1095,7 @@ static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *
     if constexpr (hess_cheap(MODEL, PSD))
       BT_CUDA(cudaFuncSetAttribute(k_hess<MODEL, PSD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kChunkFloats * (int)sizeof(float)));
-    attr_set = true;
+    attrs.set(ctx->device);
   }
   const int pb = plan->psd_block;
   float4 *fslot = nullptr;

@@ -188,10 +188,10 @@ static int make_map(CUtensorMap *m, const __nv_bfloat16 *p, int rows, int cols, 
 template <int N, int K>
 static int launch_gemm_t(bartels_ctx ctx, const GemmArgs &g) {
   using S = GemmSmem<N, K>;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attrs;
+  if (attrs.pending(ctx->device)) {
     BT_CUDA(cudaFuncSetAttribute(k_gemm_tc<N, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDyn));
-    attr = true;
+    attrs.set(ctx->device);
   }
   CUtensorMap mx, mw;
   BT_CHECK(make_map(&mx, g.x, g.M, K, g.ldx, 128));

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "bartels_gpu.h"
+#include "device_once.h"
 
 namespace bartels {
 

@@ -333,11 +333,11 @@ int pcg_small_fill(bartels_ctx ctx, PcgSmall &s, char *base, const std::vector<i
 
 int pcg_small_run(bartels_ctx ctx, const PcgSmall &s, const float *rres, const float *minv, float *x, float *p,
                   PcgState *st, double inner_rel2, double abs_tol2, int max_it, int cont) {
-  static bool attr_set = false;
-  if (!attr_set) {
+  static DeviceOnce attrs;
+  if (attrs.pending(ctx->device)) {
     BT_CUDA(cudaFuncSetAttribute(k_pcg_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     BT_CUDA(cudaFuncSetAttribute(k_pcg_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    attr_set = true;
+    attrs.set(ctx->device);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kCtas);
