@@ -138,6 +138,8 @@ int bartels_ctx_create(int device, bartels_ctx *out) {
     const int g = std::atoi(e);
     if (g == 4 || g == 8) ctx->tri_lanes = g;
   }
+  if (const char *e = std::getenv("BARTELS_PCG_SMALL"))
+    if (e[0] == '0') ctx->small_hosted = 0;
   *out = ctx;
   return BARTELS_OK;
 }

@@ -167,6 +167,8 @@ struct bartels_ctx_s {
   int spmv_lanes = 8;
   // lanes per vertex row in the triangular factor passes (4 or 8; BARTELS_TRI_LANES)
   int tri_lanes = 4;
+  // whether the device can host the small solves' cluster (-1: not asked yet; BARTELS_PCG_SMALL=0: no)
+  int small_hosted = -1;
   // autotuner results per size bucket (floor(log2 nV)): {SpMV lanes, factor-pass lanes}
   std::map<int, std::pair<int, int>> tune_cache;
   // Hessian autotuner results per size bucket: {vertices per assembly CTA, PSD block size}

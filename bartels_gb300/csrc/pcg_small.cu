@@ -331,26 +331,42 @@ int pcg_small_fill(bartels_ctx ctx, PcgSmall &s, char *base, const std::vector<i
   return BARTELS_OK;
 }
 
-int pcg_small_run(bartels_ctx ctx, const PcgSmall &s, const float *rres, const float *minv, float *x, float *p,
-                  PcgState *st, double inner_rel2, double abs_tol2, int max_it, int cont) {
-  static DeviceOnce attrs;
-  if (attrs.pending(ctx->device)) {
-    BT_CUDA(cudaFuncSetAttribute(k_pcg_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    BT_CUDA(cudaFuncSetAttribute(k_pcg_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    attrs.set(ctx->device);
-  }
+// launch configuration of one solve's cluster
+static cudaLaunchConfig_t small_config(bartels_ctx ctx, int threads, int smem, cudaLaunchAttribute *at) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kCtas);
-  // a warp per group of the CTA's rows: barriers cost less with fewer threads
-  cfg.blockDim = dim3(std::min(kMaxThreads, std::max(256, s.rows)));
-  cfg.dynamicSmemBytes = s.smem;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = kCtas;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  return cfg;
+}
+
+bool pcg_small_hosted(bartels_ctx ctx) {
+  if (ctx->small_hosted < 0) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = small_config(ctx, kMaxThreads, kSmemBytes, at);
+    int fit = 0;
+    const bool ok = cudaFuncSetAttribute(k_pcg_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) ==
+                        cudaSuccess &&
+                    cudaFuncSetAttribute(k_pcg_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                        cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&fit, k_pcg_small, &cfg) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    ctx->small_hosted = ok && fit >= 1;
+  }
+  return ctx->small_hosted != 0;
+}
+
+int pcg_small_run(bartels_ctx ctx, const PcgSmall &s, const float *rres, const float *minv, float *x, float *p,
+                  PcgState *st, double inner_rel2, double abs_tol2, int max_it, int cont) {
+  cudaLaunchAttribute at[1];
+  // a warp per group of the CTA's rows: barriers cost less with fewer threads
+  const cudaLaunchConfig_t cfg = small_config(ctx, std::min(kMaxThreads, std::max(256, s.rows)), s.smem, at);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, k_pcg_small, s, rres, minv, x, p, st, inner_rel2, abs_tol2, max_it, cont);
   ctx->launches++;
   if (e != cudaSuccess) return fail(BARTELS_E_DEVICE, std::string("launch k_pcg_small: ") + cudaGetErrorString(e));

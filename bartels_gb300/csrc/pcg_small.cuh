@@ -17,6 +17,9 @@ struct PcgSmall {
   unsigned short *col = nullptr;
 };
 
+// Whether the context's device can host the cluster (asked once per context, which
+// also sets the kernel's attributes there; BARTELS_PCG_SMALL=0: no). Before pcg_small_run.
+bool pcg_small_hosted(bartels_ctx ctx);
 // Whether the system (row lengths len(i), i < n) runs as a cluster launch; fills
 // the sizes and the group offsets (host).
 bool pcg_small_plan(int n, const int *row_ptr, PcgSmall &s, std::vector<int> &off);

@@ -999,7 +999,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
       small_rp[i + 1] = small_rp[i] + 3 * (op.plan->h_brp[i / 3 + 1] - op.plan->h_brp[i / 3]);
     h_rp = small_rp.data();
   }
-  bool is_small = !op.mg && !op.gl && h_rp && pcg_small_plan(n, h_rp, small, small_off);
+  bool is_small = !op.mg && !op.gl && h_rp && pcg_small_plan(n, h_rp, small, small_off) && pcg_small_hosted(ctx);
   const size_t o_small = take(is_small ? pcg_small_bytes(small) : 0);
   BT_CHECK(wbuf.ensure(off));
   char *base = wbuf.as<char>();

@@ -1,0 +1,59 @@
+"""Where the small solve's cluster cannot or must not be used: a device that cannot
+host it; and what its size leaves empty (CTAs without rows, pinned vertices)."""
+import numpy as np
+import pytest
+
+from test_gpu_pcg_small import REL, _spd
+
+pytestmark = pytest.mark.gpu
+
+
+def _direction(A, g, **kw):
+    import bartels_gb300 as bg
+    d, ok, rep = bg.search_direction_newton_sparse(g, A, rel_tol=REL, **kw)
+    assert ok and rep.converged
+    assert np.linalg.norm(-g - A @ d) <= 1.001 * REL * np.linalg.norm(g)
+    return d, rep
+
+
+@pytest.fixture
+def general(monkeypatch):
+    """A default context on which the cluster counts as not hosted."""
+    from bartels_gb300.api import Context
+    monkeypatch.setenv("BARTELS_PCG_SMALL", "0")
+    ctx = Context(0)
+    monkeypatch.setattr(Context, "_default", ctx)
+    yield ctx
+    ctx.close()
+
+
+@pytest.mark.parametrize("n,band,hub", [(1, 0, False), (4, 2, False), (1537, 9, True), (10080, 40, False)])
+def test_the_general_loop_takes_over(n, band, hub, general):
+    A = _spd(n, band, n, hub)
+    before = general.kernel_launches
+    _, rep = _direction(A, np.random.default_rng(n + 1).standard_normal(n))
+    assert general.kernel_launches - before >= 3 * rep.iterations
+
+
+def test_ctas_without_rows_many_times():
+    """Up to 96 unknowns belong to the first CTA: the other fifteen only take part in the sums."""
+    for n in (1, 3, 31, 96, 97):
+        A = _spd(n, 4 if n > 1 else 0, n)
+        g = np.random.default_rng(n).standard_normal(n)
+        d0, rep0 = _direction(A, g)
+        for _ in range(50):
+            d, rep = _direction(A, g)
+            assert np.array_equal(d, d0) and rep.iterations == rep0.iterations
+
+
+@pytest.mark.parametrize("n", [1, 3, 13])
+def test_pinned_plan(n):
+    from test_gpu_multigrid import SOL_TOL, _cube, _direct, _hessian, _rhs, _solve
+    plan, V, q, pinned = _cube(n)
+    vals = _hessian(plan, q)
+    b = _rhs(len(V), pinned)
+    x, rep = _solve(plan, vals, b, "jacobi")
+    ref = _direct(plan, vals, b, pinned)
+    assert rep.converged and np.all(x[np.repeat(pinned, 3)] == 0.0)
+    assert np.linalg.norm(x - ref) <= SOL_TOL * np.linalg.norm(ref)
+    plan.close()
