@@ -92,9 +92,13 @@ __device__ __forceinline__ void small_barrier() {
   small_wait();
 }
 
-// Sums across warps and CTAs are unevaluated float pairs h + l (two-sum): exact to
-// ~2^-48, far below the FP32 rounding of the threads' partials, at a fraction of
-// the latency of this GPU's FP64 adds (a tree of nine took ~2,500 cycles).
+// Sums across warps and CTAs are unevaluated float pairs h + l (Knuth's two-sum,
+// with the low parts added up): off by ~2^-46 of the sum, or by the spacing of the
+// smallest floats (1.4e-45 a step), where the FP32 partials that they add are off by
+// 2^-24; at a fraction of the latency of this GPU's FP64 adds (a tree of nine took
+// ~2,500 cycles). That holds while the sums stay well inside the float range; r.z
+// and p.Ap scale with the matrix too, so the solve watches them: one that leaves the
+// range ends as kSmallRange, for the general loop, whose sums are FP64.
 __device__ __forceinline__ float2 pair_add(float2 a, float2 b) {
   const float s = __fadd_rn(a.x, b.x), t = __fsub_rn(s, a.x);
   const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, t)), __fsub_rn(b.x, t));
@@ -112,6 +116,8 @@ __device__ __forceinline__ float2 pair_reduce(float2 v) {
   }
   return v;
 }
+// ~40 steps of 1.4e-45 are below 1e-10 of the sum, and no partial sum overflows; NaN is out
+__device__ __forceinline__ bool small_in_range(float2 a) { return fabsf(a.x) > 1e-33f && fabsf(a.x) < 1e36f; }
 __device__ __forceinline__ double pair_value(float2 a) { return (double)a.x + (double)a.y; }
 // a / b rounded to FP32 (one correction of the FP32 quotient)
 __device__ __forceinline__ float pair_div(float2 a, float2 b) {
@@ -248,7 +254,7 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
     if (lane == 0) {
       s_alpha = 0.f;
       s_beta = (rz_old > 0.0 && rz_old < HUGE_VAL) ? (float)(pair_value(rz) / rz_old) : 0.f;
-      s_done = rr <= tol2 || max_it <= 0 || !(rr == rr);
+      s_done = rr <= tol2 || max_it <= 0 ? 1 : small_in_range(d2[0]) && small_in_range(d2[1]) ? 0 : kSmallRange;
     }
   }
   __syncthreads();
@@ -286,7 +292,10 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
     small_reduce<1>(acc, 0.f, s_warps, s_pap, rank, d1);
     if (warp == 0) {
       pap = d1[0];
-      if (lane == 0) s_alpha = pair_div(rz, pap);
+      if (lane == 0) {
+        s_alpha = pair_div(rz, pap);
+        if (!small_in_range(pap)) s_done = kSmallRange;
+      }
     }
     __syncthreads();
     update(s_alpha, arz, arr);
@@ -296,7 +305,8 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
       rr = pair_value(d2[1]);
       if (lane == 0) {
         s_beta = pair_div(d2[0], rz);
-        s_done = rr <= tol2 || it >= last || !(rr == rr);
+        if (!s_done)
+          s_done = rr <= tol2 || it >= last ? 1 : small_in_range(d2[0]) && small_in_range(d2[1]) ? 0 : kSmallRange;
       }
       rz = d2[0];
     }
@@ -314,7 +324,7 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
     st->beta = beta;
     st->it = it;
     st->max_it = last;
-    st->done = 1;
+    st->done = s_done;
   }
 }
 

@@ -28,7 +28,10 @@ size_t pcg_small_bytes(const PcgSmall &s);
 // them. rp / ci / val: device; rows of pinned vertices (3 rows each) become empty.
 int pcg_small_fill(bartels_ctx ctx, PcgSmall &s, char *base, const std::vector<int> &off, const int *rp, const int *ci,
                    const float *val, const unsigned char *pinned);
-// One inner solve: as k_pcg_init followed by the PCG loop until the state is done.
+// One inner solve: as k_pcg_init followed by the PCG loop until the state is done
+// (done = 1), or until one of its sums leaves the range of float pairs (done =
+// kSmallRange): the iterate is then of no use and the general loop has to take over.
+enum { kSmallRange = 2 };
 int pcg_small_run(bartels_ctx ctx, const PcgSmall &s, const float *rres, const float *minv, float *x, float *p,
                   PcgState *st, double inner_rel2, double abs_tol2, int max_it, int cont);
 

@@ -1043,13 +1043,18 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     return rep->converged ? BARTELS_OK : fail(BARTELS_E_NONFINITE, "non-finite right-hand side");
   }
   const double target = prm.rel_tol * bnorm;
-  // its sums are float pairs: keep the squares well inside the float range
-  is_small = is_small && bnorm < 1e12 && bnorm > 1e-9 && target > 1e-18;
+  // its sums are float pairs: keep the squares well inside the float range, down to (target / 2)^2
+  is_small = is_small && bnorm < 1e12 && bnorm > 1e-9 && target > 1e-16;
   // CUDA graph of a fixed number of PCG iterations (kernels no-op once done)
   const int chunk = op.mg ? 8 : 16;  // fixed-length fallback only
   cudaGraphExec_t exec = nullptr;
   int64_t graph_launches = 0;
   bool device_loop = false;
+  auto build_loop = [&]() {
+    return build_loop_graph(
+        ctx, w.st, [&](int k) { return pcg_enqueue_iters(ctx, op, w, n, nb, k); }, op.mg ? 1 : 4, chunk, &exec,
+        &graph_launches, &device_loop);
+  };
   if (is_small) {
     const int *rp = op.rp, *ci = op.ci;
     if (blk) {
@@ -1059,9 +1064,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     }
     BT_CHECK(pcg_small_fill(ctx, small, base + o_small, small_off, rp, ci, op.values, op.pinned));
   } else {
-    BT_CHECK(build_loop_graph(
-        ctx, w.st, [&](int k) { return pcg_enqueue_iters(ctx, op, w, n, nb, k); }, op.mg ? 1 : 4, chunk, &exec, &graph_launches,
-        &device_loop));
+    BT_CHECK(build_loop());
   }
   int status = BARTELS_OK;
   double rel = 0.0;
@@ -1100,13 +1103,22 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
     // inner FP32 PCG on rres: a fresh solve in the first pass, later passes
     // continue the direction against the replaced residual unless restart is set
     const double abs2 = (0.5 * target) * (0.5 * target);
-    const int cont = (pass > 0 && !prm.restart) ? 1 : 0;
-    const int it0 = cont ? hs.it : 0;
+    int cont = (pass > 0 && !prm.restart) ? 1 : 0;
+    int it0 = cont ? hs.it : 0;
     if (is_small) {
       BT_CHECK(pcg_small_run(ctx, small, w.rres, w.minv, w.x, w.pa, w.st, prm.inner_rel_tol * prm.inner_rel_tol, abs2,
                              prm.max_iters - rep->iterations, cont));
       BT_CUDA(cudaMemcpyAsync(&hs, w.st, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx->stream));
       BT_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (hs.done == kSmallRange) {
+        // this pass again as a fresh solve of the general loop, and every later one
+        is_small = false;
+        BT_CHECK(build_loop());
+        cont = it0 = 0;
+      }
+    }
+    if (is_small) {
+      // done
     } else if (op.mg) {
       BT_LAUNCH_PDL(ctx, k_pcg_init_f, gv, 256, 0, n, w.rres, w.x, w.r, w.pa, w.pb, w.part_a, w.st,
                 prm.inner_rel_tol * prm.inner_rel_tol, abs2, prm.max_iters - rep->iterations, cont);

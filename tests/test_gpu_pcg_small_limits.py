@@ -1,5 +1,6 @@
 """Where the small solve's cluster cannot or must not be used: a device that cannot
-host it; and what its size leaves empty (CTAs without rows, pinned vertices)."""
+host it, sums that leave the range of its float pairs; and what its size leaves
+empty (CTAs without rows, pinned vertices)."""
 import numpy as np
 import pytest
 
@@ -57,3 +58,12 @@ def test_pinned_plan(n):
     assert rep.converged and np.all(x[np.repeat(pinned, 3)] == 0.0)
     assert np.linalg.norm(x - ref) <= SOL_TOL * np.linalg.norm(ref)
     plan.close()
+
+
+# r.z and p.Ap scale with 1 / A and A where b alone is of ordinary size: sums past the largest float while
+# every term fits, sums within the range at either side, and a matrix of ordinary size
+@pytest.mark.parametrize("n,a,b", [(10080, 1e-36, 10.0), (24576, 1e-36, 3.0), (10080, 1e-30, 1.0), (10080, 1e15, 1.0),
+                                   (3001, 1.0, 1e-4)])
+def test_matrices_far_from_unit_scale(n, a, b):
+    A = a * _spd(n, 20, n)
+    _direction(A, b * np.random.default_rng(n).standard_normal(n))
