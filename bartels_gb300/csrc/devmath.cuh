@@ -919,7 +919,9 @@ BT_HD T psi_model_disp(int model, const T *H, const T *pv) {
       return pv[0] * (d.nrm2 - T(2) * (d.q2 + d.det) + T(2) * g2) + pv[1] * d.j * d.j;
     // J^-2/3 I1 - 3 = 3 g1 + 2 g2 - 2 (q2 + det) + |H|^2 + e (2 tr H + |H|^2),
     // e = J^-2/3 - 1 = expm1(y), y = -2/3 ln J, g1 = expm1(y) - y
-    const T y = T(-2) / T(3) * (d.j - g2);
+    // ln J = j - g2 within the table of g2; beyond it the difference would cost J / ln J roundings
+    const T L = bt_abs(d.j) < T(0.6875) ? d.j - g2 : bt_log1p(d.j);
+    const T y = T(-2) / T(3) * L;
     const T g1 = expm1_minus_y(y);
     const T e = g1 + y;
     return pv[0] * (T(3) * g1 + T(2) * g2 - T(2) * (d.q2 + d.det) + d.nrm2 + e * (T(2) * d.tr + d.nrm2)) +
