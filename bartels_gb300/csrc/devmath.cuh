@@ -1250,19 +1250,23 @@ BT_HD_NOINLINE void psd_eig_K(const Law &law, const T (*phi)[3], T tol, T *K) {
             M[p9(k + 3 * c, l + 3 * d)] = acc;
           }
   }
-  // scale by a power of two to entries of order one (exact)
+  // scale by a power of two to entries of order one (exact), or as far as the power is a number
   T big = T(0);
 #pragma unroll
   for (int i = 0; i < 45; ++i) big = bt_max(big, bt_abs(M[i]));
-  const int ex = (big > T(0) && big < T(1e30)) ? bt_ilogb(big) : 0;
+  constexpr int lowest = sizeof(T) == 4 ? -126 : -1022;
+  constexpr T most = T(sizeof(T) == 4 ? 3.4e38 : 1e300);
+  const int e2 = (big > T(0) && big <= most) ? bt_ilogb(big) : 0, ex = e2 < lowest ? lowest : e2;
   const T up = bt_scalbn(T(1), -ex), down = bt_scalbn(T(1), ex);
 #pragma unroll
   for (int i = 0; i < 45; ++i) M[i] *= up;
   T W[81], lam[9];
   eig9p(M, lam, W);
-  const T floor_ = tol * up;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) lam[i] = (lam[i] < floor_ ? floor_ : lam[i]) * down;
+  for (int i = 0; i < 9; ++i) {  // against tol itself: tol * up need not be finite
+    const T l = lam[i] * down;
+    lam[i] = l < tol ? tol : l;
+  }
   // Y = (Q (x) I) W for nodes 1 .. 3, in place
 #pragma unroll
   for (int e = 0; e < 9; ++e)
