@@ -7,6 +7,7 @@
 #include <string>
 
 #include "devmath.cuh"
+#include "hess_shape.h"
 #include "internal.cuh"
 
 namespace bartels {
@@ -726,7 +727,7 @@ constexpr bool hess_cheap(int model, bool psd) {
 // warps per SM, 78% of the pipe), two lanes 720 us, four 940 (the adds are issued
 // once per lane of the group); 1.05M tets with projection 375 / 270 / 300.
 // 18-KB chunks of 32 vertices: 757 us per call, 789 with 64 vertices, 871 with
-// 128. launch_hess_t chooses the lanes.
+// 128. hess_shape chooses the lanes.
 template <int MODEL, bool PSD, int G>
 __global__ void __launch_bounds__(kChunkMaxVerts * G, 4 / G)
 k_hess(const int *__restrict__ chunk_v, const int *__restrict__ brp, const int *__restrict__ inc_ptr,
@@ -1084,7 +1085,9 @@ int gradient(bartels_ctx ctx, bartels_mesh_plan plan, int model, const Objective
 template <int MODEL, bool PSD>
 static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *u, int add_identity, float cK,
                          float cM, float tol, int corot_exact, float *values) {
-  const bool small = plan->hess_chunk == 64;
+  const HessShape shape =
+      hess_shape(plan->nV, plan->nchunks, ctx->num_sms, hess_cheap(MODEL, PSD), plan->hess_chunk);
+  const bool small = shape.chunk == 64;
   const int smem = (small ? kSmallFloats : kChunkFloats) * (int)sizeof(float);
   static DeviceOnce attrs;  // per template instance
   if (attrs.pending(ctx->device)) {
@@ -1121,23 +1124,13 @@ static int launch_hess_t(bartels_ctx ctx, bartels_mesh_plan plan, const float4 *
   BT_LAUNCH(ctx, (k_hess<MODEL, PSD, G>), chunks, verts * G, smem, chunk_v, plan->brp, plan->inc_ptr,            \
             plan->inc_tet, plan->inc_pos, plan->rec32, u, ul, add_identity, cK, cM, tol, corot_exact, fslot, kbuf, \
             values)
-  // Four lanes while a vertex's pair of lanes would leave most SMs short of work
-  // (15.6k vertices: 31 us, two lanes 38). The cheap laws' one-lane form runs in
-  // one wave of three 128-vertex chunks per SM, so its time hardly grows up to
-  // there; the two-lane form's second wave starts at ~190 vertices per SM on a
-  // mesh numbered without locality. Shuffled balls, one lane / two: 27.6k
-  // vertices 66 / 60 us, 30.1k 67 / 72, 37.5k 67 / 78, 56.2k 94 / 112, 63.4k (a
-  // second wave) 153 / 128; boxes: 35.9k 52 / 43, 50.7k 64 / 69, 59.3k 96 / 72.
-  const int64_t nV = plan->nV, sms = ctx->num_sms;
   if constexpr (hess_cheap(MODEL, PSD)) {
-    if (nV > 190 * sms && plan->nchunks <= 3 * sms) {
-      BT_LAUNCH(ctx, (k_hess<MODEL, PSD, 1>), plan->nchunks, kChunkMaxVerts, kChunkFloats * (int)sizeof(float),
-                plan->chunk_v, plan->brp, plan->inc_ptr, plan->inc_tet, plan->inc_pos, plan->rec32, u, ul,
-                add_identity, cK, cM, tol, corot_exact, fslot, kbuf, values);
+    if (shape.lanes == 1) {
+      BT_HG(1);
       return BARTELS_OK;
     }
   }
-  if (nV <= 128 * sms) BT_HG(4);
+  if (shape.lanes == 4) BT_HG(4);
   else BT_HG(2);
 #undef BT_HG
   return BARTELS_OK;

@@ -214,9 +214,10 @@ struct bartels_mesh_plan_s {
   bartels::SellPattern *sell = nullptr;
   bartels::SellPattern *sell_factor[2] = {nullptr, nullptr};  // the learned factor's lower and upper parts
   int nchunks64 = 0;
-  // Hessian tuning: vertices per assembly CTA (128, or 64 with chunk_v64) and
-  // threads per CTA of the PSD pre-pass kernels (64, 128 or 256)
-  int hess_chunk = 64, psd_block = 128;
+  // Hessian tuning: assembly shape (128 vertices per CTA; 64: the small shape's
+  // kSmallVerts; 0: none, hess_shape decides) and threads per CTA of the PSD
+  // pre-pass kernels (64, 128 or 256)
+  int hess_chunk = 0, psd_block = 128;
   std::vector<int> h_brp, h_bcol, h_chunk_v;  // host copies
   // lazily built scalar CSR pattern (device)
   int *csr_rp = nullptr, *csr_col = nullptr;
