@@ -114,6 +114,7 @@ SIGNATURES = [
     ("bartels_newton_gradient_d", C.c_int, [_P, _P, C.POINTER(NewtonParams), _P, _P]),
     ("bartels_newton_energy_d", C.c_int, [_P, _P, C.POINTER(NewtonParams), _P, _D]),
     ("bartels_newton_get_problem", C.c_int, [_P, _D, _D]),
+    ("bartels_plan_tuning", C.c_int, [_P, _I, _I, _I]),
     ("bartels_plan_autotune", C.c_int, [_P, _P, _P, C.c_int, _I, _I]),
     ("bartels_segment_sumsq_d", C.c_int, [_P, C.c_int, _P, _P, _P]),
     ("bartels_plan_set_segments", C.c_int, [_P, C.c_int, _I, C.POINTER(C.c_int64)]),

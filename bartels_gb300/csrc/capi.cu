@@ -824,6 +824,14 @@ int bartels_plan_mg_info(bartels_mesh_plan plan, int max_levels, int *levels, in
   return BARTELS_OK;
 }
 
+int bartels_plan_tuning(bartels_mesh_plan plan, int *spmv_split, int *spmv_lanes, int *factor_lanes) {
+  if (!plan) return fail(BARTELS_E_INVALID_ARG, "null plan");
+  if (spmv_split) *spmv_split = plan->spmv_split;
+  if (spmv_lanes) *spmv_lanes = plan->spmv_lanes;
+  if (factor_lanes) *factor_lanes = plan->tri_lanes;
+  return BARTELS_OK;
+}
+
 int bartels_plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values_d, int force,
                           int *spmv_lanes, int *factor_lanes) {
   BT_CHECK(check_plan(ctx, plan));

@@ -169,8 +169,11 @@ struct bartels_ctx_s {
   int tri_lanes = 4;
   // whether the device can host the small solves' cluster (-1: not asked yet; BARTELS_PCG_SMALL=0: no)
   int small_hosted = -1;
-  // autotuner results per size bucket (floor(log2 nV)): {SpMV lanes, factor-pass lanes}
-  std::map<int, std::pair<int, int>> tune_cache;
+  // autotuner results per size bucket (floor(log2 nV))
+  struct Lanes {
+    int spmv, tri, split;  // SpMV lanes, factor-pass lanes, warps per slice of the PCG loop's SpMV (0: none)
+  };
+  std::map<int, Lanes> tune_cache;
   // Hessian autotuner results per size bucket: {vertices per assembly CTA, PSD block size}
   std::map<int, std::pair<int, int>> tune_cache_hess;
   // pinned host staging for small read-backs
@@ -232,8 +235,9 @@ struct bartels_mesh_plan_s {
   bartels::FactorPattern *factor = nullptr;
   bartels::LpcgPlanState *lpcg = nullptr;
   int precond = BARTELS_PRECOND_BLOCK_JACOBI;
-  // lanes per vertex row chosen by the autotuner for this plan (0: the context's)
-  int spmv_lanes = 0, tri_lanes = 0;
+  // lanes per vertex row chosen by the autotuner for this plan (0: the context's), and
+  // warps per slice of the PCG loop's SpMV over the sliced-ELL copy (0: sell_split's)
+  int spmv_lanes = 0, tri_lanes = 0, spmv_split = 0;
   bartels_lpcg lpcg_net = nullptr;
   // aggregation multigrid hierarchy (built on first use for the current pinned set)
   bartels::MgHierarchy *mg = nullptr;

@@ -820,7 +820,8 @@ static int pcg_spmv_blk(bartels_ctx ctx, const PcgOperator &op, const PcgWork &w
   const bartels_mesh_plan plan = op.plan;
   if (op.vsell) {
     const SellView sv = plan->sell->view();
-    const int S = sell_split(ctx, sv.nslices), g = sell_grid(ctx, sv.nslices, S);
+    const int S = plan->spmv_split ? plan->spmv_split : sell_split(ctx, sv.nslices);
+    const int g = sell_grid(ctx, sv.nslices, S);
     if (S == 1)
       BT_LAUNCH_PDL(ctx, k_pcg_spmv_sell<1>, g, 256, 0, sv, op.vsell, w.pa, w.pb, w.ap, op.pinned, w.part_a, w.st);
     else if (S == 2)
@@ -2220,8 +2221,9 @@ int plan_set_hessian_tuning(bartels_mesh_plan plan, int chunk, int block) {
   return BARTELS_OK;
 }
 
-// Autotuner: time the block-row SpMV over the values' own layout with 4, 8 and 16
-// lanes per vertex row and the factor passes with 4 and 8 lanes on this plan (CUDA
+// Autotuner: time the PCG loop's SpMV over the sliced-ELL copy with 1, 2 and 4 warps
+// per slice, the block-row SpMV over the values' own layout with 4, 8 and 16 lanes
+// per vertex row and the factor passes with 4 and 8 lanes on this plan (CUDA
 // events on the context's stream, 3 warm-up + 10 timed launches each, best of
 // three rounds over the candidates), keep the fastest in
 // the plan and in the context's cache for the plan's size bucket
@@ -2232,8 +2234,9 @@ int plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, 
   for (int v = plan->nV; v > 1; v >>= 1) bucket++;
   auto hit = ctx->tune_cache.find(bucket);
   if (!force && hit != ctx->tune_cache.end()) {
-    plan->spmv_lanes = hit->second.first;
-    plan->tri_lanes = hit->second.second;
+    plan->spmv_lanes = hit->second.spmv;
+    plan->tri_lanes = hit->second.tri;
+    plan->spmv_split = hit->second.split;
   } else {
     FactorPattern *fp;
     BT_CHECK(plan_factor_pattern(plan, &fp));
@@ -2295,6 +2298,37 @@ int plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, 
       });
       t_s[ci] = std::min(t_s[ci], ms);
     }
+    // the solves' own SpMV, where they make the copy that it reads
+    PcgOperator op;
+    op.plan = plan;
+    op.values = values;
+    op.pinned = plan->pinned;
+    status = plan_sell_values(ctx, plan, values, &op.vsell);
+    int best_split = 0;
+    if (op.vsell && status == BARTELS_OK) {
+      PcgWork w{};
+      w.pa = w.pb = x;
+      w.ap = y;
+      w.part_a = part;
+      w.st = st;
+      float t_split[3] = {1e30f, 1e30f, 1e30f}, b = 1e30f;
+      const int cand[3] = {1, 2, 4};
+      for (int round = 0; round < kRounds; ++round)
+        for (int ci = 0; ci < 3; ++ci) {
+          plan->spmv_split = cand[ci];
+          t_split[ci] = std::min(t_split[ci], timed([&] {
+                                   if (status == BARTELS_OK) status = pcg_spmv_blk(ctx, op, w);
+                                 }));
+        }
+      for (int ci = 0; ci < 3; ++ci)
+        if (t_split[ci] < b) b = t_split[ci], best_split = cand[ci];
+    }
+    plan->spmv_split = 0;
+    if (status != BARTELS_OK) {
+      cudaStreamSynchronize(ctx->stream);
+      cleanup();
+      return status;
+    }
     const int cand_t[2] = {4, 8};
     for (int round = 0; round < kRounds; ++round)
     for (int ci = 0; ci < 2; ++ci) {
@@ -2321,10 +2355,11 @@ int plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values, 
     cleanup();
     if (e != cudaSuccess) status = fail(BARTELS_E_DEVICE, std::string("autotuner: ") + cudaGetErrorString(e));
     if (status != BARTELS_OK) return status;
-    ctx->launches += 39 * kRounds;
+    ctx->launches += 65 * kRounds;  // 3 + 2 candidates, 13 launches each (pcg_spmv_blk counts its own)
     plan->spmv_lanes = best_s;
     plan->tri_lanes = best_t;
-    ctx->tune_cache[bucket] = {best_s, best_t};
+    plan->spmv_split = best_split;
+    ctx->tune_cache[bucket] = {best_s, best_t, best_split};
   }
   if (spmv_out) *spmv_out = plan->spmv_lanes;
   if (tri_out) *tri_out = plan->tri_lanes;

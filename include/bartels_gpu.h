@@ -463,13 +463,20 @@ int bartels_plan_precond_apply_d(bartels_ctx ctx, bartels_mesh_plan plan, const 
 int bartels_plan_pcg_d(bartels_ctx ctx, bartels_mesh_plan plan, const float *values_d, const double *b_d,
                        double *x_d, const bartels_pcg_params *params, bartels_pcg_report *report);
 /* ---------------------------------------------------------------- batching -- */
-/* Autotuner: times the PCG loop's block-row SpMV (4, 8, 16 lanes per vertex row) and the
- * factor passes (4, 8 lanes) on this plan's Hessian (values_d, or NULL for the
- * plan's internal buffer) and keeps the fastest for the plan's PCG solves. The
- * choice is cached in the context per size bucket floor(log2 nV) and reused by
- * later plans of that bucket unless force != 0. No counterpart in the reference. */
+/* Autotuner: times, on this plan's Hessian (values_d, or NULL for the plan's
+ * internal buffer), the PCG loop's SpMV over the sliced-ELL copy of the values (1,
+ * 2, 4 warps per slice), the block-row SpMV over the values' own layout (4, 8, 16
+ * lanes per vertex row: bartels_plan_spmv_d, and the solves under
+ * BARTELS_PCG_PADDED=0) and the factor passes (4, 8 lanes), and keeps the fastest of
+ * each for the plan. The choice is cached in the context per size bucket
+ * floor(log2 nV) and reused by later plans of that bucket unless force != 0. No
+ * counterpart in the reference. */
 int bartels_plan_autotune(bartels_ctx ctx, bartels_mesh_plan plan, const float *values_d, int force,
                           int *spmv_lanes, int *factor_lanes);
+/* The plan's tuned launch shapes, 0 where it has none (the library's rule, or the
+ * context's lanes): warps per slice of the PCG loop's SpMV, lanes of the block-row
+ * SpMV and of the factor passes. Any pointer may be NULL. */
+int bartels_plan_tuning(bartels_mesh_plan plan, int *spmv_split, int *spmv_lanes, int *factor_lanes);
 /* The PCG loop's SpMV kernel, y_d = A x_d with A the FP32 values_d (NULL:
  * the plan's last assembled Hessian), timed: 3 warm-up launches, then reps
  * launches between CUDA events on the context's stream; *us_per_launch gets
