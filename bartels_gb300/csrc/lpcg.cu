@@ -1172,7 +1172,7 @@ static int lp_state(bartels_mesh_plan plan, bool train, int nprobe, LpcgPlanStat
     BT_CHECK(lp_alloc(*s, &s->uprobe, (size_t)nprobe * 3 * nV));
     BT_CHECK(lp_alloc(*s, &s->vprobe, (size_t)nprobe * 3 * nV));
   }
-  *out = s;
+  *out = plan->lpcg = own.release();  // the plan's once it is complete
   return BARTELS_OK;
 }
 
