@@ -790,6 +790,7 @@ __device__ __forceinline__ unsigned cl_rank() {
   return r;
 }
 __device__ __forceinline__ void cl_barrier() {
+  __syncwarp();  // the aligned form wants the warp's lanes together
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

@@ -83,7 +83,9 @@ __device__ __forceinline__ unsigned small_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// (the aligned forms want the warp's lanes together, which a loop before may have parted)
 __device__ __forceinline__ void small_arrive() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void small_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -205,6 +207,7 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+  small_wait();
   // x += alpha p, r -= alpha Ap and z = M^-1 r of the own vertices (a last vertex may have fewer than 3
   // rows), partials of r.z and r.r
   auto update = [&](float alpha, float &arz, float &arr) {
@@ -243,7 +246,6 @@ k_pcg_small(PcgSmall m, const float *__restrict__ rres, const float *__restrict_
   const float st_beta = st->beta;
   int it = cont ? st->it : 0;
   const int last = it + max_it;
-  small_wait();
   small_reduce<2>(arz, arr, s_warps, s_rz, rank, d2);
   if (warp == 0) {
     // as k_pcg_init: beta against the replaced residual when the direction continues
