@@ -22,7 +22,7 @@ namespace bartels {
 
 namespace {
 constexpr int kCtas = 16, kMaxThreads = 1024;
-constexpr int kMaxN = 24576;                // the direction (4 B each) fits beside the rest
+constexpr int kMaxN = kSmallMaxN;
 constexpr int64_t kMaxEntries = 2 << 20;    // past this the cluster's L2 bandwidth loses to the whole GPU
 constexpr int kSmemBytes = 225 * 1024;       // beside the static arrays
 }  // namespace

@@ -7,6 +7,8 @@
 
 namespace bartels {
 
+constexpr int kSmallMaxN = 24576;  // unknowns: the direction (4 B each) fits shared memory beside the rest
+
 // A scalar-CSR system on the host's side of the decision: row pointers on the
 // host, everything else on the device.
 struct PcgSmall {

@@ -994,7 +994,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
   PcgSmall small;
   std::vector<int> small_off, small_rp;
   const int *h_rp = op.h_rp;
-  if (blk && !op.mg && !op.gl && (int64_t)n <= 65536) {
+  if (blk && !op.mg && !op.gl && n <= kSmallMaxN) {
     small_rp.assign(n + 1, 0);
     for (int i = 0; i < n; ++i)
       small_rp[i + 1] = small_rp[i] + 3 * (op.plan->h_brp[i / 3 + 1] - op.plan->h_brp[i / 3]);
