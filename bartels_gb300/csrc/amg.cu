@@ -532,7 +532,8 @@ int mg_prepare(bartels_ctx ctx, bartels_mesh_plan plan) {
   // level 1 inside the cluster launch, where a step is cheap (24^3 Newton step:
   // 1 / 2 / 3 / 4 / 5 give 12.5 / 11.6 / 11.4 / 11.5 / 11.8 ms, smaller solves
   // are best at 2)
-  const int degcl = env_int("BARTELS_MG_DEGCL", 2, 1, (kMgCoef - 1) / 2 + 1);
+  const char *set = std::getenv("BARTELS_MG_DEGC");  // chosen by the user: wherever level 1 runs
+  const int degcl = env_int("BARTELS_MG_DEGCL", set && *set ? degc : 2, 1, (kMgCoef - 1) / 2 + 1);
   const int degc2 = env_int("BARTELS_MG_DEGC2", 5, 1, (kMgCoef - 1) / 2 + 1);
   mg->lv.resize(H.size());
   for (size_t l = 0; l < H.size(); ++l) {
