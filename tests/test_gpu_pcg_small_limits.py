@@ -60,10 +60,27 @@ def test_pinned_plan(n):
     plan.close()
 
 
-# r.z and p.Ap scale with 1 / A and A where b alone is of ordinary size: sums past the largest float while
-# every term fits, sums within the range at either side, and a matrix of ordinary size
-@pytest.mark.parametrize("n,a,b", [(10080, 1e-36, 10.0), (24576, 1e-36, 3.0), (10080, 1e-30, 1.0), (10080, 1e15, 1.0),
-                                   (3001, 1.0, 1e-4)])
-def test_matrices_far_from_unit_scale(n, a, b):
+# r.z and p.Ap scale with 1 / A and A where b alone is of ordinary size. What the general loop takes has to be
+# taken, and what it refuses (a warp's FP32 sum of r.z, ~96 b^2 / (18 a), leaves the range in the first case) is
+# refused: sums of the whole system past the largest float while every warp's fits, sums near the smallest, ordinary
+@pytest.mark.parametrize("n,a,b", [(10080, 1e-36, 10.0), (24576, 1e-36, 3.0), (10080, 1e-36, 1.0), (10080, 1e-30, 1.0),
+                                   (10080, 1e15, 1.0), (3001, 1.0, 1e-4)])
+def test_matrices_far_from_unit_scale(n, a, b, general, monkeypatch):
+    import bartels_gb300 as bg
+    from bartels_gb300.api import Context
     A = a * _spd(n, 20, n)
-    _direction(A, b * np.random.default_rng(n).standard_normal(n))
+    g = b * np.random.default_rng(n).standard_normal(n)
+    try:
+        _direction(A, g)
+        taken = True
+    except bg.BartelsError:
+        taken = False
+    monkeypatch.setattr(Context, "_default", None)
+    monkeypatch.delenv("BARTELS_PCG_SMALL")
+    if taken:
+        _direction(A, g)
+    else:
+        with pytest.raises(bg.BartelsError):
+            _direction(A, g)
+    Context.default().close()
+    assert taken == (96 * b * b / (18 * a) < 3.4e38)
