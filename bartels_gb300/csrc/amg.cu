@@ -800,9 +800,9 @@ __device__ __forceinline__ void cl_barrier() {
 // as in k_mg_inv6. One thread-block cluster; each CTA keeps the rows of its
 // own nodes (split) in shared memory. Per node K: the owner inverts the 6x6 pivot
 // block, scales the node's 6 rows with it and publishes them (panel, double-
-// buffered), then every CTA updates its other rows. One cluster barrier per node: 8 / 64 nodes take
-// ~16 / ~130 us; a single CTA with a barrier per scalar pivot took 58 us for
-// 8 and 552 us for 18.
+// buffered), then every CTA updates its other rows. One cluster barrier per node: 64 nodes take
+// 320 us (406 with the pivot block inverted by one thread); a single CTA with a barrier
+// per scalar pivot took 58 us for 8 nodes and 552 us for 18.
 struct MgInvArgs {
   int nodes = 0, split[kMgClusterMax + 1] = {};
   const int *rp = nullptr, *ci = nullptr, *rev = nullptr, *dpos = nullptr;
