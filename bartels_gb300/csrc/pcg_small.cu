@@ -118,8 +118,8 @@ __device__ __forceinline__ float2 pair_reduce(float2 v) {
   }
   return v;
 }
-// ~40 steps of 1.4e-45 are below 1e-10 of the sum, and no partial sum overflows; NaN is out
-__device__ __forceinline__ bool small_in_range(float2 a) { return fabsf(a.x) > 1e-33f && fabsf(a.x) < 1e36f; }
+// ~40 steps of 1.4e-45 stay below 2^-24 of the sum, and no partial sum overflows; NaN is out
+__device__ __forceinline__ bool small_in_range(float2 a) { return fabsf(a.x) > 1e-36f && fabsf(a.x) < 1e36f; }
 __device__ __forceinline__ double pair_value(float2 a) { return (double)a.x + (double)a.y; }
 // a / b rounded to FP32 (one correction of the FP32 quotient)
 __device__ __forceinline__ float pair_div(float2 a, float2 b) {

@@ -1045,7 +1045,7 @@ static int pcg_solve(bartels_ctx ctx, const PcgOperator &op, int n, const double
   }
   const double target = prm.rel_tol * bnorm;
   // its sums are float pairs: keep the squares well inside the float range, down to (target / 2)^2
-  is_small = is_small && bnorm < 1e12 && bnorm > 1e-9 && target > 1e-16;
+  is_small = is_small && bnorm < 1e12 && bnorm > 1e-9 && target > 2e-18;
   // CUDA graph of a fixed number of PCG iterations (kernels no-op once done)
   const int chunk = op.mg ? 8 : 16;  // fixed-length fallback only
   cudaGraphExec_t exec = nullptr;
